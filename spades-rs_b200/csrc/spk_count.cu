@@ -2056,38 +2056,67 @@ __global__ void __launch_bounds__(kBlock, 4) k_admit_compact(TableView t, unsign
 // count histogram's bin 1 and, when the list keeps count-1 k-mers (lmin 1),
 // are appended to the list after the span count's entries, one reservation
 // per warp.  sums: [0] admitted singletons.
+//
+// Bound by the random sectors of the twice tier (L2).  Most singletons are
+// turned away by their first bit (about one in eight of the tier's bits is
+// set after 5 Mb x 100x at k = 55), so the second and the third position are
+// hashed and read only for those that got that far: 1.14 sectors a singleton
+// instead of 3.  kAdmitFlight singletons per thread keep as many first reads
+// in flight as three reads of one singleton did.
+constexpr int kAdmitFlight = 4;
 template <int NL>
 __global__ void __launch_bounds__(kBlock) k_admit_singletons(ListOut lo, unsigned k, FastMod fm,
                                                               const uint64_t* __restrict__ twice,
                                                               unsigned long long* __restrict__ sums) {
+  constexpr int U = kAdmitFlight;
   const unsigned lane = threadIdx.x & 31;
   const uint64_t n = min((uint64_t)lo.fill[1], lo.scap);
   uint64_t adm = 0;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x; base < n; base += stride) {
-    const uint64_t i = base + threadIdx.x;
-    bool admit = false;
-    Seq<NL> C;
-    if (i < n) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x * U;
+  for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x * U; base < n; base += stride) {
+    HashPre hp[U];
+    uint64_t p0[U], w0[U];
 #pragma unroll
-      for (int j = 0; j < NL; j++) C.v[j] = __ldcs(lo.s[j] + i);
-      uint64_t raw[3], pos[3];
-      bloom_positions<NL>(C, k, fm, raw, pos);
-      const uint64_t a = __ldg(twice + (pos[0] >> 6)), b = __ldg(twice + (pos[1] >> 6)),
-                     c = __ldg(twice + (pos[2] >> 6));
-      admit = (a >> (pos[0] & 63)) & (b >> (pos[1] & 63)) & (c >> (pos[2] & 63)) & 1;
+    for (int u = 0; u < U; u++) {
+      const uint64_t i = base + (uint64_t)u * blockDim.x + threadIdx.x;
+      w0[u] = 0;
+      p0[u] = 0;
+      hp[u] = HashPre{0, 0, 0, 0};
+      if (i < n) {
+        Seq<NL> C;
+#pragma unroll
+        for (int j = 0; j < NL; j++) C.v[j] = __ldcs(lo.s[j] + i);
+        uint64_t w4[4];
+        kmer256_limbs<NL>(C, k, w4);
+        hp[u] = hash_pre(w4);
+        p0[u] = fastmod(fm, hash_seed(hp[u], kSeed1));
+        w0[u] = __ldg(twice + (p0[u] >> 6));
+      }
     }
-    adm += admit;
-    if (lo.lmin <= 1) {
-      const unsigned m = __ballot_sync(FULL, admit);
-      if (m) {
-        unsigned long long wb = 0;
-        if (lane == 0) wb = atomicAdd(lo.fill, (unsigned long long)__popc(m));
-        const uint64_t q = __shfl_sync(FULL, wb, 0) + __popc(m & lanemask_lt());
-        if (admit && q < lo.cap) {
 #pragma unroll
-          for (int j = 0; j < NL; j++) lo.l[j][q] = C.v[j];
-          lo.cnt[q] = 1;
+    for (int u = 0; u < U; u++) {
+      bool admit = (w0[u] >> (p0[u] & 63)) & 1;
+      if (admit) {
+        const uint64_t q = fastmod(fm, hash_seed(hp[u], kSeed2));
+        admit = (__ldg(twice + (q >> 6)) >> (q & 63)) & 1;
+      }
+      if (admit) {
+        const uint64_t q = fastmod(fm, hash_seed(hp[u], kSeed3));
+        admit = (__ldg(twice + (q >> 6)) >> (q & 63)) & 1;
+      }
+      adm += admit;
+      if (lo.lmin <= 1) {
+        const unsigned m = __ballot_sync(FULL, admit);
+        if (m) {
+          unsigned long long wb = 0;
+          if (lane == 0) wb = atomicAdd(lo.fill, (unsigned long long)__popc(m));
+          const uint64_t q = __shfl_sync(FULL, wb, 0) + __popc(m & lanemask_lt());
+          if (admit && q < lo.cap) {
+            const uint64_t i = base + (uint64_t)u * blockDim.x + threadIdx.x;
+#pragma unroll
+            for (int j = 0; j < NL; j++) lo.l[j][q] = lo.s[j][i];
+            lo.cnt[q] = 1;
+          }
         }
       }
     }
