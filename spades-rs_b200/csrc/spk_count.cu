@@ -2060,67 +2060,87 @@ __global__ void __launch_bounds__(kBlock, 4) k_admit_compact(TableView t, unsign
 // Bound by the random sectors of the twice tier (L2).  Most singletons are
 // turned away by their first bit (about one in eight of the tier's bits is
 // set after 5 Mb x 100x at k = 55), so the second and the third position are
-// hashed and read only for those that got that far: 1.14 sectors a singleton
-// instead of 3.  kAdmitFlight singletons per thread keep as many first reads
-// in flight as three reads of one singleton did.
-constexpr int kAdmitFlight = 4;
+// hashed and read only for those that got that far.  Those wait in a queue of
+// the warp until 32 of them fill it: tested in place they left a warp waiting
+// for two more reads of a few of its lanes almost every time.
+constexpr int kAdmitFlight = 4;  // first reads in flight per thread
 template <int NL>
 __global__ void __launch_bounds__(kBlock) k_admit_singletons(ListOut lo, unsigned k, FastMod fm,
                                                               const uint64_t* __restrict__ twice,
                                                               unsigned long long* __restrict__ sums) {
   constexpr int U = kAdmitFlight;
+  __shared__ uint64_t queue[kBlock / 32][NL][64];
   const unsigned lane = threadIdx.x & 31;
+  uint64_t (&q)[NL][64] = queue[threadIdx.x >> 5];
   const uint64_t n = min((uint64_t)lo.fill[1], lo.scap);
   uint64_t adm = 0;
+  uint32_t nq = 0;
+  // The last `m` (at most 32) queued k-mers against their other two bits.
+  auto drain = [&](uint32_t m) {
+    __syncwarp();
+    bool admit = lane < m;
+    Seq<NL> C;
+    if (admit) {
+#pragma unroll
+      for (int j = 0; j < NL; j++) C.v[j] = q[j][nq - m + lane];
+      uint64_t w4[4];
+      kmer256_limbs<NL>(C, k, w4);
+      const HashPre hp = hash_pre(w4);
+      const uint64_t p1 = fastmod(fm, hash_seed(hp, kSeed2)), p2 = fastmod(fm, hash_seed(hp, kSeed3));
+      const uint64_t a = __ldg(twice + (p1 >> 6)), b = __ldg(twice + (p2 >> 6));
+      admit = (a >> (p1 & 63)) & (b >> (p2 & 63)) & 1;
+    }
+    nq -= m;
+    adm += admit;
+    if (lo.lmin <= 1) {
+      const unsigned mm = __ballot_sync(FULL, admit);
+      if (mm) {
+        unsigned long long wb = 0;
+        if (lane == 0) wb = atomicAdd(lo.fill, (unsigned long long)__popc(mm));
+        const uint64_t d = __shfl_sync(FULL, wb, 0) + __popc(mm & lanemask_lt());
+        if (admit && d < lo.cap) {
+#pragma unroll
+          for (int j = 0; j < NL; j++) lo.l[j][d] = C.v[j];
+          lo.cnt[d] = 1;
+        }
+      }
+    }
+    __syncwarp();
+  };
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x * U;
   for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x * U; base < n; base += stride) {
-    HashPre hp[U];
-    uint64_t p0[U], w0[U];
+    Seq<NL> C[U];
+    uint64_t w0[U];
+    uint32_t sh[U];
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const uint64_t i = base + (uint64_t)u * blockDim.x + threadIdx.x;
       w0[u] = 0;
-      p0[u] = 0;
-      hp[u] = HashPre{0, 0, 0, 0};
+      sh[u] = 0;
       if (i < n) {
-        Seq<NL> C;
 #pragma unroll
-        for (int j = 0; j < NL; j++) C.v[j] = __ldcs(lo.s[j] + i);
+        for (int j = 0; j < NL; j++) C[u].v[j] = __ldcs(lo.s[j] + i);
         uint64_t w4[4];
-        kmer256_limbs<NL>(C, k, w4);
-        hp[u] = hash_pre(w4);
-        p0[u] = fastmod(fm, hash_seed(hp[u], kSeed1));
-        w0[u] = __ldg(twice + (p0[u] >> 6));
+        kmer256_limbs<NL>(C[u], k, w4);
+        const uint64_t p0 = fastmod(fm, hash_seed(hash_pre(w4), kSeed1));
+        w0[u] = __ldg(twice + (p0 >> 6));
+        sh[u] = (uint32_t)(p0 & 63);
       }
     }
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      bool admit = (w0[u] >> (p0[u] & 63)) & 1;
-      if (admit) {
-        const uint64_t q = fastmod(fm, hash_seed(hp[u], kSeed2));
-        admit = (__ldg(twice + (q >> 6)) >> (q & 63)) & 1;
-      }
-      if (admit) {
-        const uint64_t q = fastmod(fm, hash_seed(hp[u], kSeed3));
-        admit = (__ldg(twice + (q >> 6)) >> (q & 63)) & 1;
-      }
-      adm += admit;
-      if (lo.lmin <= 1) {
-        const unsigned m = __ballot_sync(FULL, admit);
-        if (m) {
-          unsigned long long wb = 0;
-          if (lane == 0) wb = atomicAdd(lo.fill, (unsigned long long)__popc(m));
-          const uint64_t q = __shfl_sync(FULL, wb, 0) + __popc(m & lanemask_lt());
-          if (admit && q < lo.cap) {
-            const uint64_t i = base + (uint64_t)u * blockDim.x + threadIdx.x;
+      const bool on = (w0[u] >> sh[u]) & 1;
+      const unsigned m = __ballot_sync(FULL, on);
+      if (on) {
+        const uint32_t at = nq + __popc(m & lanemask_lt());
 #pragma unroll
-            for (int j = 0; j < NL; j++) lo.l[j][q] = lo.s[j][i];
-            lo.cnt[q] = 1;
-          }
-        }
+        for (int j = 0; j < NL; j++) q[j][at] = C[u].v[j];
       }
+      nq += __popc(m);
+      if (nq >= 32) drain(32);
     }
   }
+  if (nq) drain(nq);
   warp_add_u64(sums, adm);
   warp_add_u64(lo.hist + 1, adm);
 }
@@ -3525,9 +3545,7 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   // after the first group's partition, when a single group has freed its
   // coarse buckets, so that they never coexist).
   const bool early_sort = lmin_pre >= 2;
-  SideStream side;
-  if (early_sort && (rc = side.open())) return rc;
-  DevSort lsort, esort;  // after `side`: its buffers are freed on that stream first
+  DevSort lsort, esort;
   DevBuf rbase, rfill, ops, sgl[4];
   RangeView bv{};
   ListOut lo{};
@@ -3627,17 +3645,6 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   cfirst.release();
   {
     SPK_CUDA(cudaEventRecord(kc1.e, st));
-    if (early_sort) {
-      // The list is final once the spans are counted (singletons are not
-      // listed): sort it on the side stream while the job's stream builds
-      // the Bloom tiers, admits the singletons and finds the cutoff.
-      SPK_CUDA(cudaEventRecord(side.fork, st));
-      SPK_CUDA(cudaStreamWaitEvent(side.s, side.fork, 0));
-      if ((rc = sort_dev_enqueue(side.s, nl, lcap_, su + S_LFILL, 2 * k, kr.list, &kr.list[4], nullptr, lsort,
-                                 &launches)))
-        return rc;
-      SPK_CUDA(cudaEventRecord(side.join, side.s));
-    }
     region.release();
     base.release();
     fill.release();
@@ -3661,12 +3668,20 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
     SPK_CUDA(cudaGetLastError());
     launches++;
   }
+  if (early_sort) {
+    // The list is final (singletons are not listed): sorted here, while the
+    // host waits for the readback below, with the singleton buffers as
+    // temporaries.  On a second stream beside the Bloom and admission kernels
+    // (which read the tier from L2 that the sort's scattered writes evict) the
+    // three took 3.2 ms at 5 Mb x 100x, k = 55, one after another 1.95.
+    if ((rc = sort_dev_enqueue(st, nl, lcap_, su + S_LFILL, 2 * k, kr.list, &kr.list[4], sgl, lsort, &launches)))
+      return rc;
+  }
   uint32_t* thr = (uint32_t*)(sw + S_THR);
   k_cutoff<<<1, 32, 0, st>>>(su + S_HIST, fixed, list_min, thr);
   SPK_CUDA(cudaGetLastError());
   launches++;
   // ---- the one mid-job readback ----
-  if (early_sort) SPK_CUDA(cudaStreamWaitEvent(st, side.join, 0));
   SPK_CUDA(cudaMemcpyAsync(host, sw, S_WORDS * 8, cudaMemcpyDeviceToHost, st));
   SPK_CUDA(cudaStreamSynchronize(st));
   const int err = (int)host[S_ERR];

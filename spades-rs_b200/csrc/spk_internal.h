@@ -267,10 +267,9 @@ int download_bloom(spk_result* res, int ki, uint64_t* seen, uint64_t* twice, uin
 // key.  The buffers may be swapped with temporaries.
 int radix_sort_bufs(cudaStream_t st, int nl, uint64_t n, unsigned nbits, DevBuf* keys,
                     DevBuf* vals, uint32_t* launches = nullptr);
-// The same result with an MSD split into 65536 buckets by the top 16 bits and
-// a shared-memory sort per bucket (large lists; falls back to the radix sort
-// for short lists and for buckets too large for shared memory).  h_staging:
-// a pinned host staging block (kStagingBytes).
+// The same result with an MSD split into buckets of about 16 items by the top
+// bits and a sort per bucket (buckets too large for shared memory go to the
+// radix sort).  h_staging: a pinned host staging block (kStagingBytes).
 int sort_bufs(cudaStream_t st, int nl, uint64_t n, unsigned nbits, DevBuf* keys, DevBuf* vals,
               uint64_t* h_staging, uint32_t* launches = nullptr);
 // ErrorCorrector::correct_read_in_place on every read (spk_correct.cu), against
@@ -295,22 +294,18 @@ int current_sm_count();
 struct DevSort {
   int nl = 0;
   unsigned nbits = 0;
-  uint32_t bbits = 0;
   uint64_t n_cap = 0;
   bool has_vals = false;
   bool pending = false;
-  DevBuf tk[4], tv, hist, off, cur, big;
+  DevBuf tk[4], tv, work;
   void rehome(cudaStream_t s) {
     for (DevBuf& b : tk) b.st = s;
-    tv.st = hist.st = off.st = cur.st = big.st = s;
+    tv.st = work.st = s;
   }
   void release() {
     for (DevBuf& b : tk) b.release();
     tv.release();
-    hist.release();
-    off.release();
-    cur.release();
-    big.release();
+    work.release();
   }
 };
 int sort_dev_enqueue(cudaStream_t st, int nl, uint64_t n_cap, const unsigned long long* n_dev,

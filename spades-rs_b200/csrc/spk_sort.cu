@@ -272,16 +272,34 @@ int radix_sort_bufs(cudaStream_t st, int nl, uint64_t n, unsigned nbits, DevBuf*
 }
 
 // ---------------------------------------------------------------------------
-// Bucket sort: an MSD split on the top b significant bits of the key into 2^b
-// buckets (b chosen for ~128 items per bucket, 8 <= b <= 16), then a bitonic
-// sort of each bucket in shared memory.  The top bits of canonical k-mers
-// and (k+1)-mers spread their lists over the buckets; a bucket larger than
-// BS_LOCAL items is sorted by the LSD radix sort above instead.  Equal keys
-// do not occur (the lists hold distinct k-mers), so stability is not needed.
+// Bucket sort: an MSD split into buckets of about 16 items, then each bucket
+// sorted on its own.  The top 12 bits of the keys split the list into coarse
+// bins; a bin of c items is cut into ceil(c / 16) buckets (fewer and larger
+// ones beyond 2^20 buckets) by the 32 bits that follow, so bucket sizes stay
+// even where GC content makes some prefixes ten times as common as others.
+// Runs of neighbouring buckets of at most 32 items together are sorted by one
+// warp in registers, one item per lane; buckets of up to BS_WARP items by one
+// warp with up to four items per lane; larger ones by the CTA in shared
+// memory; and a bucket of more than BS_LOCAL items (keys that share a long
+// prefix) goes to the LSD radix sort above.  Equal keys do not occur (the lists
+// hold distinct k-mers), so stability is not needed.
+//
+// The split costs one read and one scattered write of the list whatever the
+// number of buckets (their write frontiers stay in L2), while a bucket's sort
+// grows with the square of its log.  With 2^16 buckets of 120 items and
+// bitonic stages in shared memory the local sort took 0.49 ms for the 5 M
+// edges of 5 Mb x 100x (k = 55), in registers 0.24; equal cuts by the top 18
+// bits took 1.34 ms for the 3.4 M k-mers of a genome of 35% GC, where the
+// A/T-rich buckets went to the shared-memory sort.  Lists below 2^18 items
+// took the LSD sort, 5 launches for each of its 8 to 32 passes (85 launches
+// for a 10 kb sample at k = 31: 1.01 -> 0.78 ms for the job).
 // ---------------------------------------------------------------------------
-constexpr uint32_t BS_MAX_BITS = 16;
+constexpr uint32_t BS_COARSE_BITS = 12, BS_COARSE = 1u << BS_COARSE_BITS;
+constexpr uint32_t BS_PER = 16;                 // items per bucket aimed at
+constexpr uint32_t BS_MAX_BUCKETS = 1u << 20;   // ... up to this many buckets (plus one per coarse bin)
 constexpr uint32_t BS_LOCAL = 2048;
 constexpr int BS_BLOCK = 256;
+constexpr uint32_t BS_CHUNK = BS_BLOCK;  // buckets a CTA takes at a time (32 per warp)
 constexpr uint32_t BS_MAX_BIG = 4096;
 constexpr uint64_t BS_STAGE_WORDS = 1024;  // big-bucket list offset in the host staging block
 
@@ -289,207 +307,313 @@ struct Limbs {
   uint64_t* p[4];
 };
 
+// Device words of one sort, zeroed before it: coarse counts, the plan (the
+// first bucket of every coarse bin, then their total), a ticket, the number
+// of big buckets and their list, and the buckets' offsets.
+struct BsWork {
+  uint32_t *coarse, *plan, *ticket, *nbig, *big, *off;
+};
+static BsWork bs_work(uint32_t* w) {
+  BsWork b{};
+  b.coarse = w;
+  b.plan = b.coarse + BS_COARSE;
+  b.ticket = b.plan + BS_COARSE + 1;
+  b.nbig = b.ticket + 1;
+  b.big = b.nbig + 1;
+  b.off = b.big + 3 * BS_MAX_BIG + 1;
+  return b;
+}
+// Most buckets a list of n items is cut into.
+static uint32_t bs_max_buckets(uint64_t n) {
+  return (uint32_t)std::min<uint64_t>((n + BS_PER - 1) / BS_PER, BS_MAX_BUCKETS) + BS_COARSE;
+}
+static size_t bs_work_bytes(uint64_t n) { return (3 + 2 * BS_COARSE + 3 * BS_MAX_BIG + 1 + (size_t)bs_max_buckets(n)) * 4; }
+
+// The top 44 of a key's nbits bits (shorter keys: followed by zeros).
 template <int NL>
-__device__ __forceinline__ uint32_t bs_digit(const Limbs& L, uint64_t i, unsigned limb, unsigned sh,
-                                             uint32_t nb) {
+__device__ __forceinline__ uint64_t bs_top(const Limbs& L, uint64_t i, unsigned nbits) {
+  if (nbits < 44) return L.p[0][i] << (44 - nbits);
+  const unsigned limb = (nbits - 44) / 64, sh = (nbits - 44) % 64;
   uint64_t lo = 0, hi = 0;
 #pragma unroll
   for (int j = 0; j < NL; j++) {
     if ((unsigned)j == limb) lo = L.p[j][i];
-    if ((unsigned)j == limb + 1) hi = L.p[j][i];
+    if ((unsigned)j == limb + 1 && sh > 20) hi = L.p[j][i];
   }
-  return (uint32_t)(((lo >> sh) | ((hi << 1) << (63 - sh))) & (nb - 1));
+  return ((lo >> sh) | ((hi << 1) << (63 - sh))) & ((1ULL << 44) - 1);
+}
+// The bucket of a key: its coarse bin's share cut evenly by the next 32 bits
+// (a non-decreasing function of the key).
+__device__ __forceinline__ uint32_t bs_bucket(uint64_t top, const uint32_t* __restrict__ plan) {
+  const uint32_t c = (uint32_t)(top >> 32);
+  const uint32_t p0 = __ldg(plan + c), p1 = __ldg(plan + c + 1);
+  return p0 + __umulhi((uint32_t)top, p1 - p0);
 }
 
+// Coarse counts; the last CTA turns them into the plan.
 // n_dev (nullable): the item count in device memory, at most n.
 template <int NL>
+__global__ void __launch_bounds__(BS_BLOCK) k_bs_coarse(Limbs L, uint64_t n, const unsigned long long* n_dev,
+                                                         unsigned nbits, BsWork W) {
+  __shared__ uint32_t h[BS_COARSE];
+  __shared__ uint32_t ws[BS_BLOCK / 32];
+  __shared__ bool last;
+  if (n_dev) n = min(n, (uint64_t)*n_dev);
+  for (uint32_t c = threadIdx.x; c < BS_COARSE; c += BS_BLOCK) h[c] = 0;
+  __syncthreads();
+  for (uint64_t i = blockIdx.x * (uint64_t)BS_BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BS_BLOCK)
+    atomicAdd(&h[bs_top<NL>(L, i, nbits) >> 32], 1u);
+  __syncthreads();
+  for (uint32_t c = threadIdx.x; c < BS_COARSE; c += BS_BLOCK)
+    if (h[c]) atomicAdd(W.coarse + c, h[c]);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(W.ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const uint64_t per = max((uint64_t)BS_PER, (n + BS_MAX_BUCKETS - 1) / BS_MAX_BUCKETS);
+  constexpr uint32_t IPT = BS_COARSE / BS_BLOCK;
+  uint32_t v[IPT], s = 0;
+#pragma unroll
+  for (uint32_t j = 0; j < IPT; j++) {
+    v[j] = (uint32_t)((__ldcg(W.coarse + threadIdx.x * IPT + j) + per - 1) / per);
+    s += v[j];
+  }
+  uint32_t tot, run = block_excl_scan(s, ws, &tot);
+#pragma unroll
+  for (uint32_t j = 0; j < IPT; j++) {
+    W.plan[threadIdx.x * IPT + j] = run;
+    run += v[j];
+  }
+  if (threadIdx.x == 0) W.plan[BS_COARSE] = tot;
+}
+
+template <int NL>
 __global__ void __launch_bounds__(BS_BLOCK) k_bs_hist(Limbs L, uint64_t n, const unsigned long long* n_dev,
-                                                       unsigned limb, unsigned sh, uint32_t nb,
-                                                       uint32_t* __restrict__ hist) {
+                                                       unsigned nbits, BsWork W) {
   if (n_dev) n = min(n, (uint64_t)*n_dev);
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x)
-    atomicAdd(hist + bs_digit<NL>(L, i, limb, sh, nb), 1u);
+    atomicAdd(W.off + bs_bucket(bs_top<NL>(L, i, nbits), W.plan), 1u);
 }
 
+// W.off: the buckets' first positions, advanced to their ends as items arrive.
 template <int NL, bool HASV>
 __global__ void __launch_bounds__(BS_BLOCK) k_bs_scatter(Limbs S, const uint32_t* __restrict__ sv, Limbs D,
                                                           uint32_t* __restrict__ dv, uint64_t n,
-                                                          const unsigned long long* n_dev,
-                                                          unsigned limb, unsigned sh, uint32_t nb,
-                                                          uint32_t* __restrict__ cur) {
+                                                          const unsigned long long* n_dev, unsigned nbits,
+                                                          BsWork W) {
   if (n_dev) n = min(n, (uint64_t)*n_dev);
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t p = atomicAdd(cur + bs_digit<NL>(S, i, limb, sh, nb), 1u);
+    const uint32_t p = atomicAdd(W.off + bs_bucket(bs_top<NL>(S, i, nbits), W.plan), 1u);
 #pragma unroll
     for (int j = 0; j < NL; j++) D.p[j][p] = S.p[j][i];
     if (HASV) dv[p] = sv[i];
   }
 }
 
-// A bitonic sort of P (a power of two, <= BS_WARP) items in one warp's
-// shared-memory region, ascending on the limbs (most significant last).
-constexpr uint32_t BS_WARP = 256;  // largest bucket one warp sorts
-template <int NL, bool HASV>
-__device__ __forceinline__ void warp_bitonic(uint64_t* sk, uint32_t* svl, uint32_t P) {
+constexpr uint32_t BS_WARP = 128;  // largest bucket one warp sorts
+
+// Items [o, o + m), m <= 32 R, of T sorted ascending into D by one warp in
+// registers: item r * 32 + lane in register r, a bitonic network whose
+// distances below 32 are lane exchanges and whose others swap registers.
+// Missing items are all-ones keys, which no item exceeds.
+template <int NL, bool HASV, int R>
+__device__ __forceinline__ void warp_sort(const Limbs& T, const uint32_t* __restrict__ tv, const Limbs& D,
+                                          uint32_t* __restrict__ dv, uint32_t o, uint32_t m) {
   const unsigned lane = threadIdx.x & 31;
-  for (uint32_t kk = 2; kk <= P; kk <<= 1) {
-    for (uint32_t j = kk >> 1; j > 0; j >>= 1) {
-      for (uint32_t i = lane; i < P; i += 32) {
-        const uint32_t x = i ^ j;
-        if (x <= i) continue;
-        bool gt = false, eq = true;
+  uint64_t key[R][NL];
+  uint32_t val[R];
 #pragma unroll
-        for (int q = NL - 1; q >= 0; q--) {
-          const uint64_t u = sk[q * BS_WARP + i], v = sk[q * BS_WARP + x];
-          if (eq && u != v) {
-            gt = u > v;
-            eq = false;
+  for (int r = 0; r < R; r++) {
+    const uint32_t i = r * 32 + lane;
+    const bool in = i < m;
+#pragma unroll
+    for (int j = 0; j < NL; j++) key[r][j] = in ? T.p[j][o + i] : ~0ULL;
+    val[r] = (HASV && in) ? tv[o + i] : 0u;
+  }
+  auto gt = [](const uint64_t (&a)[NL], const uint64_t (&b)[NL]) {
+    bool g = a[0] > b[0];
+#pragma unroll
+    for (int j = 1; j < NL; j++) g = a[j] > b[j] || (a[j] == b[j] && g);
+    return g;
+  };
+#pragma unroll
+  for (uint32_t kk = 2; kk <= 32 * R; kk <<= 1) {
+#pragma unroll
+    for (uint32_t j = kk >> 1; j > 0; j >>= 1) {
+      if (j >= 32) {
+        const int q = (int)(j / 32);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          if (r & q) continue;
+          const bool up = ((r * 32 + lane) & kk) == 0;
+          if (gt(key[r], key[r | q]) == up) {
+#pragma unroll
+            for (int l = 0; l < NL; l++) {
+              const uint64_t t = key[r][l];
+              key[r][l] = key[r | q][l];
+              key[r | q][l] = t;
+            }
+            const uint32_t t = val[r];
+            val[r] = val[r | q];
+            val[r | q] = t;
           }
         }
-        if (gt == ((i & kk) == 0) && !eq) {
+      } else {
 #pragma unroll
-          for (int q = 0; q < NL; q++) {
-            const uint64_t t = sk[q * BS_WARP + i];
-            sk[q * BS_WARP + i] = sk[q * BS_WARP + x];
-            sk[q * BS_WARP + x] = t;
-          }
-          if (HASV) {
-            const uint32_t t = svl[i];
-            svl[i] = svl[x];
-            svl[x] = t;
+        for (int r = 0; r < R; r++) {
+          uint64_t ok[NL];
+#pragma unroll
+          for (int l = 0; l < NL; l++) ok[l] = __shfl_xor_sync(FULLM, key[r][l], j);
+          const uint32_t ov = HASV ? __shfl_xor_sync(FULLM, val[r], j) : 0u;
+          const bool lower = (lane & j) == 0, up = ((r * 32 + lane) & kk) == 0;
+          // the lower lane of a pair keeps the smaller item when the run goes up
+          const bool mine_gt = gt(key[r], ok), theirs_gt = gt(ok, key[r]);
+          if (lower == up ? mine_gt : theirs_gt) {
+#pragma unroll
+            for (int l = 0; l < NL; l++) key[r][l] = ok[l];
+            val[r] = ov;
           }
         }
       }
-      __syncwarp();
     }
+  }
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    const uint32_t i = r * 32 + lane;
+    if (i >= m) continue;
+#pragma unroll
+    for (int j = 0; j < NL; j++) D.p[j][o + i] = key[r][j];
+    if (HASV) dv[o + i] = val[r];
   }
 }
 
-// Sorts every bucket of at most BS_LOCAL items from T into D: buckets of at
-// most BS_WARP items one per warp, the others one per CTA.  Larger buckets
-// are copied to D unsorted and listed in big[3i..3i+2] = (bucket, offset,
-// size) for the host, which sorts them from T.
+// Sorts every bucket of at most BS_LOCAL items from T into D; off[b] is the
+// end of bucket b (its start is off[b - 1]).  A CTA takes BS_CHUNK buckets at a
+// time, 32 per warp; the buckets too large for a warp wait in s_mid for the
+// whole CTA.  Larger ones than BS_LOCAL are copied to D unsorted and listed in
+// big[3i..3i+2] = (bucket, offset, size) for the host, which sorts them from T.
+// Bound by the exchanges (15 stages of 2 NL + 1 shuffles for 32 items).
 template <int NL, bool HASV>
 __global__ void __launch_bounds__(BS_BLOCK) k_bs_local(Limbs T, const uint32_t* __restrict__ tv, Limbs D,
-                                                        uint32_t* __restrict__ dv,
-                                                        const uint32_t* __restrict__ off,
-                                                        const uint32_t* __restrict__ size, uint32_t nb,
-                                                        uint32_t* __restrict__ big,
-                                                        unsigned* __restrict__ nbig) {
+                                                        uint32_t* __restrict__ dv, BsWork W) {
   extern __shared__ __align__(16) uint64_t bs_smem[];
-  // Warp phase: warp w sorts the small buckets b = its global warp index +
-  // j * (all warps), in its own region of BS_WARP items.
-  {
-    const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    uint64_t* wk = bs_smem + (size_t)w * BS_WARP * (NL + (HASV ? 1 : 0));
-    uint32_t* wv = (uint32_t*)(wk + NL * BS_WARP);
-    const uint32_t gw = blockIdx.x * (BS_BLOCK / 32) + w, nw = gridDim.x * (BS_BLOCK / 32);
-    for (uint32_t b = gw; b < nb; b += nw) {
-      const uint32_t m = size[b];
-      if (m == 0 || m > BS_WARP) continue;
-      const uint32_t o = off[b];
-      if (m == 1) {
-        if (lane == 0) {
+  __shared__ uint32_t s_mid[BS_CHUNK];
+  __shared__ uint32_t s_nmid;
+  const uint32_t nb = W.plan[BS_COARSE];
+  const uint32_t* __restrict__ off = W.off;
+  const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint64_t* sk = bs_smem;                                // NL arrays of BS_LOCAL limbs
+  uint32_t* svl = (uint32_t*)(bs_smem + NL * BS_LOCAL);  // values
+  for (uint32_t c0 = blockIdx.x * BS_CHUNK; c0 < nb; c0 += gridDim.x * BS_CHUNK) {
+    if (threadIdx.x == 0) s_nmid = 0;
+    __syncthreads();
+    const uint32_t b0 = c0 + w * 32;
+    if (b0 < nb) {
+      const uint32_t nw = min(32u, nb - b0);
+      const uint32_t end = off[b0 + min(lane, nw - 1)];
+      uint32_t s = b0 ? off[b0 - 1] : 0u;
+      uint32_t cur = 0;
+      while (cur < nw) {
+        // buckets cur..last hold at most 32 items together
+        const unsigned fit = __ballot_sync(FULLM, lane >= cur && lane < nw && end - s <= 32);
+        if (fit) {
+          const uint32_t last = 31 - __clz(fit);
+          const uint32_t e = __shfl_sync(FULLM, end, last);
+          if (e > s) warp_sort<NL, HASV, 1>(T, tv, D, dv, s, e - s);
+          s = e;
+          cur = last + 1;
+          continue;
+        }
+        const uint32_t e = __shfl_sync(FULLM, end, cur);
+        const uint32_t m = e - s;
+        if (m <= 64) {
+          warp_sort<NL, HASV, 2>(T, tv, D, dv, s, m);
+        } else if (m <= BS_WARP) {
+          warp_sort<NL, HASV, 4>(T, tv, D, dv, s, m);
+        } else if (lane == 0) {
+          s_mid[atomicAdd(&s_nmid, 1u)] = b0 + cur;
+        }
+        s = e;
+        cur++;
+      }
+    }
+    __syncthreads();
+    const uint32_t nmid = s_nmid;
+    for (uint32_t q = 0; q < nmid; q++) {
+      const uint32_t b = s_mid[q];
+      const uint32_t o = b ? off[b - 1] : 0u, m = off[b] - o;
+      if (m > BS_LOCAL) {
+        if (threadIdx.x == 0) {
+          const unsigned i = atomicAdd(W.nbig, 1u);
+          if (i < BS_MAX_BIG) {
+            W.big[3 * i] = b;
+            W.big[3 * i + 1] = o;
+            W.big[3 * i + 2] = m;
+          }
+        }
+        // The bucket goes to its place unsorted, so that D holds the whole
+        // list (in every bucket's range) before the host sorts this range.
+        for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
 #pragma unroll
-          for (int j = 0; j < NL; j++) D.p[j][o] = T.p[j][o];
-          if (HASV) dv[o] = tv[o];
+          for (int j = 0; j < NL; j++) D.p[j][o + i] = T.p[j][o + i];
+          if (HASV) dv[o + i] = tv[o + i];
         }
         continue;
       }
-      uint32_t P = 2;
+      uint32_t P = 1;
       while (P < m) P <<= 1;
-      for (uint32_t i = lane; i < P; i += 32) {
+      for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) {
         const bool in = i < m;
 #pragma unroll
-        for (int j = 0; j < NL; j++) wk[j * BS_WARP + i] = in ? T.p[j][o + i] : ~0ULL;
-        if (HASV) wv[i] = in ? tv[o + i] : 0u;
+        for (int j = 0; j < NL; j++) sk[j * BS_LOCAL + i] = in ? T.p[j][o + i] : ~0ULL;
+        if (HASV) svl[i] = in ? tv[o + i] : 0u;
       }
-      __syncwarp();
-      warp_bitonic<NL, HASV>(wk, wv, P);
-      for (uint32_t i = lane; i < m; i += 32) {
+      __syncthreads();
+      for (uint32_t kk = 2; kk <= P; kk <<= 1) {
+        for (uint32_t j = kk >> 1; j > 0; j >>= 1) {
+          for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) {
+            const uint32_t x = i ^ j;
+            if (x <= i) continue;
+            // a > b on the limbs, most significant first
+            bool g = false, eq = true;
 #pragma unroll
-        for (int j = 0; j < NL; j++) D.p[j][o + i] = wk[j * BS_WARP + i];
-        if (HASV) dv[o + i] = wv[i];
-      }
-      __syncwarp();
-    }
-  }
-  __syncthreads();
-  // CTA phase: the buckets of BS_WARP < items <= BS_LOCAL.
-  uint64_t* sk = bs_smem;                              // NL arrays of BS_LOCAL limbs
-  uint32_t* svl = (uint32_t*)(bs_smem + NL * BS_LOCAL);  // values
-  for (uint32_t b = blockIdx.x; b < nb; b += gridDim.x) {
-    const uint32_t m = size[b];
-    if (m <= BS_WARP) continue;
-    const uint32_t o = off[b];
-    if (m > BS_LOCAL) {
-      if (threadIdx.x == 0) {
-        const unsigned q = atomicAdd(nbig, 1u);
-        if (q < BS_MAX_BIG) {
-          big[3 * q] = b;
-          big[3 * q + 1] = o;
-          big[3 * q + 2] = m;
+            for (int l = NL - 1; l >= 0; l--) {
+              const uint64_t u = sk[l * BS_LOCAL + i], v = sk[l * BS_LOCAL + x];
+              if (eq && u != v) {
+                g = u > v;
+                eq = false;
+              }
+            }
+            const bool up = (i & kk) == 0;
+            if (g == up && !eq) {
+#pragma unroll
+              for (int l = 0; l < NL; l++) {
+                const uint64_t t = sk[l * BS_LOCAL + i];
+                sk[l * BS_LOCAL + i] = sk[l * BS_LOCAL + x];
+                sk[l * BS_LOCAL + x] = t;
+              }
+              if (HASV) {
+                const uint32_t t = svl[i];
+                svl[i] = svl[x];
+                svl[x] = t;
+              }
+            }
+          }
+          __syncthreads();
         }
       }
-      // The bucket goes to its place unsorted, so that D holds the whole
-      // list (in every bucket's range) before the host sorts this range.
       for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
 #pragma unroll
-        for (int j = 0; j < NL; j++) D.p[j][o + i] = T.p[j][o + i];
-        if (HASV) dv[o + i] = tv[o + i];
+        for (int j = 0; j < NL; j++) D.p[j][o + i] = sk[j * BS_LOCAL + i];
+        if (HASV) dv[o + i] = svl[i];
       }
-      continue;
+      __syncthreads();
     }
-    uint32_t P = 1;
-    while (P < m) P <<= 1;
-    for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) {
-      const bool in = i < m;
-#pragma unroll
-      for (int j = 0; j < NL; j++) sk[j * BS_LOCAL + i] = in ? T.p[j][o + i] : ~0ULL;
-      if (HASV) svl[i] = in ? tv[o + i] : 0u;
-    }
-    __syncthreads();
-    for (uint32_t kk = 2; kk <= P; kk <<= 1) {
-      for (uint32_t j = kk >> 1; j > 0; j >>= 1) {
-        for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) {
-          const uint32_t x = i ^ j;
-          if (x <= i) continue;
-          // a > b on the limbs, most significant first
-          bool gt = false, eq = true;
-#pragma unroll
-          for (int q = NL - 1; q >= 0; q--) {
-            const uint64_t u = sk[q * BS_LOCAL + i], v = sk[q * BS_LOCAL + x];
-            if (eq && u != v) {
-              gt = u > v;
-              eq = false;
-            }
-          }
-          const bool up = (i & kk) == 0;
-          if (gt == up && !eq) {
-#pragma unroll
-            for (int q = 0; q < NL; q++) {
-              const uint64_t t = sk[q * BS_LOCAL + i];
-              sk[q * BS_LOCAL + i] = sk[q * BS_LOCAL + x];
-              sk[q * BS_LOCAL + x] = t;
-            }
-            if (HASV) {
-              const uint32_t t = svl[i];
-              svl[i] = svl[x];
-              svl[x] = t;
-            }
-          }
-        }
-        __syncthreads();
-      }
-    }
-    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-#pragma unroll
-      for (int j = 0; j < NL; j++) D.p[j][o + i] = sk[j * BS_LOCAL + i];
-      if (HASV) dv[o + i] = svl[i];
-    }
-    __syncthreads();
+    __syncthreads();  // s_mid is reused
   }
 }
 
@@ -521,40 +645,49 @@ static void launch_segments(cudaStream_t st, bool hasv, Limbs L, uint32_t* lv, L
 
 template <int NL, bool HASV>
 static int bs_launch(cudaStream_t st, Limbs K, uint32_t* v, Limbs T, uint32_t* tv, uint64_t n,
-                     const unsigned long long* n_dev, unsigned limb, unsigned sh, uint32_t nb,
-                     uint32_t* hist, uint32_t* off, uint32_t* cur, uint32_t* big, unsigned* nbig,
-                     uint32_t* launches) {
+                     const unsigned long long* n_dev, unsigned nbits, const BsWork& W, uint32_t* launches) {
   const int sms = current_sm_count();
+  const uint32_t nb = bs_max_buckets(n);
   const unsigned g = (unsigned)std::max<uint64_t>(
       std::min<uint64_t>((n + BS_BLOCK - 1) / BS_BLOCK, (uint64_t)sms * 16), 1);
-  k_bs_hist<NL><<<g, BS_BLOCK, 0, st>>>(K, n, n_dev, limb, sh, nb, hist);
-  SPK_CUDA(cudaMemcpyAsync(off, hist, (size_t)nb * 4, cudaMemcpyDeviceToDevice, st));
+  // (a CTA of the coarse count flushes its 4,096 bins: a few CTAs per SM)
+  const unsigned gc = (unsigned)std::max<uint64_t>(std::min<uint64_t>(n / 4096, (uint64_t)sms * 4), 1);
+  k_bs_coarse<NL><<<gc, BS_BLOCK, 0, st>>>(K, n, n_dev, nbits, W);
+  k_bs_hist<NL><<<g, BS_BLOCK, 0, st>>>(K, n, n_dev, nbits, W);
   DevBuf sums;
   int rc;
-  if ((rc = scan_u32(st, off, nb, sums, launches))) return rc;
-  SPK_CUDA(cudaMemcpyAsync(cur, off, (size_t)nb * 4, cudaMemcpyDeviceToDevice, st));
-  k_bs_scatter<NL, HASV><<<g, BS_BLOCK, 0, st>>>(K, v, T, tv, n, n_dev, limb, sh, nb, cur);
-  const size_t smem = std::max<size_t>(BS_LOCAL * (NL * 8 + (HASV ? 4 : 0)),
-                                       (size_t)(BS_BLOCK / 32) * BS_WARP * (NL + (HASV ? 1 : 0)) * 8);
+  if ((rc = scan_u32(st, W.off, nb, sums, launches))) return rc;
+  k_bs_scatter<NL, HASV><<<g, BS_BLOCK, 0, st>>>(K, v, T, tv, n, n_dev, nbits, W);
+  const size_t smem = BS_LOCAL * (NL * 8 + (HASV ? 4 : 0));
   if ((rc = raise_smem_limit((const void*)k_bs_local<NL, HASV>, smem))) return rc;
-  const unsigned gl = (unsigned)std::min<uint32_t>(nb, (uint32_t)sms * 4);
-  k_bs_local<NL, HASV><<<gl, BS_BLOCK, smem, st>>>(T, tv, K, v, off, hist, nb, big, nbig);
+  const unsigned gl = (unsigned)std::min<uint32_t>((nb + BS_CHUNK - 1) / BS_CHUNK, (uint32_t)sms * 8);
+  k_bs_local<NL, HASV><<<gl, BS_BLOCK, smem, st>>>(T, tv, K, v, W);
   SPK_CUDA(cudaGetLastError());
-  if (launches) *launches += 3;
+  if (launches) *launches += 4;
   return SPK_OK;
+}
+static int bs_launch_nl(int nl, bool hasv, cudaStream_t st, Limbs K, uint32_t* v, Limbs T, uint32_t* tv,
+                        uint64_t n, const unsigned long long* n_dev, unsigned nbits, const BsWork& W,
+                        uint32_t* launches) {
+  switch (nl * 2 + (hasv ? 1 : 0)) {
+    case 2: return bs_launch<1, false>(st, K, v, T, tv, n, n_dev, nbits, W, launches);
+    case 3: return bs_launch<1, true>(st, K, v, T, tv, n, n_dev, nbits, W, launches);
+    case 4: return bs_launch<2, false>(st, K, v, T, tv, n, n_dev, nbits, W, launches);
+    case 5: return bs_launch<2, true>(st, K, v, T, tv, n, n_dev, nbits, W, launches);
+    case 6: return bs_launch<3, false>(st, K, v, T, tv, n, n_dev, nbits, W, launches);
+    case 7: return bs_launch<3, true>(st, K, v, T, tv, n, n_dev, nbits, W, launches);
+    case 8: return bs_launch<4, false>(st, K, v, T, tv, n, n_dev, nbits, W, launches);
+    default: return bs_launch<4, true>(st, K, v, T, tv, n, n_dev, nbits, W, launches);
+  }
 }
 
 int sort_bufs(cudaStream_t st, int nl, uint64_t n, unsigned nbits, DevBuf* keys, DevBuf* vals,
               uint64_t* h_staging, uint32_t* launches) {
-  // ~128 items per bucket (a few bitonic stages each), 2^8 to 2^16 buckets
-  uint32_t bbits = 8;
-  while (bbits < BS_MAX_BITS && (n >> (bbits + 1)) >= 128) bbits++;
-  const uint32_t nb = 1u << bbits;
-  if (n < (1u << 18) || nbits < bbits + 8 || !h_staging)
-    return radix_sort_bufs(st, nl, n, nbits, keys, vals, launches);
+  if (n <= 1) return SPK_OK;
+  if (!h_staging) return radix_sort_bufs(st, nl, n, nbits, keys, vals, launches);
   if (n >= (1ULL << 32)) return fail(SPK_E_INVALID_ARG, "sort: more than 2^32 items");
   int rc;
-  DevBuf tk[4], tv, hist, off, cur, big;
+  DevBuf tk[4], tv, work;
   Limbs K{}, T{};
   for (int j = 0; j < nl; j++) {
     if ((rc = tk[j].alloc(n * 8, st))) return rc;
@@ -562,32 +695,14 @@ int sort_bufs(cudaStream_t st, int nl, uint64_t n, unsigned nbits, DevBuf* keys,
     T.p[j] = tk[j].as<uint64_t>();
   }
   if (vals && (rc = tv.alloc(n * 4, st))) return rc;
-  if ((rc = hist.alloc(nb * 4, st)) || (rc = off.alloc(nb * 4, st)) || (rc = cur.alloc(nb * 4, st)) ||
-      (rc = big.alloc((3 * BS_MAX_BIG + 1) * 4, st)))
-    return rc;
-  SPK_CUDA(cudaMemsetAsync(hist.p, 0, nb * 4, st));
-  unsigned* nbig = (unsigned*)(big.as<uint32_t>() + 3 * BS_MAX_BIG);
-  SPK_CUDA(cudaMemsetAsync(nbig, 0, 4, st));
-  const unsigned hi_bit = nbits - bbits, limb = hi_bit / 64, sh = hi_bit % 64;
+  if ((rc = work.alloc(bs_work_bytes(n), st))) return rc;
+  SPK_CUDA(cudaMemsetAsync(work.p, 0, bs_work_bytes(n), st));
+  const BsWork W = bs_work(work.as<uint32_t>());
   uint32_t* v = vals ? vals->as<uint32_t>() : nullptr;
   uint32_t* tvp = vals ? tv.as<uint32_t>() : nullptr;
-  uint32_t* H = hist.as<uint32_t>();
-  uint32_t* O = off.as<uint32_t>();
-  uint32_t* Cu = cur.as<uint32_t>();
-  uint32_t* B = big.as<uint32_t>();
-  switch (nl * 2 + (vals ? 1 : 0)) {
-    case 2: rc = bs_launch<1, false>(st, K, v, T, tvp, n, nullptr, limb, sh, nb, H, O, Cu, B, nbig, launches); break;
-    case 3: rc = bs_launch<1, true>(st, K, v, T, tvp, n, nullptr, limb, sh, nb, H, O, Cu, B, nbig, launches); break;
-    case 4: rc = bs_launch<2, false>(st, K, v, T, tvp, n, nullptr, limb, sh, nb, H, O, Cu, B, nbig, launches); break;
-    case 5: rc = bs_launch<2, true>(st, K, v, T, tvp, n, nullptr, limb, sh, nb, H, O, Cu, B, nbig, launches); break;
-    case 6: rc = bs_launch<3, false>(st, K, v, T, tvp, n, nullptr, limb, sh, nb, H, O, Cu, B, nbig, launches); break;
-    case 7: rc = bs_launch<3, true>(st, K, v, T, tvp, n, nullptr, limb, sh, nb, H, O, Cu, B, nbig, launches); break;
-    case 8: rc = bs_launch<4, false>(st, K, v, T, tvp, n, nullptr, limb, sh, nb, H, O, Cu, B, nbig, launches); break;
-    default: rc = bs_launch<4, true>(st, K, v, T, tvp, n, nullptr, limb, sh, nb, H, O, Cu, B, nbig, launches); break;
-  }
-  if (rc) return rc;
+  if ((rc = bs_launch_nl(nl, vals != nullptr, st, K, v, T, tvp, n, nullptr, nbits, W, launches))) return rc;
   uint64_t* hs = h_staging + BS_STAGE_WORDS;
-  SPK_CUDA(cudaMemcpyAsync(hs, nbig, 4, cudaMemcpyDeviceToHost, st));
+  SPK_CUDA(cudaMemcpyAsync(hs, W.nbig, 4, cudaMemcpyDeviceToHost, st));
   SPK_CUDA(cudaStreamSynchronize(st));
   const unsigned nbig_h = ((unsigned*)hs)[0];
   if (nbig_h > BS_MAX_BIG) {
@@ -598,7 +713,7 @@ int sort_bufs(cudaStream_t st, int nl, uint64_t n, unsigned nbits, DevBuf* keys,
     return radix_sort_bufs(st, nl, n, nbits, keys, vals, launches);
   }
   if (nbig_h == 0) return SPK_OK;
-  SPK_CUDA(cudaMemcpyAsync(hs, B, (size_t)nbig_h * 12, cudaMemcpyDeviceToHost, st));
+  SPK_CUDA(cudaMemcpyAsync(hs, W.big, (size_t)nbig_h * 12, cudaMemcpyDeviceToHost, st));
   SPK_CUDA(cudaStreamSynchronize(st));
   std::vector<uint32_t> bl((const uint32_t*)hs, (const uint32_t*)hs + 3 * nbig_h);
   for (unsigned q = 0; q < nbig_h; q++) {
@@ -612,7 +727,7 @@ int sort_bufs(cudaStream_t st, int nl, uint64_t n, unsigned nbits, DevBuf* keys,
       if ((rc = bvv.alloc(m * 4, st))) return rc;
       SPK_CUDA(cudaMemcpyAsync(bvv.p, tvp + o, m * 4, cudaMemcpyDeviceToDevice, st));
     }
-    if ((rc = radix_sort_bufs(st, nl, m, hi_bit, bk, vals ? &bvv : nullptr, launches))) return rc;
+    if ((rc = radix_sort_bufs(st, nl, m, nbits, bk, vals ? &bvv : nullptr, launches))) return rc;
     for (int j = 0; j < nl; j++)
       SPK_CUDA(cudaMemcpyAsync(K.p[j] + o, bk[j].p, m * 8, cudaMemcpyDeviceToDevice, st));
     if (vals) SPK_CUDA(cudaMemcpyAsync(v + o, bvv.p, m * 4, cudaMemcpyDeviceToDevice, st));
@@ -629,14 +744,9 @@ int sort_bufs(cudaStream_t st, int nl, uint64_t n, unsigned nbits, DevBuf* keys,
 int sort_dev_enqueue(cudaStream_t st, int nl, uint64_t n_cap, const unsigned long long* n_dev,
                      unsigned nbits, DevBuf* keys, DevBuf* vals, DevBuf* tmp_keys, DevSort& ds,
                      uint32_t* launches) {
-  uint32_t bbits = 8;
-  while (bbits < BS_MAX_BITS && (n_cap >> (bbits + 1)) >= 128) bbits++;
-  if (nbits < bbits + 8) return fail(SPK_E_INVALID_ARG, "device-count sort: keys too short");
   if (n_cap >= (1ULL << 32)) return fail(SPK_E_INVALID_ARG, "sort: more than 2^32 items");
-  const uint32_t nb = 1u << bbits;
   ds.nl = nl;
   ds.nbits = nbits;
-  ds.bbits = bbits;
   ds.n_cap = n_cap;
   ds.has_vals = vals != nullptr;
   int rc;
@@ -648,36 +758,19 @@ int sort_dev_enqueue(cudaStream_t st, int nl, uint64_t n_cap, const unsigned lon
     T.p[j] = ds.tk[j].as<uint64_t>();
   }
   if (vals && (rc = ds.tv.alloc(std::max<uint64_t>(n_cap, 1) * 4, st))) return rc;
-  if ((rc = ds.hist.alloc(nb * 4, st)) || (rc = ds.off.alloc(nb * 4, st)) || (rc = ds.cur.alloc(nb * 4, st)) ||
-      (rc = ds.big.alloc((3 * BS_MAX_BIG + 1) * 4, st)))
-    return rc;
-  SPK_CUDA(cudaMemsetAsync(ds.hist.p, 0, nb * 4, st));
-  unsigned* nbig = (unsigned*)(ds.big.as<uint32_t>() + 3 * BS_MAX_BIG);
-  SPK_CUDA(cudaMemsetAsync(nbig, 0, 4, st));
-  const unsigned hi_bit = nbits - bbits, limb = hi_bit / 64, sh = hi_bit % 64;
+  if ((rc = ds.work.alloc(bs_work_bytes(n_cap), st))) return rc;
+  SPK_CUDA(cudaMemsetAsync(ds.work.p, 0, bs_work_bytes(n_cap), st));
   uint32_t* v = vals ? vals->as<uint32_t>() : nullptr;
   uint32_t* tvp = vals ? ds.tv.as<uint32_t>() : nullptr;
-  uint32_t* H = ds.hist.as<uint32_t>();
-  uint32_t* O = ds.off.as<uint32_t>();
-  uint32_t* Cu = ds.cur.as<uint32_t>();
-  uint32_t* B = ds.big.as<uint32_t>();
-  switch (nl * 2 + (vals ? 1 : 0)) {
-    case 2: rc = bs_launch<1, false>(st, K, v, T, tvp, n_cap, n_dev, limb, sh, nb, H, O, Cu, B, nbig, launches); break;
-    case 3: rc = bs_launch<1, true>(st, K, v, T, tvp, n_cap, n_dev, limb, sh, nb, H, O, Cu, B, nbig, launches); break;
-    case 4: rc = bs_launch<2, false>(st, K, v, T, tvp, n_cap, n_dev, limb, sh, nb, H, O, Cu, B, nbig, launches); break;
-    case 5: rc = bs_launch<2, true>(st, K, v, T, tvp, n_cap, n_dev, limb, sh, nb, H, O, Cu, B, nbig, launches); break;
-    case 6: rc = bs_launch<3, false>(st, K, v, T, tvp, n_cap, n_dev, limb, sh, nb, H, O, Cu, B, nbig, launches); break;
-    case 7: rc = bs_launch<3, true>(st, K, v, T, tvp, n_cap, n_dev, limb, sh, nb, H, O, Cu, B, nbig, launches); break;
-    case 8: rc = bs_launch<4, false>(st, K, v, T, tvp, n_cap, n_dev, limb, sh, nb, H, O, Cu, B, nbig, launches); break;
-    default: rc = bs_launch<4, true>(st, K, v, T, tvp, n_cap, n_dev, limb, sh, nb, H, O, Cu, B, nbig, launches); break;
-  }
-  if (rc) return rc;
+  if ((rc = bs_launch_nl(nl, vals != nullptr, st, K, v, T, tvp, n_cap, n_dev, nbits,
+                         bs_work(ds.work.as<uint32_t>()), launches)))
+    return rc;
   ds.pending = true;
   return SPK_OK;
 }
 
 const unsigned* sort_dev_nbig(const DevSort& ds) {
-  return (const unsigned*)(ds.big.as<uint32_t>() + 3 * BS_MAX_BIG);
+  return bs_work(ds.work.as<uint32_t>()).nbig;
 }
 
 // Sorts the buckets sort_dev_enqueue left over (nbig_host of them, read
@@ -704,7 +797,8 @@ int sort_dev_finish(cudaStream_t st, DevSort& ds, DevBuf* keys, DevBuf* vals, ui
     // their whole keys (their top bits keep the buckets apart), then put
     // back: one sort however many buckets there are.
     uint32_t* hs = (uint32_t*)(h_staging + BS_STAGE_WORDS);
-    SPK_CUDA(cudaMemcpyAsync(hs, ds.big.p, (size_t)nbig_host * 12, cudaMemcpyDeviceToHost, st));
+    uint32_t* seg = bs_work(ds.work.as<uint32_t>()).big;
+    SPK_CUDA(cudaMemcpyAsync(hs, seg, (size_t)nbig_host * 12, cudaMemcpyDeviceToHost, st));
     SPK_CUDA(cudaStreamSynchronize(st));
     std::vector<std::pair<uint32_t, uint32_t>> segs(nbig_host);  // (offset in the list, size)
     for (unsigned q = 0; q < nbig_host; q++) segs[q] = {hs[3 * q + 1], hs[3 * q + 2]};
@@ -716,7 +810,6 @@ int sort_dev_finish(cudaStream_t st, DevSort& ds, DevBuf* keys, DevBuf* vals, ui
       hs[3 * q + 2] = segs[q].second;
       total += segs[q].second;
     }
-    uint32_t* seg = ds.big.as<uint32_t>();
     SPK_CUDA(cudaMemcpyAsync(seg, hs, (size_t)nbig_host * 12, cudaMemcpyHostToDevice, st));
     DevBuf ck[4], cvb;
     Limbs L{}, Cc{};

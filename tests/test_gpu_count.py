@@ -662,3 +662,33 @@ def test_span_groups_equal_one_pass(spk, ora, k):
         np.testing.assert_array_equal(dc, tc[tc >= 2])
         r.close()
         d.close()
+
+
+@pytest.mark.parametrize("k,base", [(31, 0), (55, 0), (55, 1), (77, 1), (127, 0), (5, 0)])
+def test_sort_buckets_of_every_size(spk, ora, k, base):
+    """The bucketed sort of the list and the edges with buckets of every size
+    class: 3,000 and 500 k-mers that share their first 22 bases (one bucket
+    past the shared-memory size, one sorted by a CTA), 100 and 50 (one warp,
+    several per lane), beside even ones; on a short list (base 0: the sample
+    alone) and on one of hundreds of thousands (base 1: a GC-poor genome)."""
+    from spk import synth
+    rng = np.random.default_rng(k)
+    rows = []
+    for n, first in ((3000, 0), (500, 1), (100, 2), (50, 1)):
+        pre = np.concatenate([[0, 0, 0, first], rng.integers(0, 4, 18)]).astype(np.uint8)
+        for _ in range(n):
+            r = np.concatenate([pre, rng.integers(0, 4, max(k - 22, 0), dtype=np.uint8)])[:max(k, 22)]
+            rows += [r, r]  # twice, so that the k-mer is listed (count >= 2)
+    data, offs, lens = _pack_codes(rows)
+    if base:
+        p = synth.sample(250_000, 30.0, seed=7, gc=0.25, err=(0.002, 0.002), ks=(k,)).packed
+        offs = np.concatenate([p.offsets, offs + np.uint64(p.data.size)])
+        data, lens = np.concatenate([p.data, data]), np.concatenate([p.lengths, lens])
+    ref = ora.count(data, offs, lens, k, 1 << 26, mode=ora.MODE_TWICE, keep_bloom=False)
+    tk, tc = ref.table(2)
+    r = spk.count((data, offs, lens), [k], bloom_bits=1 << 26)
+    gk, gc = r.kmers(0)
+    np.testing.assert_array_equal(gk, tk)
+    np.testing.assert_array_equal(gc, tc)
+    sk, _ = r.solid(0)
+    np.testing.assert_array_equal(r.edges(0), ora.edges(sk, k))
