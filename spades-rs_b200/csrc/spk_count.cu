@@ -1318,12 +1318,15 @@ constexpr bool kSortedOps = SPK_SORTED_OPS;
 template <int NL>
 __device__ __forceinline__ void span_emit_sorted(const typename SpanKey<NL>::T* keys, uint32_t* buf, uint32_t S,
                                                  uint32_t* rs, uint32_t* rcur,
-                                                 const unsigned long long* rbase, const RangeView& rv) {
+                                                 const unsigned long long* rbase, const RangeView& rv,
+                                                 const uint16_t* used = nullptr, uint32_t nused = 0) {
   __shared__ uint32_t wpart[32], wmax[32], bnd[8];
   __shared__ uint32_t s_total, s_maxc;
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const uint32_t nr = rv.nranges;
   const uint32_t mask = (1u << kLog2Range) - 1u;
+  // the span's slots, or the `nused` of them that hold a key
+  const uint32_t nslots = used ? nused : S;
   // counts -> starts (exclusive scan in place), their total and largest count
   const uint32_t per = (nr + blockDim.x - 1) / blockDim.x;
   const uint32_t r0 = min(nr, threadIdx.x * per), r1 = min(nr, r0 + per);
@@ -1365,17 +1368,17 @@ __device__ __forceinline__ void span_emit_sorted(const typename SpanKey<NL>::T* 
   const uint32_t total = s_total, H = s_maxc <= (S >> 1) ? S - s_maxc : 0u;
   if (H == 0) {
     // direct emission (a range holds more than half a span's worth)
-    for (uint32_t s = threadIdx.x; s < S; s += blockDim.x) {
-      const uint32_t* st = (const uint32_t*)&keys[s];
-      if (st[1] == 0xFFFFFFFFu) continue;  // empty slot
+    for (uint32_t i = threadIdx.x; i < nslots; i += blockDim.x) {
+      const uint32_t* st = (const uint32_t*)&keys[used ? used[i] : i];
+      if (!used && st[1] == 0xFFFFFFFFu) continue;  // empty slot
       const uint32_t flag = st[0] >> 31;
       const uint32_t pk[3] = {st[0] & 0x7FFFFFFFu, st[1], st[2]};
 #pragma unroll
       for (int j = 0; j < 3; j++) {
         const uint32_t r = pk[j] >> kLog2Range;
-        const uint64_t i = rbase[r] + atomicAdd(rcur + r, 1u);
+        const uint64_t q = rbase[r] + atomicAdd(rcur + r, 1u);
         const uint64_t end = rv.uniform ? (uint64_t)(r + 1) * rv.uniform : rv.base[r + 1];
-        if (i < end) rv.ops[i] = ((pk[j] & mask) << 1) | flag;
+        if (q < end) rv.ops[q] = ((pk[j] & mask) << 1) | flag;
         else atomicOr(rv.err, (int)kErrRange);
       }
     }
@@ -1397,9 +1400,9 @@ __device__ __forceinline__ void span_emit_sorted(const typename SpanKey<NL>::T* 
   __syncthreads();
   for (uint32_t g = 0; g < G; g++) {
     const uint32_t gb = g * H;
-    for (uint32_t s = threadIdx.x; s < S; s += blockDim.x) {
-      const uint32_t* st = (const uint32_t*)&keys[s];
-      if (st[1] == 0xFFFFFFFFu) continue;  // empty slot
+    for (uint32_t i = threadIdx.x; i < nslots; i += blockDim.x) {
+      const uint32_t* st = (const uint32_t*)&keys[used ? used[i] : i];
+      if (!used && st[1] == 0xFFFFFFFFu) continue;  // empty slot
       const uint32_t flag = st[0] >> 31;
       const uint32_t pk[3] = {st[0] & 0x7FFFFFFFu, st[1], st[2]};
 #pragma unroll
@@ -1443,6 +1446,10 @@ struct ListOut {
   unsigned long long* hist;     // kHistBins counts of the k-mers counted >= 2 times
   unsigned long long* occ2;     // occurrences of the k-mers counted >= 2 times
 };
+
+}  // namespace spk
+#include "spk_superk.cuh"
+namespace spk {
 
 template <int NL, bool OPS>
 __global__ void __launch_bounds__(kPartBlock, kPartCtasPerSm) k_part_count(PartView pv, TableView t, unsigned k,
@@ -2485,16 +2492,24 @@ __global__ void __launch_bounds__(kBlock) k_prior_inject(const uint8_t* __restri
   }
 }
 
-// Occurrences of a read set (sum of max(len - k + 1, 0)).
+// Occurrences of a read set (sum of max(len - k + 1, 0)), and its longest read
+// (nullable).
 __global__ void __launch_bounds__(kBlock) k_occ(const uint32_t* __restrict__ lengths, uint64_t n,
-                                               unsigned k, unsigned long long* __restrict__ out) {
+                                               unsigned k, unsigned long long* __restrict__ out,
+                                               unsigned long long* __restrict__ longest) {
   uint64_t s = 0;
+  uint32_t mx = 0;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t len = lengths[i];
     s += len >= k ? len - k + 1 : 0;
+    mx = max(mx, len);
   }
   warp_add_u64(out, s);
+  if (longest) {
+    mx = __reduce_max_sync(FULL, mx);
+    if ((threadIdx.x & 31) == 0 && mx) atomicMax(longest, (unsigned long long)mx);
+  }
 }
 
 // flag = 1 if some read starts before the end of the read before it (the
@@ -2913,7 +2928,7 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
   DevBuf sgl[4];           // list mode: keys of the k-mers counted once
   if (!gated) {
     // ---- fused: Bloom and the count of every k-mer in one pass ----
-    k_occ<<<grid_for(ctx, 2), kBlock, 0, st>>>(rv.lengths, rv.n_reads, k, su + S_OCC0);
+    k_occ<<<grid_for(ctx, 2), kBlock, 0, st>>>(rv.lengths, rv.n_reads, k, su + S_OCC0, nullptr);
     SPK_CUDA(cudaGetLastError());
     launches++;
     if ((rc = fetch(S_OCC0 + 1))) return rc;
@@ -3450,8 +3465,108 @@ struct SideStream {
   }
 };
 
+// The super-k-mer records of a read set, by bin, and the batches of bins.
+struct SkJob {
+  DevBuf recs, bstart;
+  uint32_t nbat = 0;
+};
+template <int R>
+static void launch_sk_reads(spk_ctx* ctx, cudaStream_t st, const ReadsView& rv, unsigned k, const SkStream& S,
+                            unsigned long long* occ) {
+  const int grid = grid_for(ctx, 8);
+  const uint64_t warps = (uint64_t)grid * (kSkReadBlock / 32);
+  const uint32_t rpw = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(rv.n_reads / (warps * 4), 1), 32);
+  k_sk_reads<R><<<grid, kSkReadBlock, 0, st>>>(rv, k, sk_m(k), rpw, S, occ);
+}
+// occ: the k-mer windows of the reads; longest: the longest read.
+template <int NL>
+static int sk_partition(spk_ctx* ctx, cudaStream_t st, const ReadsView& rv, unsigned k, uint64_t occ,
+                        uint64_t longest, bool per_chunk, int* errp, unsigned long long* occ_out,
+                        unsigned long long* fill, SkJob& sj, uint32_t* launches) {
+  const uint32_t m = sk_m(k), w = k - m + 1;
+  // m-mer positions a warp holds: the longest read's, if that is at most 256
+  // (else in segments of 256), and at least 32 windows' worth
+  const uint64_t want = std::max<uint64_t>(longest > m ? longest - m + 1 : 1, w + 31);
+  const uint32_t R = want <= 96 ? 3 : want <= 128 ? 4 : want <= 160 ? 5 : want <= 192 ? 6 : 8;
+  const uint32_t seg = 32 * R - w + 1;
+  // A random sequence has 2 / (w + 1) runs per window, every read and segment
+  // one more; a stream that overflows (sequences made of other things) sends
+  // the job to the general path.
+  uint32_t nbins = 4096;
+  while (nbins < kSkMaxBins && (uint64_t)nbins * 512 < occ) nbins *= 2;
+  const uint64_t warps = (uint64_t)grid_for(ctx, 8) * (kSkReadBlock / 32);
+  const uint64_t cap = (uint64_t)((double)occ * (2.8 / (w + 1) + 1.0 / seg)) + rv.n_reads + rv.n_reads / 2 +
+                       (rv.chunks ? rv.chunks->n : 1) * std::min<uint64_t>(warps, rv.n_reads) * kSkChunk + 4096;
+  if (cap >= (1ULL << 32)) return kNotThisPath;
+  // Windows per batch: what fits a table, or fewer so that every CTA has one
+  const uint32_t T = (uint32_t)std::min<uint64_t>(
+      SkShape<NL>::T, std::max<uint64_t>(occ / ((uint64_t)ctx->sm_count * SkShape<NL>::ctas), 1024));
+  sj.nbat = (uint32_t)(occ / T) + 1;
+  int rc;
+  DevBuf stream, bins, sums, base;
+  const uint32_t nchunks = (nbins + kSkBinChunk - 1) / kSkBinChunk;
+  if ((rc = stream.alloc(cap * 16, st)) || (rc = bins.alloc((uint64_t)nbins * 8, st)) ||
+      (rc = sums.alloc((uint64_t)nchunks * 16, st)) || (rc = base.alloc((uint64_t)nbins * 4, st)) ||
+      (rc = sj.bstart.alloc(((uint64_t)sj.nbat + 1) * 4, st)) || (rc = sj.recs.alloc(cap * 8, st)))
+    return rc;
+  SPK_CUDA(cudaMemsetAsync(bins.p, 0, (uint64_t)nbins * 8, st));
+  SkStream S{stream.as<uint4>(), cap, fill, bins.as<unsigned long long>(), nbins, errp};
+  auto reads = [&](const ReadsView& r) {
+    switch (R) {
+      case 3: launch_sk_reads<3>(ctx, st, r, k, S, occ_out); break;
+      case 4: launch_sk_reads<4>(ctx, st, r, k, S, occ_out); break;
+      case 5: launch_sk_reads<5>(ctx, st, r, k, S, occ_out); break;
+      case 6: launch_sk_reads<6>(ctx, st, r, k, S, occ_out); break;
+      default: launch_sk_reads<8>(ctx, st, r, k, S, occ_out); break;
+    }
+    ++*launches;
+  };
+  if (per_chunk) {
+    // the reads of each uploaded piece as soon as it is on the device
+    uint64_t r0 = 0;
+    for (int c = 0; c < rv.chunks->n; c++) {
+      SPK_CUDA(cudaStreamWaitEvent(st, rv.chunks->ready[c], 0));
+      const uint64_t r1 = std::min<uint64_t>(std::max<uint64_t>(rv.chunks->read_end[c], r0), rv.n_reads);
+      if (r1 > r0) {
+        ReadsView p = rv;
+        p.offsets += r0;
+        p.lengths += r0;
+        p.n_reads = r1 - r0;
+        reads(p);
+      }
+      r0 = r1;
+    }
+  } else {
+    if (rv.chunks) SPK_CUDA(cudaStreamWaitEvent(st, rv.chunks->ready[rv.chunks->n - 1], 0));
+    reads(rv);
+  }
+  k_sk_bins_reduce<<<nchunks, kSkBinBlock, 0, st>>>(S.bins, nbins, sums.as<unsigned long long>());
+  k_sk_bins_apply<<<nchunks, kSkBinBlock, 0, st>>>(S.bins, nbins, sums.as<unsigned long long>(), T, sj.nbat,
+                                                  base.as<uint32_t>(), sj.bstart.as<uint32_t>());
+  k_sk_place<<<grid_for(ctx, 8), 256, 0, st>>>(S, base.as<uint32_t>(), sj.recs.as<uint64_t>());
+  SPK_CUDA(cudaGetLastError());
+  *launches += 3;
+  return SPK_OK;
+}
+template <int NL>
+static int sk_count(spk_ctx* ctx, cudaStream_t st, const ReadsView& rv, const SkJob& sj,
+                    unsigned long long* next_batch, unsigned k, const FastMod& fm, const RangeView& bv,
+                    const ListOut& lo, int* errp) {
+  const SkStage g = sk_stage<NL>(k, bv.nranges);
+  int rc;
+  if ((rc = raise_smem_limit((const void*)k_sk_count<NL>, g.smem))) return rc;
+  const int grid = (int)std::min<uint64_t>(sj.nbat, (uint64_t)ctx->sm_count * SkShape<NL>::ctas);
+  k_sk_count<NL><<<grid, SkShape<NL>::threads, g.smem, st>>>(rv.words, sj.recs.as<uint64_t>(),
+                                                             sj.bstart.as<uint32_t>(), sj.nbat, next_batch, k, g.rc,
+                                                             g.dd, fm, bv, lo, errp);
+  SPK_CUDA(cudaGetLastError());
+  return SPK_OK;
+}
+
+// *slots (0: sized here) is the room for distinct k-mers; after kGrow it holds
+// what the super-k-mers' count found, or 0 when the table's spans ran out.
 int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& rv_in, unsigned k,
-                     const spk_count_opts& o, KResult& kr) {
+                     const spk_count_opts& o, uint64_t* slots, KResult& kr) {
   const int nl = (int)((k + 31) / 32);
   // (k = 96 fills its top limb, which the solid set's empty mark needs free)
   if (k < 12 || (nl >= 3 && 2 * k == 64u * nl)) return kNotThisPath;
@@ -3465,31 +3580,40 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   if (nranges > kMaxRanges) return kNotThisPath;
   int rc;
   DevBuf scratch;
-  constexpr int S_ORDER = S_WORDS;  // reads out of order (chunked upload)
-  if ((rc = scratch.alloc((S_WORDS + 1) * 8, st))) return rc;
+  // reads out of order (chunked upload); the longest read; super-k-mer stream
+  // entries and the next batch to count
+  constexpr int S_ORDER = S_WORDS, S_LONGEST = S_WORDS + 1, S_SKFILL = S_WORDS + 2, S_SKNEXT = S_WORDS + 3;
+  constexpr int kWords = S_WORDS + 4;
+  if ((rc = scratch.alloc(kWords * 8, st))) return rc;
   uint64_t* sw = scratch.as<uint64_t>();
-  SPK_CUDA(cudaMemsetAsync(sw, 0, (S_WORDS + 1) * 8, st));
+  SPK_CUDA(cudaMemsetAsync(sw, 0, kWords * 8, st));
   unsigned long long* su = (unsigned long long*)sw;
   // ---- the first readback: occurrences, which size the table ----
   Ev e0, e1, e2, e3, e4, e5, e6, kb0, kb1, kc0, kc1, ks0, ks1, ksm;
   SPK_CUDA(cudaEventRecord(e0.e, st));
-  k_occ<<<grid_for(ctx, 2), kBlock, 0, st>>>(rv_in.lengths, rv_in.n_reads, k, su + S_OCC0);
+  k_occ<<<grid_for(ctx, 2), kBlock, 0, st>>>(rv_in.lengths, rv_in.n_reads, k, su + S_OCC0, su + S_LONGEST);
   SPK_CUDA(cudaGetLastError());
   if (rv_in.chunks) {
     k_read_order<<<grid_for(ctx, 2), kBlock, 0, st>>>(rv_in.offsets, rv_in.lengths, rv_in.n_reads, su + S_ORDER);
     SPK_CUDA(cudaGetLastError());
-    SPK_CUDA(cudaMemcpyAsync(host + S_ORDER, sw + S_ORDER, 8, cudaMemcpyDeviceToHost, st));
   }
-  SPK_CUDA(cudaMemcpyAsync(host + S_OCC0, sw + S_OCC0, 8, cudaMemcpyDeviceToHost, st));
+  SPK_CUDA(cudaMemcpyAsync(host, sw, kWords * 8, cudaMemcpyDeviceToHost, st));
   SPK_CUDA(cudaStreamSynchronize(st));
   const uint64_t occ0 = host[S_OCC0];
   const bool per_chunk = rv_in.chunks && host[S_ORDER] == 0;
   uint64_t cap = o.table_log2 ? (1ULL << std::min<uint32_t>(o.table_log2, 40)) : list_capacity(occ0, nl);
+  cap = std::max(cap, *slots);
+  *slots = 0;
   const uint32_t log2span = part_log2span(nl);
   uint32_t log2cap = 0;
   while ((1ULL << log2cap) < cap) log2cap++;
-  if (log2cap <= log2span) return kNotThisPath;
-  const uint32_t log2parts = log2cap - log2span;
+  // Super-k-mers unless the caller sizes the table or the groups of spans: read
+  // sets of any size for k <= 63, and for wider keys those with spans enough for
+  // two partition levels (smaller ones count with global atomics).
+  bool superk = sk_fits(k) && !o.table_log2 && !o.span_groups_log2 && occ0 > 0 &&
+                (nl <= 2 || log2cap > log2span + kCoarseBits);
+  if (!superk && log2cap <= log2span) return kNotThisPath;
+  const uint32_t log2parts = log2cap > log2span ? log2cap - log2span : 0;
   // Span groups: a read set whose partition buffers (span regions and coarse
   // buckets, 2.6 keys per occurrence) would pass a quarter of the device is
   // partitioned and counted in 2^lg passes, each keeping the keys of one group
@@ -3503,8 +3627,9 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   while (lg < kMaxLog2Groups && part_bytes(lg) > ctx->total_mem / 4) lg++;
   if (part_bytes(lg) > ctx->total_mem / 4) return kNotThisPath;
   while (lg > 0 && log2parts - lg <= kCoarseBits) lg--;
-  if (!SPK_TWO_LEVEL || log2parts - lg <= kCoarseBits || log2parts - lg - kCoarseBits > kFineMaxBits ||
-      part_bytes(lg) > ctx->total_mem / 4)
+  superk = superk && lg == 0;  // (read sets that need groups take them)
+  if (!superk && (!SPK_TWO_LEVEL || log2parts - lg <= kCoarseBits || log2parts - lg - kCoarseBits > kFineMaxBits ||
+                  part_bytes(lg) > ctx->total_mem / 4))
     return kNotThisPath;
   // The span count holds at most one distinct k-mer per slot (a full span
   // sends the job back), so the singleton keys and the list, up to one entry
@@ -3513,7 +3638,6 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   // share of the distinct ones (the mid-job readback sends the job back if
   // it overflowed).
   const uint64_t lcap_ = lg ? cap >> 1 : cap, scap_ = cap;
-
   kr.k = k;
   kr.nl = nl;
   kr.num_words = num_words;
@@ -3568,14 +3692,30 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
 
   // ---- two-level read partition (k_part_coarse, k_part_fine) and span
   // count, once per group of spans ----
+  if (superk) {
+    SPK_CUDA(cudaEventRecord(ks0.e, st));
+    SkJob sj;
+    rc = SPK_NL_CALL(nl, sk_partition, ctx, st, rv, k, occ0, host[S_LONGEST], per_chunk, errp, su + S_OCC,
+                     su + S_SKFILL, sj, &launches);
+    if (rc) return rc;
+    SPK_CUDA(cudaEventRecord(ks1.e, st));
+    info.part_passes = 2;
+    info.span_groups = 1;
+    if ((rc = alloc_count_buffers())) return rc;
+    SPK_CUDA(cudaEventRecord(kc0.e, st));
+    rc = SPK_NL_CALL(nl, sk_count, ctx, st, rv, sj, su + S_SKNEXT, k, kr.fm, bv, lo, errp);
+    if (rc) return rc;
+    launches++;
+  }
   DevBuf base, fill, region;
+  DevBuf cbase, cfill, cregion, cfirst;
+  if (!superk) {
   const uint64_t per = occ0 / nparts;
   const uint64_t capu = nl >= 3 ? 2 * per + 512 : per + (per >> 1) + 256;
   if ((rc = base.alloc((nparts_g + 1) * 8, st)) || (rc = fill.alloc(nparts_g * 4 * kFillStride, st)) ||
       (rc = region.alloc(nparts_g * capu * nl * 8, st)))
     return rc;
   k_part_uniform<<<64, kBlock, 0, st>>>((uint32_t)nparts_g, capu, base.as<uint64_t>());
-  DevBuf cbase, cfill, cregion, cfirst;
   const uint64_t cper = (occ0 >> lg) / kCoarse;
   const uint64_t ccap = (cper + (cper >> 3) + 8192 + 1) & ~1ULL;  // even: chunks start 16-byte aligned
   if ((rc = cbase.alloc((kCoarse + 1) * 8, st)) || (rc = cfill.alloc(kCoarse * 4 * kFillStride, st)) ||
@@ -3639,6 +3779,7 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   launches++;
   }  // span groups
   launches += 2;  // k_part_uniform x 2
+  }  // !superk
   cregion.release();
   cbase.release();
   cfill.release();
@@ -3688,6 +3829,12 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   if (err & 4) return fail(SPK_E_INVALID_ARG, "a read extends past the end of the packed data");
   if (err & 2) return fail(SPK_E_TIMEOUT, "count table: claim wait timed out");
   if (err & (int)kErrStage) return fail(SPK_E_TIMEOUT, "partition: a staged copy never completed");
+  if (superk && !(err & (int)kErrRegion) && (host[S_LFILL] > lcap_ || host[S_LFILL + 1] > scap_)) {
+    // more distinct k-mers than the buffers were sized for (reads of low
+    // coverage or many errors): again with room for them
+    *slots = next_pow2(host[S_LFILL] + host[S_LFILL + 1]);
+    return kGrow;
+  }
   if (err & (kErrRegion | kErrRange)) return kRedo;  // an overflowed region
   if (err & 1) return kGrow;                           // a span with more distinct k-mers than slots
   info.occurrences = host[S_OCC];
@@ -3826,7 +3973,7 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   info.ms_bloom_kernel = ms_between(kb0, kb1);
   info.ms_count_kernel = ms_between(kc0, kc1);
   info.ms_scatter_kernel = ms_between(ks0, ks1);
-  info.ms_coarse_kernel = lg == 0 ? ms_between(ks0, ksm) : 0.f;
+  info.ms_coarse_kernel = lg == 0 && !superk ? ms_between(ks0, ksm) : 0.f;
   info.kernel_launches = launches;
   info.schedule = SPK_SCHEDULE_PARTITIONED;
   return SPK_OK;
@@ -3884,14 +4031,16 @@ static int count_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsVie
 // overflow there) the general one.
 static int count_k_job(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& rv, unsigned k,
                        const spk_count_opts& o, KResult& kr) {
-  int rc = count_one_k_list(ctx, st, host, rv, k, o, kr);
-  // A span with more distinct k-mers than slots: twice the slots, twice at most.
+  uint64_t slots = 0;
+  int rc = count_one_k_list(ctx, st, host, rv, k, o, &slots, kr);
+  // More distinct k-mers than the buffers hold: again with room for what the
+  // count found; a span with more than its slots: twice the slots, twice at most.
   for (uint32_t grow = 1; rc == kGrow && grow <= 2; grow++) {
     SPK_CUDA(cudaStreamSynchronize(st));  // the abandoned job's buffers are freed in stream order
     spk_count_opts og = o;
-    og.table_log2 = kr.table.log2cap + 1;
+    if (!slots) og.table_log2 = kr.table.log2cap + 1;
     kr = KResult();
-    rc = count_one_k_list(ctx, st, host, rv, k, og, kr);
+    rc = count_one_k_list(ctx, st, host, rv, k, og, &slots, kr);
     if (rc == SPK_OK) {
       kr.info.table_regrows = grow;
       return SPK_OK;

@@ -1,0 +1,828 @@
+// spk_superk.cuh -- the default job's partition by minimizer and the count of
+// its super-k-mers (included by spk_count.cu, which holds the span helpers).
+//
+// A read's k-mer windows are cut into super-k-mers: runs of consecutive windows
+// whose smallest hashed canonical m-mer (the minimizer; Roberts et al. 2004, Li
+// et al. 2013 for the partitioning) is the same.  All occurrences of a k-mer, on
+// either strand, have the same minimizer, so a bin of minimizers holds every
+// occurrence of its k-mers.  What moves to the bins is one 8-byte record per
+// super-k-mer (where it starts in the packed reads, how many windows it has)
+// instead of one 8- to 32-byte key per occurrence, twice: at k = 55 a record
+// stands for 20 windows.
+//
+//   k_sk_reads   one warp per read: hashed canonical m-mers, sliding minimum,
+//                a record per run to a stream, with its bin and its rank there
+//                (one atomic per record, which also sums the bin's windows)
+//   k_sk_bins_*  exact bin offsets, and the batches: runs of neighbouring bins
+//                with about T windows, so that every batch fits one CTA's table
+//   k_sk_place   the stream's records to their bins
+//   k_sk_count   one CTA per batch: gathers the records' bases, drops repeated
+//                super-k-mers, rolls the windows of the others and counts their
+//                k-mers in shared memory; then list, singletons and Bloom
+//                operations as k_part_count writes them
+//
+// Bins have exact sizes, so no read set overflows them; a batch with more
+// distinct k-mers than slots is counted in parts (by hash bits), alone.
+#pragma once
+
+namespace spk {
+
+constexpr uint32_t kSkChunk = 128;    // stream entries a warp reserves at a time
+constexpr int kSkReadBlock = 256;
+constexpr uint32_t kSkBinBlock = 256, kSkBinIpt = 16, kSkBinChunk = kSkBinBlock * kSkBinIpt;
+constexpr uint32_t kSkMaxBins = 1u << 22;
+constexpr uint32_t kSkWinBits = 36;   // bins: windows in the low bits, records above
+constexpr uint64_t kSkWinMask = (1ULL << kSkWinBits) - 1;
+
+// Length of the minimizers: 15 above 32 bases; 13 and 11 below, where a longer
+// one leaves fewer windows per super-k-mer.
+__host__ __device__ constexpr unsigned sk_m(unsigned k) { return k > 32 ? 15u : k >= 27 ? 13u : 11u; }
+// k this partition takes: windows of at least 11 m-mers, and for keys of several
+// limbs a spare top bit (the table's claim mark).
+__host__ constexpr bool sk_fits(unsigned k) { return k >= 21 && (k <= 32 || 2 * k < 64 * ((k + 31) / 32)); }
+
+struct SkStream {
+  uint4* rec;                 // x, y: record; z: bin; w: rank in the bin
+  uint64_t cap;
+  unsigned long long* fill;   // entries reserved (a record of no windows is a gap)
+  unsigned long long* bins;   // per bin: records << kSkWinBits | windows
+  uint32_t nbins;
+  int* err;
+};
+// A record: start (bases from the start of `words`) << 8 | windows (1..255).
+
+__device__ __forceinline__ uint32_t sk_hash(uint32_t c) {
+  uint32_t h = (c ^ 0x2545F491u) * 0x9E3779B1u;
+  h ^= h >> 15;
+  h *= 0x2C1B3C6Du;
+  h ^= h >> 13;
+  return h;
+}
+// (minimizers are small hashes: mixed again before they pick a bin)
+__device__ __forceinline__ uint32_t sk_bin(uint32_t h, uint32_t nbins) {
+  uint32_t g = h * 0x85EBCA6Bu;
+  g ^= g >> 16;
+  g *= 0x7FEB352Du;
+  g ^= g >> 15;
+  return __umulhi(g, nbins);
+}
+
+// One warp per read, 32 R m-mer positions at a time (position p of the segment
+// in register p / 32 of lane p % 32).  The sliding minimum over the w = k - m + 1
+// m-mers of a window doubles its reach with log2(w) exchanges of neighbours.
+// rpw: reads a warp takes at a time (at most 32).
+template <int R>
+__global__ void __launch_bounds__(kSkReadBlock) k_sk_reads(ReadsView rd, unsigned k, unsigned m, uint32_t rpw,
+                                                            SkStream S, unsigned long long* __restrict__ occ_out) {
+  const unsigned lane = threadIdx.x & 31;
+  const uint32_t w = k - m + 1, seg = 32 * R - w + 1;
+  const unsigned msh = 32 - 2 * m;
+  unsigned p2 = 1;  // largest power of two <= w
+  while (2 * p2 <= w) p2 *= 2;
+  const unsigned d = w - p2, dr = d >> 5, ds = d & 31;
+  uint64_t occ = 0;
+  uint64_t cur = 0;   // this warp's reserved stream entries
+  uint32_t rem = 0;
+  __shared__ uint2 s_runs[kSkReadBlock / 32][32 * R + 1];
+  uint2* runs = s_runs[threadIdx.x >> 5];
+  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  // Stream places of the lanes with `act` set.
+  auto place = [&](bool act) -> uint64_t {
+    const unsigned mask = __ballot_sync(FULL, act);
+    const uint32_t n = __popc(mask), t = __popc(mask & lanemask_lt());
+    uint64_t at = cur + t;
+    if (n > rem) {
+      unsigned long long nb = 0;
+      if (lane == 0) nb = atomicAdd(S.fill, (unsigned long long)kSkChunk);
+      nb = __shfl_sync(FULL, nb, 0);
+      if (t >= rem) at = nb + (t - rem);
+      cur = nb + (n - rem);
+      rem = kSkChunk - (n - rem);
+    } else {
+      cur += n;
+      rem -= n;
+    }
+    return at;
+  };
+  auto put = [&](uint64_t at, uint64_t base, uint32_t nw, uint32_t bin, uint32_t rank) {
+    if (at < S.cap) {
+      const uint64_t r = base << 8 | nw;
+      S.rec[at] = make_uint4((uint32_t)r, (uint32_t)(r >> 32), bin, rank);
+    } else {
+      atomicOr(S.err, (int)kErrRegion);
+    }
+  };
+  for (uint64_t b = warp * rpw; b < rd.n_reads; b += nwarps * rpw) {
+    uint32_t len = 0;
+    uint64_t off = 0;
+    if (lane < rpw && b + lane < rd.n_reads) {
+      len = __ldg(rd.lengths + b + lane);
+      off = __ldg(rd.offsets + b + lane);
+      if (off + ((uint64_t)len + 3) / 4 > rd.data_len) {  // src/packed_reads.rs:600-602
+        atomicOr(rd.err, 4);
+        len = 0;
+      }
+    }
+    for (uint32_t j = 0; j < rpw; j++) {
+      const uint32_t L = __shfl_sync(FULL, len, j);
+      if (L < k) continue;
+      const uint64_t base0 = 4 * (rd.byte_base + __shfl_sync(FULL, off, j));
+      const uint32_t nwin = L - k + 1;
+      occ += nwin;
+      for (uint32_t a = 0; a < nwin; a += seg) {
+        const uint32_t nw = min(seg, nwin - a), nm = nw + w - 1;
+        const uint64_t base = base0 + a, bit0 = 2 * base;
+        const unsigned s = (unsigned)(bit0 & 63);
+        const uint64_t* p = rd.words + (bit0 >> 6);
+        const uint32_t need = s + 2 * (nm + m - 1);  // bits from p that the segment covers
+        uint64_t A[R + 1];
+        {
+          uint64_t u = bswap64(__ldg(p));
+#pragma unroll
+          for (int r = 0; r <= R; r++) {
+            const uint64_t v = 64u * (r + 1) < need ? bswap64(__ldg(p + r + 1)) : 0ULL;
+            A[r] = shl2(u, v, s);
+            u = v;
+          }
+        }
+        uint32_t M[R], T[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          // the 16 bases from position 32 r + lane
+          const uint32_t x0 = (uint32_t)(A[r] >> 32), x1 = (uint32_t)A[r], x2 = (uint32_t)(A[r + 1] >> 32);
+          const uint32_t v = __funnelshift_l(lane < 16 ? x1 : x2, lane < 16 ? x0 : x1, (2 * lane) & 31) >> msh;
+          uint32_t z = __brev(~(v << msh) & (~0u << msh));  // the complement, bits reversed: low 2m bits
+          z = ((z >> 1) & 0x55555555u) | ((z & 0x55555555u) << 1);
+          const uint32_t h = sk_hash(min(v, z));
+          M[r] = 32u * r + lane < nm ? h : 0xFFFFFFFFu;
+        }
+#pragma unroll
+        for (unsigned e = 1; e <= 16; e *= 2) {
+          if (2 * e > w) break;
+#pragma unroll
+          for (int r = 0; r < R; r++) T[r] = __shfl_sync(FULL, M[r], (lane + e) & 31);
+#pragma unroll
+          for (int r = 0; r < R; r++)
+            M[r] = min(M[r], lane + e < 32 ? T[r] : r + 1 < R ? T[r + 1 < R ? r + 1 : r] : 0xFFFFFFFFu);
+        }
+        if (64 <= w) {
+#pragma unroll
+          for (int r = 0; r + 1 < R; r++) M[r] = min(M[r], M[r + 1]);
+        }
+        if (d) {
+#pragma unroll
+          for (int r = 0; r < R; r++) T[r] = __shfl_sync(FULL, M[r], (lane + ds) & 31);
+          if (dr == 0) {
+#pragma unroll
+            for (int r = 0; r < R; r++)
+              M[r] = min(M[r], lane + ds < 32 ? T[r] : r + 1 < R ? T[r + 1 < R ? r + 1 : r] : 0xFFFFFFFFu);
+          } else {
+#pragma unroll
+            for (int r = 0; r < R; r++)
+              M[r] = min(M[r], lane + ds < 32 ? (r + 1 < R ? T[r + 1 < R ? r + 1 : r] : 0xFFFFFFFFu)
+                                              : (r + 2 < R ? T[r + 2 < R ? r + 2 : r] : 0xFFFFFFFFu));
+          }
+        }
+        // runs of equal minima among the segment's nw windows: their first
+        // windows and minima side by side in shared memory, then a lane per run
+#pragma unroll
+        for (int r = 0; r < R; r++) T[r] = __shfl_sync(FULL, M[r], (lane + 31) & 31);
+        uint32_t nruns = 0;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          const uint32_t pv = lane ? T[r] : r ? T[r ? r - 1 : 0] : ~M[0];
+          const bool start = 32u * r + lane < nw && M[r] != pv;
+          const unsigned mk = __ballot_sync(FULL, start);
+          if (start) runs[nruns + __popc(mk & lanemask_lt())] = make_uint2(32u * r + lane, M[r]);
+          nruns += __popc(mk);
+        }
+        if (lane == 0) runs[nruns] = make_uint2(nw, 0);
+        __syncwarp();
+        for (uint32_t t0 = 0; t0 < nruns; t0 += 32) {
+          const uint32_t t = t0 + lane;
+          uint32_t at0 = 0, left = 0, bin = 0;
+          if (t < nruns) {
+            const uint2 q = runs[t];
+            at0 = q.x;
+            left = runs[t + 1].x - at0;
+            bin = sk_bin(q.y, S.nbins);
+          }
+          // (a run of more than w windows, a minimizer repeated in a tandem
+          // repeat, becomes several records)
+          do {
+            const uint32_t c = min(left, w);
+            uint32_t rank = 0;
+            if (c) rank = (uint32_t)(atomicAdd(S.bins + bin, (1ULL << kSkWinBits) | c) >> kSkWinBits);
+            const uint64_t at = place(c > 0);
+            if (c) put(at, base + at0, c, bin, rank);
+            at0 += c;
+            left -= c;
+          } while (__any_sync(FULL, left > 0));
+        }
+        __syncwarp();
+      }
+    }
+  }
+  for (uint32_t t = lane; t < rem; t += 32)
+    if (cur + t < S.cap) S.rec[cur + t] = make_uint4(0, 0, 0, 0);
+  if (lane == 0 && occ) atomicAdd(occ_out, (unsigned long long)occ);
+}
+
+// Sums of each chunk of bins: records, windows.
+__global__ void __launch_bounds__(kSkBinBlock) k_sk_bins_reduce(const unsigned long long* __restrict__ bins,
+                                                                 uint32_t n, unsigned long long* __restrict__ sums) {
+  __shared__ unsigned long long sr, sw;
+  if (threadIdx.x == 0) sr = sw = 0;
+  __syncthreads();
+  uint64_t r = 0, w = 0;
+  for (uint32_t j = 0; j < kSkBinIpt; j++) {
+    const uint32_t i = blockIdx.x * kSkBinChunk + j * kSkBinBlock + threadIdx.x;
+    const uint64_t v = i < n ? bins[i] : 0;
+    r += v >> kSkWinBits;
+    w += v & kSkWinMask;
+  }
+  warp_add_u64(&sr, r);
+  warp_add_u64(&sw, w);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    sums[2 * blockIdx.x] = sr;
+    sums[2 * blockIdx.x + 1] = sw;
+  }
+}
+
+// Each bin's first record (base) and each batch's (bstart[b], b = 0..nbat): a
+// batch is the bins whose windows start in [b T, (b + 1) T) of the prefix sum.
+__global__ void __launch_bounds__(kSkBinBlock) k_sk_bins_apply(const unsigned long long* __restrict__ bins,
+                                                                uint32_t n,
+                                                                const unsigned long long* __restrict__ sums,
+                                                                uint32_t T, uint32_t nbat,
+                                                                uint32_t* __restrict__ base,
+                                                                uint32_t* __restrict__ bstart) {
+  __shared__ unsigned long long pre[2];
+  __shared__ unsigned long long wr[kSkBinBlock / 32], ww[kSkBinBlock / 32];
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) pre[0] = pre[1] = 0;
+  __syncthreads();
+  {
+    uint64_t r = 0, w = 0;  // the chunks before this one
+    for (uint32_t c = threadIdx.x; c < blockIdx.x; c += kSkBinBlock) {
+      r += sums[2 * c];
+      w += sums[2 * c + 1];
+    }
+    warp_add_u64(&pre[0], r);
+    warp_add_u64(&pre[1], w);
+  }
+  const uint32_t i0 = blockIdx.x * kSkBinChunk + threadIdx.x * kSkBinIpt;
+  uint64_t v[kSkBinIpt], r = 0, w = 0;
+#pragma unroll
+  for (uint32_t j = 0; j < kSkBinIpt; j++) {
+    v[j] = i0 + j < n ? bins[i0 + j] : 0;
+    r += v[j] >> kSkWinBits;
+    w += v[j] & kSkWinMask;
+  }
+  uint64_t xr = r, xw = w;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint64_t yr = __shfl_up_sync(FULL, xr, d), yw = __shfl_up_sync(FULL, xw, d);
+    if ((int)lane >= d) {
+      xr += yr;
+      xw += yw;
+    }
+  }
+  if (lane == 31) {
+    wr[warp] = xr;
+    ww[warp] = xw;
+  }
+  __syncthreads();
+  uint64_t pr = pre[0] + xr - r, pw = pre[1] + xw - w;
+  for (unsigned q = 0; q < warp; q++) {
+    pr += wr[q];
+    pw += ww[q];
+  }
+  uint64_t prevw = (i0 > 0 && i0 <= n) ? bins[i0 - 1] & kSkWinMask : 0;
+#pragma unroll
+  for (uint32_t j = 0; j < kSkBinIpt; j++) {
+    const uint32_t i = i0 + j;
+    if (i >= n) break;
+    base[i] = (uint32_t)pr;
+    const uint32_t b1 = (uint32_t)(pw / T);
+    const uint32_t b0 = i ? (uint32_t)((pw - prevw) / T) + 1 : 0;
+    for (uint32_t b = b0; b <= b1 && b <= nbat; b++) bstart[b] = (uint32_t)pr;
+    prevw = v[j] & kSkWinMask;
+    pr += v[j] >> kSkWinBits;
+    pw += prevw;
+    if (i == n - 1)
+      for (uint32_t b = b1 + 1; b <= nbat; b++) bstart[b] = (uint32_t)pr;
+  }
+}
+
+// The stream's records to their bins.
+__global__ void __launch_bounds__(256) k_sk_place(SkStream S, const uint32_t* __restrict__ base,
+                                                   uint64_t* __restrict__ out) {
+  const uint64_t n = min((uint64_t)*S.fill, S.cap);
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
+       i += (uint64_t)gridDim.x * blockDim.x) {
+    const uint4 q = __ldcs(S.rec + i);
+    const uint64_t r = (uint64_t)q.y << 32 | q.x;
+    const uint64_t at = (r & 255) ? (uint64_t)__ldg(base + q.z) + q.w : S.cap;
+    if (at < S.cap) out[at] = r;  // (beyond it only after the stream overflowed: the job runs again)
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The count of a batch.
+// ---------------------------------------------------------------------------
+template <int NL>
+struct SkShape {
+  static constexpr int threads = NL <= 2 ? 512 : 256;
+  static constexpr int ctas = NL == 1 || NL == 3 ? 3 : 2;
+  static constexpr uint32_t log2s = NL <= 2 ? 12 : 11;
+  static constexpr uint32_t S = 1u << log2s;  // slots
+  // windows per batch: slots over the distinct share expected (0.27 of the
+  // occurrences at k = 55, 0.38 at 77, 0.52 at 127 on the reads of the benchmark)
+  static constexpr uint32_t T = NL <= 2 ? 7000 : NL == 3 ? 2700 : 2000;
+};
+// 32-bit words a record's bases take: at most w windows, w + k - 1 = 2k - m bases.
+__host__ __device__ __forceinline__ uint32_t sk_words(unsigned k) { return (2 * k - sk_m(k) + 15) / 16; }
+constexpr uint32_t kSkMaxRecs = 2048;  // a record's index takes 11 bits
+// Records staged at a time, and the entries (a power of two) of their table.
+struct SkStage {
+  uint32_t rc, dd;
+  size_t smem;
+};
+// Shared memory: keys, counts, used slots; then the staged records (bases,
+// multiplicities, the records' table or the live records, window counts) or,
+// while the batch is written out, the Bloom ranges' counts, cursors and places.
+// As many records are staged as leave room for the CTAs an SM is to hold.
+template <int NL>
+static SkStage sk_stage(unsigned k, uint32_t nranges) {
+  typedef SkShape<NL> P;
+  const size_t budget = (size_t)(228 * 1024) / P::ctas - 1024 - 2560;  // of one CTA, less its static arrays
+  const size_t table = (size_t)P::S * (8 * NL + 4 + 2);
+  const size_t nr2 = (nranges + 1) & ~1u;
+  const size_t ranges = nr2 * 4 * (NL >= 2 ? 2 : 1) + (size_t)nranges * 8;
+  auto bytes = [&](uint32_t rc, uint32_t dd) { return (size_t)rc * (4 * sk_words(k) + 4 + 1) + (size_t)dd * 4; };
+  SkStage g{128, 256, 0};
+  for (uint32_t rc = 128; rc <= kSkMaxRecs; rc += 64) {
+    uint32_t dd = 256;
+    while (dd < rc + rc / 4) dd *= 2;
+    if (table + bytes(rc, dd) <= budget) g = SkStage{rc, dd, 0};
+  }
+  g.smem = table + std::max(bytes(g.rc, g.dd), ranges);
+  return g;
+}
+
+// The slot hash (not the reference's: it never leaves the batch): a multilinear
+// sum over the key's 32-bit words, mixed.
+template <int NL>
+__device__ __forceinline__ uint32_t sk_key_hash(const Seq<NL>& C) {
+  uint32_t a = 0x9E3779B9u;
+  const uint32_t A[8] = {0x2C1B3C6Du, 0x297A2D39u, 0x85EBCA6Bu, 0xC2B2AE35u,
+                         0x27D4EB2Fu, 0x165667B1u, 0x7FEB352Du, 0x846CA68Bu};
+#pragma unroll
+  for (int j = 0; j < NL; j++) a += (uint32_t)C.v[j] * A[2 * j] + (uint32_t)(C.v[j] >> 32) * A[2 * j + 1];
+  a ^= a >> 16;
+  a *= 0x9E3779B1u;
+  return a ^ a >> 15;
+}
+
+__device__ __forceinline__ ulonglong2 lds2(const uint64_t* p) {
+  ulonglong2 v;
+  asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+  return v;
+}
+
+// A claimed slot's top limb carries this bit until the other limbs are written.
+constexpr uint64_t kSkBusy = 1ULL << 63;
+
+// One probe step of key C at slot kp: 1 = C's slot, 2 = claimed for C now,
+// 0 = another key's, 3 = being written by a key with C's top limb (look again).
+// Empty slots are all ones, which no key's top limb is.  The top limb is claimed
+// with one 64-bit CAS and published last.  (A 128-bit CAS of the whole key took
+// the place of the claim in k_part_count.)
+template <int NL>
+__device__ __forceinline__ int sk_step(uint64_t* kp, const Seq<NL>& C) {
+  volatile uint64_t* v = kp;
+  if constexpr (NL == 1) {
+    const uint64_t cur = v[0];
+    if (cur == C.v[0]) return 1;
+    if (cur != kEmpty) return 0;
+    const uint64_t old = atomicCAS((unsigned long long*)kp, (unsigned long long)kEmpty, (unsigned long long)C.v[0]);
+    return old == kEmpty ? 2 : old == C.v[0] ? 1 : 0;
+  } else {
+    const uint64_t mine = C.v[NL - 1];
+    uint64_t top, low = kEmpty;
+    if constexpr (NL == 2) {
+      const ulonglong2 q = lds2(kp);
+      low = q.x;
+      top = q.y;
+    } else {
+      top = v[NL - 1];
+    }
+    if (top == kEmpty) {
+      top = atomicCAS((unsigned long long*)(kp + NL - 1), (unsigned long long)kEmpty, (unsigned long long)(mine | kSkBusy));
+      if (top == kEmpty) {
+#pragma unroll
+        for (int j = 0; j < NL - 1; j++) v[j] = C.v[j];
+        __threadfence_block();
+        v[NL - 1] = mine;
+        return 2;
+      }
+      low = kEmpty;
+    }
+    if (top == (mine | kSkBusy)) return 3;
+    if (top != mine) return 0;
+    if constexpr (NL == 2) {
+      // (a low limb read before its write is all ones: read it again, after the top)
+      if (low == kEmpty) {
+        __threadfence_block();
+        low = v[0];
+      }
+      return low == C.v[0];
+    } else {
+      __threadfence_block();
+      bool eq = true;
+#pragma unroll
+      for (int j = 0; j < NL - 1; j++) eq &= v[j] == C.v[j];
+      return eq;
+    }
+  }
+}
+
+template <int NL>
+__global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
+    k_sk_count(const uint64_t* __restrict__ words, const uint64_t* __restrict__ recs,
+               const uint32_t* __restrict__ bstart, uint32_t nbat, unsigned long long* __restrict__ next_batch,
+               unsigned k, uint32_t RC, uint32_t DD, FastMod fm, RangeView rv, ListOut lo, int* __restrict__ err) {
+  typedef SkShape<NL> P;
+  typedef typename SpanKey<NL>::T KeyT;
+  constexpr uint32_t S = P::S;
+  constexpr int TH = P::threads, kWarps = TH / 32, kRounds = S / TH;
+  constexpr int W2 = 2 * NL;  // 32-bit words of a key
+  extern __shared__ __align__(16) unsigned char sk_smem_[];
+  uint64_t* keys = (uint64_t*)sk_smem_;
+  uint32_t* cnt = (uint32_t*)(keys + (size_t)S * NL);
+  uint16_t* used = (uint16_t*)(cnt + S);
+  unsigned char* uni = (unsigned char*)(used + S);
+  const uint32_t SW = sk_words(k);
+  uint32_t* seq = (uint32_t*)uni;        // word i (16 bases, the first on top) of record t: seq[i * RC + t]
+  uint32_t* mult = seq + (size_t)SW * RC;
+  uint32_t* dd = mult + RC;
+  uint32_t* lrec = dd;                   // live records: first window << 16 | record (over the records' table)
+  uint8_t* nws = (uint8_t*)(dd + DD);
+  uint32_t* rhist = (uint32_t*)uni;
+  const uint32_t nr2 = (rv.nranges + 1) & ~1u;
+  uint32_t* rcur = rhist + nr2;
+  unsigned long long* rbase = (unsigned long long*)(rcur + (NL >= 2 ? nr2 : 0u));
+  __shared__ uint32_t lw[2][kRounds * kWarps];
+  __shared__ uint32_t wsum[kWarps];
+  __shared__ unsigned long long lbase[2];
+  __shared__ unsigned s_hist[kHistBins];
+  __shared__ uint32_t s_batch, s_used, s_live;
+  __shared__ int s_full;
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t lmin = lo.lmin < 2 ? 2u : lo.lmin;
+  // a key's 2k bits at the top of W2 words: the bits below them, and their number
+  const uint32_t low = 64 * NL - 2 * k, lrot = low & 31;
+  const uint32_t mask1 = low >= 32 ? 0u : ~0u << lrot, mask2 = low >= 32 ? ~0u << lrot : ~0u;
+  uint64_t occ2 = 0;
+  if (*(volatile int*)err & (int)kErrRegion) return;  // the stream overflowed: records are missing
+  for (int i = threadIdx.x; i < kHistBins; i += TH) s_hist[i] = 0;
+  for (uint32_t i = threadIdx.x; i < S * NL; i += TH) keys[i] = kEmpty;
+  for (uint32_t i = threadIdx.x; i < S; i += TH) cnt[i] = 0;
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_batch = (uint32_t)min((unsigned long long)nbat, atomicAdd(next_batch, 1ULL));
+    __syncthreads();
+    const uint32_t bt = s_batch;
+    if (bt >= nbat) break;
+    const uint32_t r0 = bstart[bt], r1 = bstart[bt + 1];
+    if (r0 == r1) continue;
+    // The batch, or the part of it whose hash bits [0, depth) are `part`: a part
+    // with too many distinct k-mers for the table is cut in two.
+    uint32_t depth = 0, part = 0;
+    for (;;) {
+      if (threadIdx.x == 0) {
+        s_used = 0;
+        s_full = 0;
+      }
+      for (uint32_t q0 = r0; q0 < r1; q0 += RC) {
+        // ---- stage up to RC records: their bases, the first on top ----
+        __syncthreads();
+        if (*(volatile int*)&s_full) break;
+        const uint32_t n = min(RC, r1 - q0);
+        if (threadIdx.x == 0) s_live = 0;
+        for (uint32_t i = threadIdx.x; i < DD; i += TH) dd[i] = 0xFFFFFFFFu;
+        for (uint32_t t = threadIdx.x; t < n; t += TH) {
+          const uint64_t rec = __ldcs(recs + q0 + t);
+          const uint32_t nw = (uint32_t)(rec & 255);
+          const uint64_t bit0 = 2 * (rec >> 8);
+          const unsigned s = (unsigned)(bit0 & 63);
+          const uint64_t* p = words + (bit0 >> 6);
+          const uint32_t bits = 2 * (nw + k - 1);
+          uint64_t u = bswap64(__ldg(p));
+#pragma unroll
+          for (uint32_t i = 0; i < 2 * NL; i++) {
+            if (64 * i >= bits) break;
+            const uint64_t v = 64 * (i + 1) < s + bits ? bswap64(__ldg(p + i + 1)) : 0ULL;
+            uint64_t x = shl2(u, v, s);
+            u = v;
+            if (bits - 64 * i < 64) x &= ~(~0ULL >> (bits - 64 * i));  // nothing past the last base
+            seq[2 * i * RC + t] = (uint32_t)(x >> 32);
+            if (bits - 64 * i > 32) seq[(2 * i + 1) * RC + t] = (uint32_t)x;
+          }
+          nws[t] = (uint8_t)nw;
+          mult[t] = 1;
+        }
+        __syncthreads();
+        // ---- equal records become one with a multiplicity ----
+        uint32_t dead = 0;  // bit j: this thread's j-th record repeats another
+        for (uint32_t t = threadIdx.x, j = 0; t < n; t += TH, j++) {
+          const uint32_t nw = nws[t], words32 = (nw + k + 14) / 16;
+          uint32_t h = nw;
+          for (uint32_t i = 0; i < words32; i++) h = (h ^ seq[i * RC + t]) * 0x9E3779B1u + (h >> 15);
+          h ^= h >> 16;
+          h *= 0x7FEB352Du;
+          const uint32_t tag = h & ~(kSkMaxRecs - 1);
+          uint32_t at = (h ^ (h >> 13)) & (DD - 1);
+          for (;;) {
+            const uint32_t old = atomicCAS(dd + at, 0xFFFFFFFFu, tag | t);
+            if (old == 0xFFFFFFFFu) break;
+            if ((old & ~(kSkMaxRecs - 1)) == tag) {
+              const uint32_t o = old & (kSkMaxRecs - 1);
+              bool eq = nws[o] == nw;
+              for (uint32_t i = 0; eq && i < words32; i++) eq = seq[i * RC + o] == seq[i * RC + t];
+              if (eq) {
+                atomicAdd(mult + o, 1u);
+                dead |= 1u << j;
+                break;
+              }
+            }
+            at = (at + 1) & (DD - 1);
+          }
+        }
+        __syncthreads();  // (the records' table is done with: the live records take its place)
+        // ---- the live records side by side, with the windows before each ----
+        for (uint32_t t0 = 0, j = 0; t0 < n; t0 += TH, j++) {
+          const uint32_t t = t0 + threadIdx.x;
+          const bool live = t < n && !(dead >> j & 1);
+          const uint32_t lv = live ? 1u << 20 | nws[t] : 0u;  // (at most 2,048 records, 231,424 windows)
+          uint32_t x = lv;
+#pragma unroll
+          for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, x, d);
+            if ((int)lane >= d) x += y;
+          }
+          if (lane == 31) wsum[warp] = x;
+          __syncthreads();
+          const uint32_t before = s_live;
+          uint32_t at = before + x - lv, total = before;
+#pragma unroll
+          for (int q = 0; q < kWarps; q++) {
+            if (q < (int)warp) at += wsum[q];
+            total += wsum[q];
+          }
+          if (live) lrec[at >> 20] = (at & 0xFFFFF) << 11 | t;
+          __syncthreads();
+          if (threadIdx.x == 0) s_live = total;
+        }
+        __syncthreads();
+        const uint32_t nlive = s_live >> 20, nwin = s_live & 0xFFFFF;
+        // ---- count: each warp a share of the windows ----
+        // Lanes without a k-mer to place take the next windows, a dozen at a
+        // time at least; every turn is one probe step for the lanes that have
+        // one, so a long probe sequence holds up its own lane only.
+        {
+          const uint32_t share = (nwin + kWarps - 1) / kWarps;
+          uint32_t cur = warp * share;
+          const uint32_t end = min(nwin, cur + share);
+          uint32_t r = 0;  // the live record that holds window cur
+          for (uint32_t b = kSkMaxRecs / 2; b; b >>= 1)
+            if (r + b < nlive && (lrec[r + b] >> 11) <= cur) r += b;
+          bool pend = false;
+          Seq<NL> C;
+          uint32_t slot = 0, step = 0, waits = 0, mu = 0;
+#pragma unroll
+          for (int q = 0; q < NL; q++) C.v[q] = 0;
+          for (;;) {
+            const unsigned idle = __ballot_sync(FULL, !pend);
+            const uint32_t ni = __popc(idle);
+            if (cur < end && ni >= 12) {
+              // records that start among the next 32 windows
+              const uint32_t q = r + 1 + lane;
+              const uint32_t st = q < nlive ? (lrec[q] >> 11) - cur : 32u;
+              const unsigned mk = __reduce_or_sync(FULL, st < 32 ? 1u << st : 0u);
+              const uint32_t rank = __popc(idle & lanemask_lt()), taken = min(ni, end - cur);
+              if (!pend && rank < taken) {
+                const uint32_t e = lrec[r + __popc(mk & (unsigned)((2ULL << rank) - 1))];
+                const uint32_t rt = e & (kSkMaxRecs - 1), o = cur + rank - (e >> 11);
+                mu = mult[rt];
+                // the window's 2k bits at the top of L (words past the record are masked off)
+                const uint32_t* sq = seq + (o >> 4) * RC + rt;
+                const uint32_t sh = 2 * (o & 15);
+                uint32_t L[W2], u = sq[0];
+#pragma unroll
+                for (int i = 0; i < W2; i++) {
+                  const uint32_t v = sq[(i + 1) * RC];
+                  L[i] = __funnelshift_l(v, u, sh);
+                  u = v;
+                }
+                L[W2 - 1] &= mask1;
+                L[W2 - 2] &= mask2;
+                // its reverse complement at the bottom of G (word 0 most significant)
+                uint32_t G[W2], F[W2];
+#pragma unroll
+                for (int i = 0; i < W2; i++) {
+                  uint32_t z = ~L[W2 - 1 - i];
+                  if (i == 0) z &= mask1;
+                  if (i == 1) z &= mask2;
+                  z = __brev(z);
+                  G[i] = ((z >> 1) & 0x55555555u) | ((z & 0x55555555u) << 1);
+                }
+                // ... and the window at the bottom of F
+#pragma unroll
+                for (int i = W2 - 1; i >= 0; i--) {
+                  const uint32_t a = low >= 32 ? (i >= 1 ? L[i >= 1 ? i - 1 : 0] : 0u) : L[i];
+                  const uint32_t b = low >= 32 ? (i >= 2 ? L[i >= 2 ? i - 2 : 0] : 0u) : (i >= 1 ? L[i >= 1 ? i - 1 : 0] : 0u);
+                  F[i] = __funnelshift_r(a, b, lrot);
+                }
+                Seq<NL> V, Rc;
+#pragma unroll
+                for (int i = 0; i < NL; i++) {
+                  V.v[i] = (uint64_t)F[W2 - 2 - 2 * i] << 32 | F[W2 - 1 - 2 * i];
+                  Rc.v[i] = (uint64_t)G[W2 - 2 - 2 * i] << 32 | G[W2 - 1 - 2 * i];
+                }
+                C = seq_le<NL>(V, Rc) ? V : Rc;  // canonical, src/dna.rs:185-192
+                const uint32_t h = sk_key_hash<NL>(C);
+                slot = h >> (32 - P::log2s);
+                step = 0;
+                waits = 0;
+                pend = depth == 0 || (h & ((1u << depth) - 1)) == part;
+              }
+              r += __popc(mk & (unsigned)((2ULL << taken) - 1));
+              cur += taken;
+            }
+            if (!__any_sync(FULL, pend)) {
+              if (cur >= end) break;
+              continue;
+            }
+            const int got = pend ? sk_step<NL>(keys + (size_t)NL * slot, C) : -1;
+            const unsigned won = __ballot_sync(FULL, got == 2);
+            if (won) {
+              uint32_t u0 = 0;
+              if (lane == 0) u0 = atomicAdd(&s_used, (uint32_t)__popc(won));
+              u0 = __shfl_sync(FULL, u0, 0) + __popc(won & lanemask_lt());
+              if (got == 2 && u0 < S) used[u0] = (uint16_t)slot;
+              if (u0 >= S - S / 16) s_full = 1;
+            }
+            if (got == 1 || got == 2) {
+              atomicAdd(cnt + slot, mu);
+              pend = false;
+            } else if (got == 0) {
+              slot = (slot + ++step) & (S - 1);  // (triangular steps reach every slot)
+              if (step >= S) s_full = 1;
+              // (a full table's counts are dropped: no long probes for them)
+              if ((step & 31) == 0 && *(volatile int*)&s_full) pend = false;
+            } else if (got == 3 && ++waits > (uint32_t)kSpinLimit) {
+              atomicOr(err, 2);  // a claim that never settled: the job fails
+              pend = false;
+            }
+          }
+        }
+      }
+      __syncthreads();
+      const uint32_t n = min(s_used, S);
+      if (s_full) {
+        // too many distinct k-mers: this part again as two
+        for (uint32_t i = threadIdx.x; i < S * NL; i += TH) keys[i] = kEmpty;
+        for (uint32_t i = threadIdx.x; i < S; i += TH) cnt[i] = 0;
+        if (++depth > 16) {
+          if (threadIdx.x == 0) atomicOr(err, 1);
+          break;
+        }
+        __syncthreads();
+        continue;
+      }
+      // ---- write the part out ----
+      // Entries of each (round, warp) of the loop below: a ballot per round,
+      // then one reservation for the list and one for the singletons.
+      for (uint32_t i = threadIdx.x; i < rv.nranges; i += TH) {
+        rhist[i] = 0;
+        if (NL >= 2) rcur[i] = 0;
+      }
+      const uint32_t rounds = (n + TH - 1) / TH;
+      for (uint32_t r = 0; r < rounds; r++) {
+        const uint32_t i = r * TH + threadIdx.x;
+        const uint32_t c = i < n ? cnt[used[i]] : 0u;
+        const unsigned bl = __ballot_sync(FULL, c >= lmin), bs = __ballot_sync(FULL, c == 1);
+        if (lane == 0) {
+          lw[0][r * kWarps + warp] = __popc(bl);
+          lw[1][r * kWarps + warp] = __popc(bs);
+        }
+        if (c >= 2) {
+          atomicAdd(&s_hist[c < kHistBins - 1 ? c : kHistBins - 1], 1u);
+          occ2 += c;
+        }
+      }
+      __syncthreads();
+      if (warp < 2) {
+        const uint32_t m = rounds * kWarps;
+        uint32_t carry = 0;
+        for (uint32_t b = 0; b < m; b += 32) {
+          const uint32_t v = b + lane < m ? lw[warp][b + lane] : 0u;
+          uint32_t x = v;
+#pragma unroll
+          for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, x, d);
+            if ((int)lane >= d) x += y;
+          }
+          if (b + lane < m) lw[warp][b + lane] = carry + x - v;
+          carry += __shfl_sync(FULL, x, 31);
+        }
+        if (lane == 0) lbase[warp] = carry ? atomicAdd(lo.fill + warp, (unsigned long long)carry) : 0ULL;
+      }
+      __syncthreads();
+      for (uint32_t r = 0; r < rounds; r++) {
+        const uint32_t i = r * TH + threadIdx.x;
+        const uint32_t s = i < n ? used[i] : 0u;
+        const uint32_t c = i < n ? cnt[s] : 0u;
+        Seq<NL> C;
+#pragma unroll
+        for (int j = 0; j < NL; j++) C.v[j] = keys[(size_t)NL * s + j];
+        const unsigned bl = __ballot_sync(FULL, c >= lmin), bs = __ballot_sync(FULL, c == 1);
+        if (c >= lmin) {
+          const uint64_t q = lbase[0] + lw[0][r * kWarps + warp] + __popc(bl & lanemask_lt());
+          if (q < lo.cap) {
+#pragma unroll
+            for (int j = 0; j < NL; j++) lo.l[j][q] = C.v[j];
+            lo.cnt[q] = c;
+          }
+        } else if (c == 1) {
+          const uint64_t q = lbase[1] + lw[1][r * kWarps + warp] + __popc(bs & lanemask_lt());
+          if (q < lo.scap) {
+#pragma unroll
+            for (int j = 0; j < NL; j++) lo.s[j][q] = C.v[j];
+          }
+        }
+        if (!c) continue;
+        uint64_t raw[3], pos[3];
+        bloom_positions<NL>(C, k, fm, raw, pos);
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+          atomicAdd(rhist + (uint32_t)(pos[j] >> kLog2Range), 1u);
+          if (NL >= 2) ((uint32_t*)(keys + (size_t)NL * s))[j] = (uint32_t)pos[j];
+        }
+        if (NL >= 2 && c >= 2) ((uint32_t*)(keys + (size_t)NL * s))[0] |= 0x80000000u;
+      }
+      __syncthreads();
+      for (uint32_t r = threadIdx.x; r < rv.nranges; r += TH) {
+        const uint32_t c = rhist[r];
+        rbase[r] = c ? range_base(rv, r) + atomicAdd(rv.fill + (uint64_t)r * kFillStride, c) : 0ULL;
+        if (NL == 1) rhist[r] = 0;
+      }
+      __syncthreads();
+      if constexpr (NL >= 2) {
+        span_emit_sorted<NL>((const KeyT*)keys, cnt, S, rhist, rcur, rbase, rv, used, n);
+      } else {
+        for (uint32_t i = threadIdx.x; i < n; i += TH) {
+          const uint32_t s = used[i], c = cnt[s];
+          Seq<NL> C;
+          C.v[0] = keys[s];
+          uint64_t raw[3], pos[3];
+          bloom_positions<NL>(C, k, fm, raw, pos);
+#pragma unroll
+          for (int j = 0; j < 3; j++) {
+            const uint32_t r = (uint32_t)(pos[j] >> kLog2Range);
+            const uint64_t q = rbase[r] + atomicAdd(rhist + r, 1u);
+            const uint64_t end = rv.uniform ? (uint64_t)(r + 1) * rv.uniform : rv.base[r + 1];
+            if (q < end)
+              rv.ops[q] = (((uint32_t)pos[j] & ((1u << kLog2Range) - 1)) << 1) | (c >= 2 ? 1u : 0u);
+            else
+              atomicOr(rv.err, (int)kErrRange);
+          }
+        }
+        __syncthreads();
+      }
+      for (uint32_t i = threadIdx.x; i < n; i += TH) {
+#pragma unroll
+        for (int j = 0; j < NL; j++) keys[(size_t)NL * used[i] + j] = kEmpty;
+      }
+      for (uint32_t i = threadIdx.x; i < S; i += TH) cnt[i] = 0;
+      // the next part: the sibling of the deepest one not yet counted
+      while (depth > 0 && (part >> (depth - 1) & 1)) {
+        depth--;
+        part &= (1u << depth) - 1;
+      }
+      if (depth == 0) break;
+      part |= 1u << (depth - 1);
+      __syncthreads();
+    }
+  }
+  warp_add_u64(lo.occ2, occ2);
+  __syncthreads();
+  for (int i = threadIdx.x; i < kHistBins; i += TH)
+    if (s_hist[i]) atomicAdd(lo.hist + i, (unsigned long long)s_hist[i]);
+}
+
+}  // namespace spk

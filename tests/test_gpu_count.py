@@ -692,3 +692,74 @@ def test_sort_buckets_of_every_size(spk, ora, k, base):
     np.testing.assert_array_equal(gc, tc)
     sk, _ = r.solid(0)
     np.testing.assert_array_equal(r.edges(0), ora.edges(sk, k))
+
+
+def _superk_reads(kind, k, rng):
+    """Read sets for the minimizer partition (about a million windows each)."""
+    g = rng.integers(0, 4, 60_000, dtype=np.uint8)
+
+    def from_genome(n, length):
+        out = []
+        for a in rng.integers(0, g.size - length, n):
+            r = g[a:a + length].copy()
+            e = rng.random(length) < 0.005
+            r[e] = (r[e] + 1) % 4
+            out.append((3 - r)[::-1] if rng.random() < 0.5 else r)
+        return out
+
+    if kind == "ragged":  # every length around k and the 32-base steps of a warp's positions
+        lens = [k - 1, k, k + 1, k + 31, k + 32, 160, 161, 150, 250, 256, 257, 300]
+        rows = []
+        for ln in lens:
+            rows += from_genome(1_500, ln)
+        return rows
+    if kind == "long":  # several segments of 256 positions per read
+        return from_genome(300, 5_000) + from_genome(40, 270)
+    if kind == "repeats":  # runs of one minimizer longer than a window, and one k-mer over and over
+        rows = from_genome(12_000, 150)
+        unit = rng.integers(0, 4, 7, dtype=np.uint8)
+        rows += [np.tile(unit, 60)[:400]] * 40 + [np.zeros(400, np.uint8)] * 200 + [np.full(151, 3, np.uint8)] * 30
+        rows += [np.tile(np.array([0, 3], np.uint8), 100)] * 30
+        return rows
+    # "distinct": almost every window a new k-mer, more than a batch's slots
+    return [rng.integers(0, 4, 300, dtype=np.uint8) for _ in range(5_000)]
+
+
+@pytest.mark.parametrize("k,kind", [
+    (21, "ragged"), (26, "ragged"), (27, "ragged"), (32, "ragged"), (33, "ragged"), (55, "ragged"), (63, "ragged"),
+    (65, "ragged"), (95, "ragged"), (97, "ragged"), (127, "ragged"),
+    (21, "long"), (55, "long"), (127, "long"),
+    (21, "repeats"), (31, "repeats"), (55, "repeats"), (77, "repeats"), (127, "repeats"),
+    (21, "distinct"), (47, "distinct"), (49, "distinct"), (79, "distinct"), (113, "distinct")])
+def test_super_kmer_partition(spk, ora, k, kind):
+    """The default job's minimizer partition and batched count: every key
+    width's smallest and largest k, reads of every length around the kernel's
+    steps, runs of one minimizer, and batches with more distinct k-mers than
+    slots (counted in parts).  The whole admitted table, both tiers, the cutoff
+    and the edges equal the oracle's."""
+    import os
+    rows = _superk_reads(kind, k, np.random.default_rng(1000 + k))
+    data, offs, lens = _pack_codes(rows)
+    bits = 1 << 24
+    tw = ora.count(data, offs, lens, k, bits, mode=ora.MODE_TWICE, threads=os.cpu_count() or 1)
+    tk, tc = tw.table(1)
+    oseen, otwice = tw.bloom()
+    r = spk.count((data, offs, lens), [k], bloom_bits=bits, list_min_count=1, flags=BASE)
+    info = r.info(0)
+    assert info["schedule"] == 3 and info["part_rescatters"] == 0
+    # (distinct k-mers past the room made for them: counted again with more)
+    assert info["table_regrows"] == (1 if kind == "distinct" else 0)
+    assert info["occurrences"] == occ(lens, k)
+    gk, gc = r.kmers(0, 1)
+    np.testing.assert_array_equal(gk, tk)
+    np.testing.assert_array_equal(gc, tc)
+    seen, twice = r.bloom(0)
+    np.testing.assert_array_equal(seen, oseen)
+    np.testing.assert_array_equal(twice, otwice)
+    assert info["cutoff"] == ora.cutoff(tc, 5.0)
+    sk, _ = r.solid(0)
+    np.testing.assert_array_equal(r.edges(0), ora.edges(sk, k))
+    d = spk.count((data, offs, lens), [k], bloom_bits=bits)  # counts >= 2 only
+    dk, dc = d.kmers(0)
+    np.testing.assert_array_equal(dk, tk[tc >= 2])
+    np.testing.assert_array_equal(dc, tc[tc >= 2])
