@@ -1315,18 +1315,17 @@ __device__ __forceinline__ uint64_t range_base(const RangeView& rv, uint32_t r) 
 #endif
 constexpr bool kSortedOps = SPK_SORTED_OPS;
 
-template <int NL>
-__device__ __forceinline__ void span_emit_sorted(const typename SpanKey<NL>::T* keys, uint32_t* buf, uint32_t S,
+// get(i, st): the three positions stashed for item i of nslots, "count >= 2" in
+// bit 31 of the first; false if the item has none.
+template <class Get>
+__device__ __forceinline__ void span_emit_sorted(Get get, uint32_t nslots, uint32_t* buf, uint32_t S,
                                                  uint32_t* rs, uint32_t* rcur,
-                                                 const unsigned long long* rbase, const RangeView& rv,
-                                                 const uint16_t* used = nullptr, uint32_t nused = 0) {
+                                                 const unsigned long long* rbase, const RangeView& rv) {
   __shared__ uint32_t wpart[32], wmax[32], bnd[8];
   __shared__ uint32_t s_total, s_maxc;
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const uint32_t nr = rv.nranges;
   const uint32_t mask = (1u << kLog2Range) - 1u;
-  // the span's slots, or the `nused` of them that hold a key
-  const uint32_t nslots = used ? nused : S;
   // counts -> starts (exclusive scan in place), their total and largest count
   const uint32_t per = (nr + blockDim.x - 1) / blockDim.x;
   const uint32_t r0 = min(nr, threadIdx.x * per), r1 = min(nr, r0 + per);
@@ -1369,8 +1368,8 @@ __device__ __forceinline__ void span_emit_sorted(const typename SpanKey<NL>::T* 
   if (H == 0) {
     // direct emission (a range holds more than half a span's worth)
     for (uint32_t i = threadIdx.x; i < nslots; i += blockDim.x) {
-      const uint32_t* st = (const uint32_t*)&keys[used ? used[i] : i];
-      if (!used && st[1] == 0xFFFFFFFFu) continue;  // empty slot
+      uint32_t st[3];
+      if (!get(i, st)) continue;
       const uint32_t flag = st[0] >> 31;
       const uint32_t pk[3] = {st[0] & 0x7FFFFFFFu, st[1], st[2]};
 #pragma unroll
@@ -1401,8 +1400,8 @@ __device__ __forceinline__ void span_emit_sorted(const typename SpanKey<NL>::T* 
   for (uint32_t g = 0; g < G; g++) {
     const uint32_t gb = g * H;
     for (uint32_t i = threadIdx.x; i < nslots; i += blockDim.x) {
-      const uint32_t* st = (const uint32_t*)&keys[used ? used[i] : i];
-      if (!used && st[1] == 0xFFFFFFFFu) continue;  // empty slot
+      uint32_t st[3];
+      if (!get(i, st)) continue;
       const uint32_t flag = st[0] >> 31;
       const uint32_t pk[3] = {st[0] & 0x7FFFFFFFu, st[1], st[2]};
 #pragma unroll
@@ -1672,7 +1671,14 @@ __global__ void __launch_bounds__(kPartBlock, kPartCtasPerSm) k_part_count(PartV
       }
       __syncthreads();
       if (NL >= 2 && kSortedOps) {
-        span_emit_sorted<NL>(keys, cnt, S, rhist, rcur, rbase, rv);
+        span_emit_sorted(
+            [&](uint32_t i, uint32_t (&st)[3]) {
+              const uint32_t* q = (const uint32_t*)&keys[i];
+#pragma unroll
+              for (int j = 0; j < 3; j++) st[j] = q[j];
+              return st[1] != 0xFFFFFFFFu;  // (an empty slot's stash stays all ones)
+            },
+            S, cnt, S, rhist, rcur, rbase, rv);
       } else {
       // Emit the operations.
       for (uint32_t s = threadIdx.x; s < S; s += blockDim.x) {

@@ -335,13 +335,17 @@ __global__ void __launch_bounds__(256) k_sk_place(SkStream S, const uint32_t* __
 // ---------------------------------------------------------------------------
 template <int NL>
 struct SkShape {
-  static constexpr int threads = NL <= 2 ? 512 : 256;
-  static constexpr int ctas = NL == 1 || NL == 3 ? 3 : 2;
-  static constexpr uint32_t log2s = NL <= 2 ? 12 : 11;
+  // Keys of three and four limbs stay in the staged records: their slots hold a
+  // hash tag and where the k-mer was first seen, 8 bytes instead of 24 or 32.
+  static constexpr bool ref = NL >= 3;
+  static constexpr int threads = 512;
+  static constexpr int ctas = NL == 1 ? 3 : 2;
+  static constexpr uint32_t log2s = 12;
   static constexpr uint32_t S = 1u << log2s;  // slots
   // windows per batch: slots over the distinct share expected (0.27 of the
   // occurrences at k = 55, 0.38 at 77, 0.52 at 127 on the reads of the benchmark)
-  static constexpr uint32_t T = NL <= 2 ? 7000 : NL == 3 ? 2700 : 2000;
+  static constexpr uint32_t T = NL <= 2 ? 7000 : NL == 3 ? 5400 : 3900;
+  static constexpr uint32_t slot = ref ? 8 : 8 * NL;  // bytes of a slot's key
 };
 // 32-bit words a record's bases take: at most w windows, w + k - 1 = 2k - m bases.
 __host__ __device__ __forceinline__ uint32_t sk_words(unsigned k) { return (2 * k - sk_m(k) + 15) / 16; }
@@ -352,16 +356,18 @@ struct SkStage {
   size_t smem;
 };
 // Shared memory: keys, counts, used slots; then the staged records (bases,
-// multiplicities, the records' table or the live records, window counts) or,
-// while the batch is written out, the Bloom ranges' counts, cursors and places.
-// As many records are staged as leave room for the CTAs an SM is to hold.
+// multiplicities, the records' table or the live records, window counts) and,
+// while the batch is written out, the Bloom ranges' counts, cursors and places
+// (over the records, unless slots refer to them; those also keep a third word per
+// slot for the positions).  As many records are staged as leave room for the CTAs
+// an SM is to hold.
 template <int NL>
 static SkStage sk_stage(unsigned k, uint32_t nranges) {
   typedef SkShape<NL> P;
   const size_t budget = (size_t)(228 * 1024) / P::ctas - 1024 - 2560;  // of one CTA, less its static arrays
-  const size_t table = (size_t)P::S * (8 * NL + 4 + 2);
   const size_t nr2 = (nranges + 1) & ~1u;
   const size_t ranges = nr2 * 4 * (NL >= 2 ? 2 : 1) + (size_t)nranges * 8;
+  const size_t table = (size_t)P::S * (P::slot + 4 + 2 + (P::ref ? 4 : 0)) + (P::ref ? ranges : 0);
   auto bytes = [&](uint32_t rc, uint32_t dd) { return (size_t)rc * (4 * sk_words(k) + 4 + 1) + (size_t)dd * 4; };
   SkStage g{128, 256, 0};
   for (uint32_t rc = 128; rc <= kSkMaxRecs; rc += 64) {
@@ -369,7 +375,7 @@ static SkStage sk_stage(unsigned k, uint32_t nranges) {
     while (dd < rc + rc / 4) dd *= 2;
     if (table + bytes(rc, dd) <= budget) g = SkStage{rc, dd, 0};
   }
-  g.smem = table + std::max(bytes(g.rc, g.dd), ranges);
+  g.smem = table + (P::ref ? bytes(g.rc, g.dd) : std::max(bytes(g.rc, g.dd), ranges));
   return g;
 }
 
@@ -393,16 +399,17 @@ __device__ __forceinline__ ulonglong2 lds2(const uint64_t* p) {
   return v;
 }
 
-// A claimed slot's top limb carries this bit until the other limbs are written.
+// A claimed slot's top limb carries this bit until the other limb is written.
 constexpr uint64_t kSkBusy = 1ULL << 63;
 
-// One probe step of key C at slot kp: 1 = C's slot, 2 = claimed for C now,
-// 0 = another key's, 3 = being written by a key with C's top limb (look again).
-// Empty slots are all ones, which no key's top limb is.  The top limb is claimed
-// with one 64-bit CAS and published last.  (A 128-bit CAS of the whole key took
-// the place of the claim in k_part_count.)
+// One probe step of key C (k <= 63) at slot kp: 1 = C's slot, 2 = claimed for C
+// now, 0 = another key's, 3 = being written by a key with C's top limb (look
+// again).  Empty slots are all ones, which no key's top limb is.  The top limb is
+// claimed with one 64-bit CAS and published after the other.  (k_part_count
+// claims the whole key with a 128-bit CAS.)
 template <int NL>
 __device__ __forceinline__ int sk_step(uint64_t* kp, const Seq<NL>& C) {
+  static_assert(NL <= 2, "wider keys are referred to");
   volatile uint64_t* v = kp;
   if constexpr (NL == 1) {
     const uint64_t cur = v[0];
@@ -411,43 +418,115 @@ __device__ __forceinline__ int sk_step(uint64_t* kp, const Seq<NL>& C) {
     const uint64_t old = atomicCAS((unsigned long long*)kp, (unsigned long long)kEmpty, (unsigned long long)C.v[0]);
     return old == kEmpty ? 2 : old == C.v[0] ? 1 : 0;
   } else {
-    const uint64_t mine = C.v[NL - 1];
-    uint64_t top, low = kEmpty;
-    if constexpr (NL == 2) {
-      const ulonglong2 q = lds2(kp);
-      low = q.x;
-      top = q.y;
-    } else {
-      top = v[NL - 1];
-    }
+    const uint64_t mine = C.v[1];
+    const ulonglong2 q = lds2(kp);
+    uint64_t top = q.y, low = q.x;
     if (top == kEmpty) {
-      top = atomicCAS((unsigned long long*)(kp + NL - 1), (unsigned long long)kEmpty, (unsigned long long)(mine | kSkBusy));
+      top = atomicCAS((unsigned long long*)(kp + 1), (unsigned long long)kEmpty, (unsigned long long)(mine | kSkBusy));
       if (top == kEmpty) {
-#pragma unroll
-        for (int j = 0; j < NL - 1; j++) v[j] = C.v[j];
+        v[0] = C.v[0];
         __threadfence_block();
-        v[NL - 1] = mine;
+        v[1] = mine;
         return 2;
       }
       low = kEmpty;
     }
     if (top == (mine | kSkBusy)) return 3;
     if (top != mine) return 0;
-    if constexpr (NL == 2) {
-      // (a low limb read before its write is all ones: read it again, after the top)
-      if (low == kEmpty) {
-        __threadfence_block();
-        low = v[0];
-      }
-      return low == C.v[0];
-    } else {
+    // (a low limb read before its write is all ones: read it again, after the top)
+    if (low == kEmpty) {
       __threadfence_block();
-      bool eq = true;
-#pragma unroll
-      for (int j = 0; j < NL - 1; j++) eq &= v[j] == C.v[j];
-      return eq;
+      low = v[0];
     }
+    return low == C.v[0];
   }
+}
+
+// ---- windows as W2 = 2 NL 32-bit words, word 0 most significant ----
+// The bits of a key sit at the top of its words; `low` = 64 NL - 2k bits below
+// them are clear (mask1 and mask2 of the last two words).
+template <int NL>
+struct SkCut {
+  uint32_t low, rot, mask1, mask2;
+};
+template <int NL>
+__device__ __forceinline__ SkCut<NL> sk_cut(unsigned k) {
+  const uint32_t low = 64 * NL - 2 * k, rot = low & 31;
+  return SkCut<NL>{low, rot, low >= 32 ? 0u : ~0u << rot, low >= 32 ? ~0u << rot : ~0u};
+}
+// The window that starts at base o of the staged record whose words are sq[i * RC]
+// (words past the record are masked off).
+template <int NL>
+__device__ __forceinline__ void sk_window(const uint32_t* sq, uint32_t RC, uint32_t o, const SkCut<NL>& c,
+                                          uint32_t (&L)[2 * NL]) {
+  sq += (o >> 4) * RC;
+  const uint32_t sh = 2 * (o & 15);
+  uint32_t u = sq[0];
+#pragma unroll
+  for (int i = 0; i < 2 * NL; i++) {
+    const uint32_t v = sq[(i + 1) * RC];
+    L[i] = __funnelshift_l(v, u, sh);
+    u = v;
+  }
+  L[2 * NL - 1] &= c.mask1;
+  L[2 * NL - 2] &= c.mask2;
+}
+// The same from the packed reads, base `b` (a reference to a record staged in an
+// earlier round).
+template <int NL>
+__device__ __forceinline__ void sk_window_far(const uint64_t* __restrict__ words, uint64_t b, unsigned k,
+                                              const SkCut<NL>& c, uint32_t (&L)[2 * NL]) {
+  const uint64_t* p = words + (b >> 5);
+  const unsigned s = 2 * (unsigned)(b & 31);
+  uint64_t u = bswap64(__ldg(p));
+#pragma unroll
+  for (int i = 0; i < NL; i++) {
+    const uint64_t v = 64u * (i + 1) < s + 2 * k ? bswap64(__ldg(p + i + 1)) : 0ULL;
+    const uint64_t x = shl2(u, v, s);
+    L[2 * i] = (uint32_t)(x >> 32);
+    L[2 * i + 1] = (uint32_t)x;
+    u = v;
+  }
+  L[2 * NL - 1] &= c.mask1;
+  L[2 * NL - 2] &= c.mask2;
+}
+// The reverse complement, at the bottom of G.
+template <int NL>
+__device__ __forceinline__ void sk_revcomp(const uint32_t (&L)[2 * NL], const SkCut<NL>& c, uint32_t (&G)[2 * NL]) {
+  constexpr int W2 = 2 * NL;
+#pragma unroll
+  for (int i = 0; i < W2; i++) {
+    uint32_t z = ~L[W2 - 1 - i];
+    if (i == 0) z &= c.mask1;
+    if (i == 1) z &= c.mask2;
+    z = __brev(z);
+    G[i] = ((z >> 1) & 0x55555555u) | ((z & 0x55555555u) << 1);
+  }
+}
+// Words from the top to the bottom (down) and back (up).
+template <int NL>
+__device__ __forceinline__ void sk_down(const uint32_t (&L)[2 * NL], const SkCut<NL>& c, uint32_t (&F)[2 * NL]) {
+#pragma unroll
+  for (int i = 2 * NL - 1; i >= 0; i--) {
+    const uint32_t l1 = i >= 1 ? L[i >= 1 ? i - 1 : 0] : 0u, l2 = i >= 2 ? L[i >= 2 ? i - 2 : 0] : 0u;
+    F[i] = c.low >= 32 ? __funnelshift_r(l1, l2, c.rot) : __funnelshift_r(L[i], l1, c.rot);
+  }
+}
+template <int NL>
+__device__ __forceinline__ void sk_up(const uint32_t (&F)[2 * NL], const SkCut<NL>& c, uint32_t (&L)[2 * NL]) {
+  constexpr int W2 = 2 * NL;
+#pragma unroll
+  for (int i = 0; i < W2; i++) {
+    const uint32_t f1 = i + 1 < W2 ? F[i + 1 < W2 ? i + 1 : 0] : 0u, f2 = i + 2 < W2 ? F[i + 2 < W2 ? i + 2 : 0] : 0u;
+    L[i] = c.low >= 32 ? __funnelshift_l(f2, f1, c.rot) : __funnelshift_l(f1, F[i], c.rot);
+  }
+}
+template <int NL>
+__device__ __forceinline__ Seq<NL> sk_seq(const uint32_t (&F)[2 * NL]) {
+  Seq<NL> V;
+#pragma unroll
+  for (int i = 0; i < NL; i++) V.v[i] = (uint64_t)F[2 * NL - 2 - 2 * i] << 32 | F[2 * NL - 1 - 2 * i];
+  return V;
 }
 
 template <int NL>
@@ -456,25 +535,29 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
                const uint32_t* __restrict__ bstart, uint32_t nbat, unsigned long long* __restrict__ next_batch,
                unsigned k, uint32_t RC, uint32_t DD, FastMod fm, RangeView rv, ListOut lo, int* __restrict__ err) {
   typedef SkShape<NL> P;
-  typedef typename SpanKey<NL>::T KeyT;
   constexpr uint32_t S = P::S;
   constexpr int TH = P::threads, kWarps = TH / 32, kRounds = S / TH;
   constexpr int W2 = 2 * NL;  // 32-bit words of a key
   extern __shared__ __align__(16) unsigned char sk_smem_[];
+  constexpr bool REF = P::ref;
+  constexpr uint32_t KW = P::slot / 8;  // 64-bit words of a slot
+  const uint32_t nr2 = (rv.nranges + 1) & ~1u;
   uint64_t* keys = (uint64_t*)sk_smem_;
-  uint32_t* cnt = (uint32_t*)(keys + (size_t)S * NL);
+  uint32_t* cnt = (uint32_t*)(keys + (size_t)S * KW);
   uint16_t* used = (uint16_t*)(cnt + S);
   unsigned char* uni = (unsigned char*)(used + S);
+  uint32_t* third = (uint32_t*)uni;      // REF: a slot's third Bloom position
+  if (REF) uni += S * 4;
+  uint32_t* rhist = (uint32_t*)uni;
+  uint32_t* rcur = rhist + nr2;
+  unsigned long long* rbase = (unsigned long long*)(rcur + (NL >= 2 ? nr2 : 0u));
+  if (REF) uni = (unsigned char*)(rbase + rv.nranges);
   const uint32_t SW = sk_words(k);
   uint32_t* seq = (uint32_t*)uni;        // word i (16 bases, the first on top) of record t: seq[i * RC + t]
   uint32_t* mult = seq + (size_t)SW * RC;
   uint32_t* dd = mult + RC;
   uint32_t* lrec = dd;                   // live records: first window << 16 | record (over the records' table)
   uint8_t* nws = (uint8_t*)(dd + DD);
-  uint32_t* rhist = (uint32_t*)uni;
-  const uint32_t nr2 = (rv.nranges + 1) & ~1u;
-  uint32_t* rcur = rhist + nr2;
-  unsigned long long* rbase = (unsigned long long*)(rcur + (NL >= 2 ? nr2 : 0u));
   __shared__ uint32_t lw[2][kRounds * kWarps];
   __shared__ uint32_t wsum[kWarps];
   __shared__ unsigned long long lbase[2];
@@ -483,13 +566,12 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
   __shared__ int s_full;
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t lmin = lo.lmin < 2 ? 2u : lo.lmin;
-  // a key's 2k bits at the top of W2 words: the bits below them, and their number
-  const uint32_t low = 64 * NL - 2 * k, lrot = low & 31;
-  const uint32_t mask1 = low >= 32 ? 0u : ~0u << lrot, mask2 = low >= 32 ? ~0u << lrot : ~0u;
+  const SkCut<NL> cut = sk_cut<NL>(k);
+  constexpr uint64_t kFree = REF ? 0ULL : kEmpty;  // an empty slot
   uint64_t occ2 = 0;
   if (*(volatile int*)err & (int)kErrRegion) return;  // the stream overflowed: records are missing
   for (int i = threadIdx.x; i < kHistBins; i += TH) s_hist[i] = 0;
-  for (uint32_t i = threadIdx.x; i < S * NL; i += TH) keys[i] = kEmpty;
+  for (uint32_t i = threadIdx.x; i < S * KW; i += TH) keys[i] = kFree;
   for (uint32_t i = threadIdx.x; i < S; i += TH) cnt[i] = 0;
   for (;;) {
     __syncthreads();
@@ -499,6 +581,10 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
     if (bt >= nbat) break;
     const uint32_t r0 = bstart[bt], r1 = bstart[bt + 1];
     if (r0 == r1) continue;
+    if (REF && r1 - r0 > 1u << 25) {  // (a reference holds 25 bits of record)
+      if (threadIdx.x == 0) atomicOr(err, (int)kErrRegion);
+      continue;
+    }
     // The batch, or the part of it whose hash bits [0, depth) are `part`: a part
     // with too many distinct k-mers for the table is cut in two.
     uint32_t depth = 0, part = 0;
@@ -601,10 +687,14 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
           for (uint32_t b = kSkMaxRecs / 2; b; b >>= 1)
             if (r + b < nlive && (lrec[r + b] >> 11) <= cur) r += b;
           bool pend = false;
-          Seq<NL> C;
+          Seq<NL> C;                       // the k-mer to place; REF: its window and
+          uint32_t L[W2], G[W2];           // the reverse complement, a tag and the reference
+          uint64_t mine = 0;
           uint32_t slot = 0, step = 0, waits = 0, mu = 0;
 #pragma unroll
           for (int q = 0; q < NL; q++) C.v[q] = 0;
+#pragma unroll
+          for (int q = 0; q < W2; q++) L[q] = G[q] = 0;
           for (;;) {
             const unsigned idle = __ballot_sync(FULL, !pend);
             const uint32_t ni = __popc(idle);
@@ -618,43 +708,27 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
                 const uint32_t e = lrec[r + __popc(mk & (unsigned)((2ULL << rank) - 1))];
                 const uint32_t rt = e & (kSkMaxRecs - 1), o = cur + rank - (e >> 11);
                 mu = mult[rt];
-                // the window's 2k bits at the top of L (words past the record are masked off)
-                const uint32_t* sq = seq + (o >> 4) * RC + rt;
-                const uint32_t sh = 2 * (o & 15);
-                uint32_t L[W2], u = sq[0];
+                sk_window<NL>(seq + rt, RC, o, cut, L);
+                uint32_t F[W2];
+                sk_revcomp<NL>(L, cut, F);
+                uint32_t h;
+                if constexpr (REF) {
+                  sk_up<NL>(F, cut, G);
+                  bool fwd = true;  // canonical: the smaller of the two, src/dna.rs:185-192
 #pragma unroll
-                for (int i = 0; i < W2; i++) {
-                  const uint32_t v = sq[(i + 1) * RC];
-                  L[i] = __funnelshift_l(v, u, sh);
-                  u = v;
-                }
-                L[W2 - 1] &= mask1;
-                L[W2 - 2] &= mask2;
-                // its reverse complement at the bottom of G (word 0 most significant)
-                uint32_t G[W2], F[W2];
+                  for (int i = W2 - 1; i >= 0; i--) fwd = L[i] < G[i] || (L[i] == G[i] && fwd);
+                  uint32_t D[W2];
 #pragma unroll
-                for (int i = 0; i < W2; i++) {
-                  uint32_t z = ~L[W2 - 1 - i];
-                  if (i == 0) z &= mask1;
-                  if (i == 1) z &= mask2;
-                  z = __brev(z);
-                  G[i] = ((z >> 1) & 0x55555555u) | ((z & 0x55555555u) << 1);
+                  for (int i = 0; i < W2; i++) D[i] = fwd ? L[i] : G[i];
+                  h = sk_key_hash<NL>(sk_seq<NL>(D));
+                  const uint32_t tag = (h * 0x297A2D39u ^ D[1] * 0x85EBCA6Bu ^ D[2] * 0xC2B2AE35u) | 1u;
+                  mine = (uint64_t)tag << 32 | ((q0 - r0 + rt) << 7 | o);
+                } else {
+                  sk_down<NL>(L, cut, G);
+                  const Seq<NL> V = sk_seq<NL>(G), Rc = sk_seq<NL>(F);
+                  C = seq_le<NL>(V, Rc) ? V : Rc;  // canonical, src/dna.rs:185-192
+                  h = sk_key_hash<NL>(C);
                 }
-                // ... and the window at the bottom of F
-#pragma unroll
-                for (int i = W2 - 1; i >= 0; i--) {
-                  const uint32_t a = low >= 32 ? (i >= 1 ? L[i >= 1 ? i - 1 : 0] : 0u) : L[i];
-                  const uint32_t b = low >= 32 ? (i >= 2 ? L[i >= 2 ? i - 2 : 0] : 0u) : (i >= 1 ? L[i >= 1 ? i - 1 : 0] : 0u);
-                  F[i] = __funnelshift_r(a, b, lrot);
-                }
-                Seq<NL> V, Rc;
-#pragma unroll
-                for (int i = 0; i < NL; i++) {
-                  V.v[i] = (uint64_t)F[W2 - 2 - 2 * i] << 32 | F[W2 - 1 - 2 * i];
-                  Rc.v[i] = (uint64_t)G[W2 - 2 - 2 * i] << 32 | G[W2 - 1 - 2 * i];
-                }
-                C = seq_le<NL>(V, Rc) ? V : Rc;  // canonical, src/dna.rs:185-192
-                const uint32_t h = sk_key_hash<NL>(C);
                 slot = h >> (32 - P::log2s);
                 step = 0;
                 waits = 0;
@@ -667,7 +741,35 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
               if (cur >= end) break;
               continue;
             }
-            const int got = pend ? sk_step<NL>(keys + (size_t)NL * slot, C) : -1;
+            int got = -1;
+            if (pend) {
+              if constexpr (REF) {
+                // An empty slot is claimed by one CAS of tag and reference (the
+                // bases it refers to do not change); a slot with the same tag is
+                // compared base by base with both strands of the window.
+                uint64_t v = *(volatile uint64_t*)(keys + slot);
+                got = 0;
+                if (v == kFree) {
+                  v = atomicCAS((unsigned long long*)(keys + slot), (unsigned long long)kFree, (unsigned long long)mine);
+                  if (v == kFree) got = 2;
+                }
+                if (got == 0 && (uint32_t)(v >> 32) == (uint32_t)(mine >> 32)) {
+                  const uint32_t ir = ((uint32_t)v >> 7) - (q0 - r0), io = (uint32_t)v & 127;
+                  uint32_t D[W2];
+                  if (ir < n) sk_window<NL>(seq + ir, RC, io, cut, D);
+                  else sk_window_far<NL>(words, (__ldg(recs + r0 + ((uint32_t)v >> 7)) >> 8) + io, k, cut, D);
+                  bool eq = true, er = true;
+#pragma unroll
+                  for (int i = 0; i < W2; i++) {
+                    eq &= D[i] == L[i];
+                    er &= D[i] == G[i];
+                  }
+                  got = eq || er;
+                }
+              } else {
+                got = sk_step<NL>(keys + (size_t)KW * slot, C);
+              }
+            }
             const unsigned won = __ballot_sync(FULL, got == 2);
             if (won) {
               uint32_t u0 = 0;
@@ -693,9 +795,11 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
       }
       __syncthreads();
       const uint32_t n = min(s_used, S);
+      // (REF) the records still staged: those of the last round
+      const uint32_t qlast = (r1 - r0 - 1) / RC * RC, nlast = r1 - r0 - qlast;
       if (s_full) {
         // too many distinct k-mers: this part again as two
-        for (uint32_t i = threadIdx.x; i < S * NL; i += TH) keys[i] = kEmpty;
+        for (uint32_t i = threadIdx.x; i < S * KW; i += TH) keys[i] = kFree;
         for (uint32_t i = threadIdx.x; i < S; i += TH) cnt[i] = 0;
         if (++depth > 16) {
           if (threadIdx.x == 0) atomicOr(err, 1);
@@ -748,8 +852,21 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
         const uint32_t s = i < n ? used[i] : 0u;
         const uint32_t c = i < n ? cnt[s] : 0u;
         Seq<NL> C;
+        if constexpr (REF) {
+          // the key from where it was first seen (in the last staged records, or
+          // in the reads)
+          const uint32_t ref = c ? (uint32_t)keys[s] : qlast << 7, ir = (ref >> 7) - qlast, io = ref & 127;
+          uint32_t L[W2], G[W2], F[W2];
+          if (ir < nlast) sk_window<NL>(seq + ir, RC, io, cut, L);
+          else sk_window_far<NL>(words, (__ldg(recs + r0 + (ref >> 7)) >> 8) + io, k, cut, L);
+          sk_revcomp<NL>(L, cut, G);
+          sk_down<NL>(L, cut, F);
+          const Seq<NL> V = sk_seq<NL>(F), Rc = sk_seq<NL>(G);
+          C = seq_le<NL>(V, Rc) ? V : Rc;
+        } else {
 #pragma unroll
-        for (int j = 0; j < NL; j++) C.v[j] = keys[(size_t)NL * s + j];
+          for (int j = 0; j < NL; j++) C.v[j] = keys[(size_t)KW * s + j];
+        }
         const unsigned bl = __ballot_sync(FULL, c >= lmin), bs = __ballot_sync(FULL, c == 1);
         if (c >= lmin) {
           const uint64_t q = lbase[0] + lw[0][r * kWarps + warp] + __popc(bl & lanemask_lt());
@@ -771,9 +888,10 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
 #pragma unroll
         for (int j = 0; j < 3; j++) {
           atomicAdd(rhist + (uint32_t)(pos[j] >> kLog2Range), 1u);
-          if (NL >= 2) ((uint32_t*)(keys + (size_t)NL * s))[j] = (uint32_t)pos[j];
+          // (positions are below 2^31: the first carries "count >= 2" on top)
+          const uint32_t q = (uint32_t)pos[j] | (j == 0 && c >= 2 ? 0x80000000u : 0u);
+          if (NL >= 2) (REF && j == 2 ? third[s] : ((uint32_t*)(keys + (size_t)KW * s))[j]) = q;
         }
-        if (NL >= 2 && c >= 2) ((uint32_t*)(keys + (size_t)NL * s))[0] |= 0x80000000u;
       }
       __syncthreads();
       for (uint32_t r = threadIdx.x; r < rv.nranges; r += TH) {
@@ -783,7 +901,16 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
       }
       __syncthreads();
       if constexpr (NL >= 2) {
-        span_emit_sorted<NL>((const KeyT*)keys, cnt, S, rhist, rcur, rbase, rv, used, n);
+        span_emit_sorted(
+            [&](uint32_t i, uint32_t (&st)[3]) {
+              const uint32_t s = used[i];
+              const uint32_t* q = (const uint32_t*)(keys + (size_t)KW * s);
+              st[0] = q[0];
+              st[1] = q[1];
+              st[2] = REF ? third[s] : q[2];
+              return true;
+            },
+            n, cnt, S, rhist, rcur, rbase, rv);
       } else {
         for (uint32_t i = threadIdx.x; i < n; i += TH) {
           const uint32_t s = used[i], c = cnt[s];
@@ -806,7 +933,7 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
       }
       for (uint32_t i = threadIdx.x; i < n; i += TH) {
 #pragma unroll
-        for (int j = 0; j < NL; j++) keys[(size_t)NL * used[i] + j] = kEmpty;
+        for (uint32_t j = 0; j < KW; j++) keys[(size_t)KW * used[i] + j] = kFree;
       }
       for (uint32_t i = threadIdx.x; i < S; i += TH) cnt[i] = 0;
       // the next part: the sibling of the deepest one not yet counted
