@@ -3558,13 +3558,16 @@ template <int NL>
 static int sk_count(spk_ctx* ctx, cudaStream_t st, const ReadsView& rv, const SkJob& sj,
                     unsigned long long* next_batch, unsigned k, const FastMod& fm, const RangeView& bv,
                     const ListOut& lo, int* errp) {
-  const SkStage g = sk_stage<NL>(k, bv.nranges);
+  const SkStage g = sk_stage<NL>(k);
   int rc;
   if ((rc = raise_smem_limit((const void*)k_sk_count<NL>, g.smem))) return rc;
   const int grid = (int)std::min<uint64_t>(sj.nbat, (uint64_t)ctx->sm_count * SkShape<NL>::ctas);
   k_sk_count<NL><<<grid, SkShape<NL>::threads, g.smem, st>>>(rv.words, sj.recs.as<uint64_t>(),
                                                              sj.bstart.as<uint32_t>(), sj.nbat, next_batch, k, g.rc,
-                                                             g.dd, fm, bv, lo, errp);
+                                                             g.dd, lo, errp);
+  const size_t osm = ops_smem(bv.nranges);
+  if ((rc = raise_smem_limit((const void*)k_bloom_ops<NL>, osm))) return rc;
+  k_bloom_ops<NL><<<grid_for(ctx, 3), kOpsBlock, osm, st>>>(lo, k, fm, bv);
   SPK_CUDA(cudaGetLastError());
   return SPK_OK;
 }
@@ -3711,7 +3714,7 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
     SPK_CUDA(cudaEventRecord(kc0.e, st));
     rc = SPK_NL_CALL(nl, sk_count, ctx, st, rv, sj, su + S_SKNEXT, k, kr.fm, bv, lo, errp);
     if (rc) return rc;
-    launches++;
+    launches += 2;
   }
   DevBuf base, fill, region;
   DevBuf cbase, cfill, cregion, cfirst;

@@ -17,9 +17,9 @@
 //                with about T windows, so that every batch fits one CTA's table
 //   k_sk_place   the stream's records to their bins
 //   k_sk_count   one CTA per batch: gathers the records' bases, drops repeated
-//                super-k-mers, rolls the windows of the others and counts their
-//                k-mers in shared memory; then list, singletons and Bloom
-//                operations as k_part_count writes them
+//                super-k-mers and counts the k-mers of the others in shared
+//                memory; then the k-mer list and the singletons
+//   k_bloom_ops  the Bloom operations of list and singletons, by Bloom range
 //
 // Bins have exact sizes, so no read set overflows them; a batch with more
 // distinct k-mers than slots is counted in parts (by hash bits), alone.
@@ -37,8 +37,8 @@ constexpr uint64_t kSkWinMask = (1ULL << kSkWinBits) - 1;
 // Length of the minimizers: 15 above 32 bases; 13 and 11 below, where a longer
 // one leaves fewer windows per super-k-mer.
 __host__ __device__ constexpr unsigned sk_m(unsigned k) { return k > 32 ? 15u : k >= 27 ? 13u : 11u; }
-// k this partition takes: windows of at least 11 m-mers, and for keys of several
-// limbs a spare top bit (the table's claim mark).
+// k this partition takes: windows of at least 11 m-mers (and, for keys of several
+// limbs, a top limb with a bit to spare, as the solid set needs).
 __host__ constexpr bool sk_fits(unsigned k) { return k >= 21 && (k <= 32 || 2 * k < 64 * ((k + 31) / 32)); }
 
 struct SkStream {
@@ -335,16 +335,22 @@ __global__ void __launch_bounds__(256) k_sk_place(SkStream S, const uint32_t* __
 // ---------------------------------------------------------------------------
 template <int NL>
 struct SkShape {
-  // Keys of three and four limbs stay in the staged records: their slots hold a
-  // hash tag and where the k-mer was first seen, 8 bytes instead of 24 or 32.
-  static constexpr bool ref = NL >= 3;
-  static constexpr int threads = 512;
-  static constexpr int ctas = NL == 1 ? 3 : 2;
-  static constexpr uint32_t log2s = 12;
+  // Keys of several limbs stay in the staged records: their slots hold a hash
+  // tag and where the k-mer was first seen, 8 bytes instead of 16 to 32.
+  static constexpr bool ref = NL >= 2;
+  // Small tables leave room for five CTAs an SM, whose barriers and gathers
+  // overlap (k = 33, 3 Mb x 60x: 1.24 ms against 1.37 with 4,096 slots and three
+  // CTAs; k = 55, 5 Mb x 100x: 4.4 either way); the longer records of k > 64 need
+  // the larger ones (k = 127: 1.8 against 3.6 ms, where 2,048 slots stage too few).
+  static constexpr int threads = NL <= 2 ? 256 : 384;
+  static constexpr int ctas = NL <= 2 ? 5 : 3;
+  static constexpr uint32_t log2s = NL <= 2 ? 11 : 12;
   static constexpr uint32_t S = 1u << log2s;  // slots
-  // windows per batch: slots over the distinct share expected (0.27 of the
-  // occurrences at k = 55, 0.38 at 77, 0.52 at 127 on the reads of the benchmark)
-  static constexpr uint32_t T = NL <= 2 ? 7000 : NL == 3 ? 5400 : 3900;
+  // Windows per batch: about a third of the slots filled at the distinct share of
+  // the benchmark's reads (0.14 of the occurrences at k = 21, 0.27 at 55, 0.38 at
+  // 77, 0.52 at 127); fuller tables probe longer, emptier ones end in more batches
+  // (k = 55: 4.73, 4.50, 4.40, 4.40 ms at 6,500, 5,500, 4,500, 4,000 in 4,096 slots).
+  static constexpr uint32_t T = NL == 1 ? 3500 : NL == 2 ? 2800 : NL == 3 ? 4100 : 2600;
   static constexpr uint32_t slot = ref ? 8 : 8 * NL;  // bytes of a slot's key
 };
 // 32-bit words a record's bases take: at most w windows, w + k - 1 = 2k - m bases.
@@ -356,18 +362,13 @@ struct SkStage {
   size_t smem;
 };
 // Shared memory: keys, counts, used slots; then the staged records (bases,
-// multiplicities, the records' table or the live records, window counts) and,
-// while the batch is written out, the Bloom ranges' counts, cursors and places
-// (over the records, unless slots refer to them; those also keep a third word per
-// slot for the positions).  As many records are staged as leave room for the CTAs
-// an SM is to hold.
+// multiplicities, the records' table or the live records, window counts).  As many
+// records are staged as leave room for the CTAs an SM is to hold.
 template <int NL>
-static SkStage sk_stage(unsigned k, uint32_t nranges) {
+static SkStage sk_stage(unsigned k) {
   typedef SkShape<NL> P;
   const size_t budget = (size_t)(228 * 1024) / P::ctas - 1024 - 2560;  // of one CTA, less its static arrays
-  const size_t nr2 = (nranges + 1) & ~1u;
-  const size_t ranges = nr2 * 4 * (NL >= 2 ? 2 : 1) + (size_t)nranges * 8;
-  const size_t table = (size_t)P::S * (P::slot + 4 + 2 + (P::ref ? 4 : 0)) + (P::ref ? ranges : 0);
+  const size_t table = (size_t)P::S * (P::slot + 4 + 2);
   auto bytes = [&](uint32_t rc, uint32_t dd) { return (size_t)rc * (4 * sk_words(k) + 4 + 1) + (size_t)dd * 4; };
   SkStage g{128, 256, 0};
   for (uint32_t rc = 128; rc <= kSkMaxRecs; rc += 64) {
@@ -375,7 +376,7 @@ static SkStage sk_stage(unsigned k, uint32_t nranges) {
     while (dd < rc + rc / 4) dd *= 2;
     if (table + bytes(rc, dd) <= budget) g = SkStage{rc, dd, 0};
   }
-  g.smem = table + (P::ref ? bytes(g.rc, g.dd) : std::max(bytes(g.rc, g.dd), ranges));
+  g.smem = table + bytes(g.rc, g.dd);
   return g;
 }
 
@@ -393,53 +394,14 @@ __device__ __forceinline__ uint32_t sk_key_hash(const Seq<NL>& C) {
   return a ^ a >> 15;
 }
 
-__device__ __forceinline__ ulonglong2 lds2(const uint64_t* p) {
-  ulonglong2 v;
-  asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
-  return v;
-}
-
-// A claimed slot's top limb carries this bit until the other limb is written.
-constexpr uint64_t kSkBusy = 1ULL << 63;
-
-// One probe step of key C (k <= 63) at slot kp: 1 = C's slot, 2 = claimed for C
-// now, 0 = another key's, 3 = being written by a key with C's top limb (look
-// again).  Empty slots are all ones, which no key's top limb is.  The top limb is
-// claimed with one 64-bit CAS and published after the other.  (k_part_count
-// claims the whole key with a 128-bit CAS.)
-template <int NL>
-__device__ __forceinline__ int sk_step(uint64_t* kp, const Seq<NL>& C) {
-  static_assert(NL <= 2, "wider keys are referred to");
-  volatile uint64_t* v = kp;
-  if constexpr (NL == 1) {
-    const uint64_t cur = v[0];
-    if (cur == C.v[0]) return 1;
-    if (cur != kEmpty) return 0;
-    const uint64_t old = atomicCAS((unsigned long long*)kp, (unsigned long long)kEmpty, (unsigned long long)C.v[0]);
-    return old == kEmpty ? 2 : old == C.v[0] ? 1 : 0;
-  } else {
-    const uint64_t mine = C.v[1];
-    const ulonglong2 q = lds2(kp);
-    uint64_t top = q.y, low = q.x;
-    if (top == kEmpty) {
-      top = atomicCAS((unsigned long long*)(kp + 1), (unsigned long long)kEmpty, (unsigned long long)(mine | kSkBusy));
-      if (top == kEmpty) {
-        v[0] = C.v[0];
-        __threadfence_block();
-        v[1] = mine;
-        return 2;
-      }
-      low = kEmpty;
-    }
-    if (top == (mine | kSkBusy)) return 3;
-    if (top != mine) return 0;
-    // (a low limb read before its write is all ones: read it again, after the top)
-    if (low == kEmpty) {
-      __threadfence_block();
-      low = v[0];
-    }
-    return low == C.v[0];
-  }
+// One probe step of a one-limb key C at slot kp: 1 = C's slot, 2 = claimed for C
+// now, 0 = another key's.  Empty slots are all ones, which no key is.
+__device__ __forceinline__ int sk_step(uint64_t* kp, uint64_t C) {
+  const uint64_t cur = *(volatile uint64_t*)kp;
+  if (cur == C) return 1;
+  if (cur != kEmpty) return 0;
+  const uint64_t old = atomicCAS((unsigned long long*)kp, (unsigned long long)kEmpty, (unsigned long long)C);
+  return old == kEmpty ? 2 : old == C ? 1 : 0;
 }
 
 // ---- windows as W2 = 2 NL 32-bit words, word 0 most significant ----
@@ -533,25 +495,18 @@ template <int NL>
 __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
     k_sk_count(const uint64_t* __restrict__ words, const uint64_t* __restrict__ recs,
                const uint32_t* __restrict__ bstart, uint32_t nbat, unsigned long long* __restrict__ next_batch,
-               unsigned k, uint32_t RC, uint32_t DD, FastMod fm, RangeView rv, ListOut lo, int* __restrict__ err) {
+               unsigned k, uint32_t RC, uint32_t DD, ListOut lo, int* __restrict__ err) {
   typedef SkShape<NL> P;
   constexpr uint32_t S = P::S;
-  constexpr int TH = P::threads, kWarps = TH / 32, kRounds = S / TH;
+  constexpr int TH = P::threads, kWarps = TH / 32, kRounds = (S + TH - 1) / TH;
   constexpr int W2 = 2 * NL;  // 32-bit words of a key
   extern __shared__ __align__(16) unsigned char sk_smem_[];
   constexpr bool REF = P::ref;
   constexpr uint32_t KW = P::slot / 8;  // 64-bit words of a slot
-  const uint32_t nr2 = (rv.nranges + 1) & ~1u;
   uint64_t* keys = (uint64_t*)sk_smem_;
   uint32_t* cnt = (uint32_t*)(keys + (size_t)S * KW);
   uint16_t* used = (uint16_t*)(cnt + S);
   unsigned char* uni = (unsigned char*)(used + S);
-  uint32_t* third = (uint32_t*)uni;      // REF: a slot's third Bloom position
-  if (REF) uni += S * 4;
-  uint32_t* rhist = (uint32_t*)uni;
-  uint32_t* rcur = rhist + nr2;
-  unsigned long long* rbase = (unsigned long long*)(rcur + (NL >= 2 ? nr2 : 0u));
-  if (REF) uni = (unsigned char*)(rbase + rv.nranges);
   const uint32_t SW = sk_words(k);
   uint32_t* seq = (uint32_t*)uni;        // word i (16 bases, the first on top) of record t: seq[i * RC + t]
   uint32_t* mult = seq + (size_t)SW * RC;
@@ -690,7 +645,7 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
           Seq<NL> C;                       // the k-mer to place; REF: its window and
           uint32_t L[W2], G[W2];           // the reverse complement, a tag and the reference
           uint64_t mine = 0;
-          uint32_t slot = 0, step = 0, waits = 0, mu = 0;
+          uint32_t slot = 0, step = 0, mu = 0;
 #pragma unroll
           for (int q = 0; q < NL; q++) C.v[q] = 0;
 #pragma unroll
@@ -731,7 +686,6 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
                 }
                 slot = h >> (32 - P::log2s);
                 step = 0;
-                waits = 0;
                 pend = depth == 0 || (h & ((1u << depth) - 1)) == part;
               }
               r += __popc(mk & (unsigned)((2ULL << taken) - 1));
@@ -767,7 +721,7 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
                   got = eq || er;
                 }
               } else {
-                got = sk_step<NL>(keys + (size_t)KW * slot, C);
+                got = sk_step(keys + slot, C.v[0]);
               }
             }
             const unsigned won = __ballot_sync(FULL, got == 2);
@@ -786,9 +740,6 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
               if (step >= S) s_full = 1;
               // (a full table's counts are dropped: no long probes for them)
               if ((step & 31) == 0 && *(volatile int*)&s_full) pend = false;
-            } else if (got == 3 && ++waits > (uint32_t)kSpinLimit) {
-              atomicOr(err, 2);  // a claim that never settled: the job fails
-              pend = false;
             }
           }
         }
@@ -811,10 +762,6 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
       // ---- write the part out ----
       // Entries of each (round, warp) of the loop below: a ballot per round,
       // then one reservation for the list and one for the singletons.
-      for (uint32_t i = threadIdx.x; i < rv.nranges; i += TH) {
-        rhist[i] = 0;
-        if (NL >= 2) rcur[i] = 0;
-      }
       const uint32_t rounds = (n + TH - 1) / TH;
       for (uint32_t r = 0; r < rounds; r++) {
         const uint32_t i = r * TH + threadIdx.x;
@@ -882,60 +829,14 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
             for (int j = 0; j < NL; j++) lo.s[j][q] = C.v[j];
           }
         }
-        if (!c) continue;
-        uint64_t raw[3], pos[3];
-        bloom_positions<NL>(C, k, fm, raw, pos);
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-          atomicAdd(rhist + (uint32_t)(pos[j] >> kLog2Range), 1u);
-          // (positions are below 2^31: the first carries "count >= 2" on top)
-          const uint32_t q = (uint32_t)pos[j] | (j == 0 && c >= 2 ? 0x80000000u : 0u);
-          if (NL >= 2) (REF && j == 2 ? third[s] : ((uint32_t*)(keys + (size_t)KW * s))[j]) = q;
-        }
       }
       __syncthreads();
-      for (uint32_t r = threadIdx.x; r < rv.nranges; r += TH) {
-        const uint32_t c = rhist[r];
-        rbase[r] = c ? range_base(rv, r) + atomicAdd(rv.fill + (uint64_t)r * kFillStride, c) : 0ULL;
-        if (NL == 1) rhist[r] = 0;
-      }
-      __syncthreads();
-      if constexpr (NL >= 2) {
-        span_emit_sorted(
-            [&](uint32_t i, uint32_t (&st)[3]) {
-              const uint32_t s = used[i];
-              const uint32_t* q = (const uint32_t*)(keys + (size_t)KW * s);
-              st[0] = q[0];
-              st[1] = q[1];
-              st[2] = REF ? third[s] : q[2];
-              return true;
-            },
-            n, cnt, S, rhist, rcur, rbase, rv);
-      } else {
-        for (uint32_t i = threadIdx.x; i < n; i += TH) {
-          const uint32_t s = used[i], c = cnt[s];
-          Seq<NL> C;
-          C.v[0] = keys[s];
-          uint64_t raw[3], pos[3];
-          bloom_positions<NL>(C, k, fm, raw, pos);
-#pragma unroll
-          for (int j = 0; j < 3; j++) {
-            const uint32_t r = (uint32_t)(pos[j] >> kLog2Range);
-            const uint64_t q = rbase[r] + atomicAdd(rhist + r, 1u);
-            const uint64_t end = rv.uniform ? (uint64_t)(r + 1) * rv.uniform : rv.base[r + 1];
-            if (q < end)
-              rv.ops[q] = (((uint32_t)pos[j] & ((1u << kLog2Range) - 1)) << 1) | (c >= 2 ? 1u : 0u);
-            else
-              atomicOr(rv.err, (int)kErrRange);
-          }
-        }
-        __syncthreads();
-      }
       for (uint32_t i = threadIdx.x; i < n; i += TH) {
+        const uint32_t s = used[i];
 #pragma unroll
-        for (uint32_t j = 0; j < KW; j++) keys[(size_t)KW * used[i] + j] = kFree;
+        for (uint32_t j = 0; j < KW; j++) keys[(size_t)KW * s + j] = kFree;
+        cnt[s] = 0;
       }
-      for (uint32_t i = threadIdx.x; i < S; i += TH) cnt[i] = 0;
       // the next part: the sibling of the deepest one not yet counted
       while (depth > 0 && (part >> (depth - 1) & 1)) {
         depth--;
@@ -950,6 +851,102 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
   __syncthreads();
   for (int i = threadIdx.x; i < kHistBins; i += TH)
     if (s_hist[i]) atomicAdd(lo.hist + i, (unsigned long long)s_hist[i]);
+}
+
+// ---------------------------------------------------------------------------
+// The Bloom operations of the counted k-mers (three per distinct k-mer: its bit
+// in the range, and whether it was counted twice or more), binned by range for
+// k_bloom_apply.  Tiles of 4,096 k-mers, first of the list, then of the
+// singletons: positions and ranks in their range's share of the tile in
+// registers, one reservation per tile and range, then the tile in range order
+// out of shared memory, in runs of a dozen operations.
+//
+// Bound by the ranking's shared-memory atomics and by issue (three hashes per
+// k-mer).  As the write-out of each counted batch these operations came in runs
+// of five, behind a dozen barriers per 1,800 k-mers.
+// ---------------------------------------------------------------------------
+constexpr int kOpsBlock = 512;
+constexpr uint32_t kOpsPer = 8;                       // k-mers per thread and tile
+constexpr uint32_t kOpsTile = kOpsBlock * kOpsPer;
+static size_t ops_smem(uint32_t nranges) { return (size_t)3 * kOpsTile * 4 + (size_t)nranges * (8 + 4 + 4); }
+
+template <int NL>
+__global__ void __launch_bounds__(kOpsBlock, 3) k_bloom_ops(ListOut lo, unsigned k, FastMod fm, RangeView rv) {
+  extern __shared__ __align__(16) unsigned char ops_smem_[];
+  const uint32_t nr = rv.nranges;
+  unsigned long long* gb = (unsigned long long*)ops_smem_;  // where a range's share goes, less its start
+  uint32_t* sorted = (uint32_t*)(gb + nr);
+  uint32_t* hist = sorted + 3 * kOpsTile;
+  uint32_t* start = hist + nr;
+  __shared__ uint32_t wsum[kOpsBlock / 32];
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint64_t nl = min((uint64_t)lo.fill[0], lo.cap), ns = min((uint64_t)lo.fill[1], lo.scap);
+  const uint64_t tl = (nl + kOpsTile - 1) / kOpsTile, ts = (ns + kOpsTile - 1) / kOpsTile;
+  const uint32_t per = (nr + kOpsBlock - 1) / kOpsBlock;
+  const uint32_t b0 = min(nr, threadIdx.x * per), b1 = min(nr, b0 + per);
+  for (uint64_t tile = blockIdx.x; tile < tl + ts; tile += gridDim.x) {
+    const bool list = tile < tl;
+    const uint64_t i0 = (list ? tile : tile - tl) * kOpsTile, n = list ? nl : ns;
+    for (uint32_t r = threadIdx.x; r < nr; r += kOpsBlock) hist[r] = 0;
+    __syncthreads();
+    uint32_t op[kOpsPer][3];
+    uint16_t rk[kOpsPer][3];
+#pragma unroll
+    for (uint32_t u = 0; u < kOpsPer; u++) {
+      const uint64_t i = i0 + u * kOpsBlock + threadIdx.x;
+      if (i < n) {
+        Seq<NL> C;
+#pragma unroll
+        for (int j = 0; j < NL; j++) C.v[j] = list ? lo.l[j][i] : lo.s[j][i];
+        uint64_t raw[3], pos[3];
+        bloom_positions<NL>(C, k, fm, raw, pos);
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+          const uint32_t r = (uint32_t)(pos[j] >> kLog2Range);
+          op[u][j] = r << 20 | ((uint32_t)pos[j] & ((1u << kLog2Range) - 1)) << 1 | (list ? 1u : 0u);
+          rk[u][j] = (uint16_t)atomicAdd(hist + r, 1u);
+        }
+      }
+    }
+    __syncthreads();
+    uint32_t sum = 0;
+    for (uint32_t r = b0; r < b1; r++) sum += hist[r];
+    uint32_t x = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(FULL, x, d);
+      if ((int)lane >= d) x += y;
+    }
+    if (lane == 31) wsum[warp] = x;
+    __syncthreads();
+    uint32_t before = x - sum, total = 0;
+#pragma unroll
+    for (unsigned w = 0; w < kOpsBlock / 32; w++) {
+      if (w < warp) before += wsum[w];
+      total += wsum[w];
+    }
+    for (uint32_t r = b0; r < b1; r++) {
+      const uint32_t c = hist[r];
+      start[r] = before;
+      gb[r] = (c ? range_base(rv, r) + atomicAdd(rv.fill + (uint64_t)r * kFillStride, c) : 0ULL) - before;
+      before += c;
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t u = 0; u < kOpsPer; u++)
+      if (i0 + u * kOpsBlock + threadIdx.x < n)
+#pragma unroll
+        for (int j = 0; j < 3; j++) sorted[start[op[u][j] >> 20] + rk[u][j]] = op[u][j];
+    __syncthreads();
+    for (uint32_t q = threadIdx.x; q < total; q += kOpsBlock) {
+      const uint32_t v = sorted[q], r = v >> 20;
+      const uint64_t at = gb[r] + q;
+      const uint64_t end = rv.uniform ? (uint64_t)(r + 1) * rv.uniform : rv.base[r + 1];
+      if (at < end) rv.ops[at] = v & 0xFFFFFu;
+      else atomicOr(rv.err, (int)kErrRange);
+    }
+    __syncthreads();
+  }
 }
 
 }  // namespace spk
