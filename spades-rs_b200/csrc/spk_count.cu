@@ -471,22 +471,6 @@ __device__ __forceinline__ void table_add(const TableView& t, const Seq<NL>& C, 
   atomicOr(t.err, 1);  // probe limit: the host regrows the table and recounts
 }
 
-// Read-only lookup after counting: the count (with the kRejected flag) or 0.
-template <int NL>
-__device__ __forceinline__ uint32_t table_find(const TableView& t, const Seq<NL>& C, uint64_t home) {
-  for (uint32_t i = 0; i < t.max_probe; i++) {
-    const uint64_t s = probe_slot(t, home, i);
-    const uint32_t c = __ldg(slot_count<NL>(t, s));
-    if (c == 0) return 0;  // empty slot ends the probe sequence
-    const uint64_t* kp = slot_key<NL>(t, s);
-    bool eq = true;
-#pragma unroll
-    for (int j = 0; j < NL; j++) eq &= __ldg(kp + j) == C.v[j];
-    if (eq) return c;
-  }
-  return 0;
-}
-
 template <int NL>
 __device__ __forceinline__ void warp_table_add(const TableView& t, bool take, const Seq<NL>& C,
                                                uint64_t raw0, const SlotPeek* peek = nullptr) {
@@ -2239,36 +2223,39 @@ __device__ __forceinline__ Seq<NLE> prepend_wide(const Seq<NL>& RC, unsigned c, 
   return R;
 }
 
-// The solid k-mers (count >= cutoff) of a list as a set: open addressing with
-// linear probing over 2^log2cap slots of NL key limbs (k <= 64), all-ones =
-// empty (never a canonical k-mer: all-ones full limbs would be poly-T, whose
-// reverse complement poly-A is smaller, and a partial top limb never has its
-// unused bits set).  Home slot: hash_kmer256(key, seed 1) >> (64 - log2cap).
-// Probed 8 times per solid k-mer by k_edges, it is small enough to stay
-// mostly in L2, unlike the count table.  A bit filter of 2^log2filter bits
-// (bit: the low hash bits of each solid k-mer) answers most lookups of
-// k-mers that are not solid with one L2-resident bit.
-struct SetView {
-  uint64_t* keys;
-  uint32_t log2cap;
-  uint32_t log2filter;
-  uint32_t* filter;
-};
-__device__ __forceinline__ uint64_t filter_bit(const SetView& sv, uint64_t raw0) {
-  return raw0 & ((1ULL << sv.log2filter) - 1);
-}
-
-// Wide keys (k > 64) take a slot with a CAS on their top limb and then write
-// the others: the keys inserted are distinct, and lookups run in a later
-// kernel.  The top limb of a key with 2k < 64 NL has unused high bits, so it
-// is never all-ones (k = 96 fills it and does not use the set).
+// The solid k-mers (count >= cutoff) of a list as a set: 2^log2cap slots of 8
+// bytes, a 32-bit hash tag above the k-mer's index in the list (all-ones: empty),
+// in buckets of four, one 32-byte sector each, probed one bucket after another;
+// a bucket fills from its first slot, so an empty slot ends a search.  Equal tags
+// are settled by the list's key.  At 5 M solid k-mers the slots are 67 MB (whole
+// 16-byte keys were 134).  A bit filter of 2^log2filter bits (16 or more per solid
+// k-mer, 16 MB there) turns most other k-mers away.
 struct ListCols {
   const uint64_t* p[4];
 };
+struct SetView {
+  unsigned long long* slots;
+  uint32_t log2cap, log2filter;
+  uint32_t* filter;
+  ListCols L;
+};
+__device__ __forceinline__ uint32_t filter_bit(const SetView& sv, uint64_t x) {
+  return (uint32_t)x & ((1u << sv.log2filter) - 1);
+}
+// The set's hash: a multilinear sum of the limbs, mixed.
 template <int NL>
-__global__ void __launch_bounds__(kBlock) k_solid_set(ListCols L, const uint32_t* __restrict__ cnt, uint64_t n,
-                                                       const uint32_t* __restrict__ thr, unsigned k,
-                                                       SetView sv) {
+__device__ __forceinline__ uint64_t set_hash(const Seq<NL>& C) {
+  const uint64_t K[4] = {0x9E3779B97F4A7C15ULL, 0xBF58476D1CE4E5B9ULL, 0x94D049BB133111EBULL, 0xD6E8FEB86659FD93ULL};
+  uint64_t x = 0x2545F4914F6CDD1DULL;
+#pragma unroll
+  for (int j = 0; j < NL; j++) x += C.v[j] * K[j];
+  x ^= x >> 32;
+  x *= 0xD6E8FEB86659FD93ULL;
+  return x ^ x >> 29;
+}
+template <int NL>
+__global__ void __launch_bounds__(kBlock) k_solid_set(const uint32_t* __restrict__ cnt, uint64_t n,
+                                                       const uint32_t* __restrict__ thr, SetView sv) {
   const uint32_t cutoff = thr[0];
   const uint64_t mask = (1ULL << sv.log2cap) - 1;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
@@ -2276,147 +2263,134 @@ __global__ void __launch_bounds__(kBlock) k_solid_set(ListCols L, const uint32_t
     if (cnt[i] < cutoff) continue;
     Seq<NL> C;
 #pragma unroll
-    for (int j = 0; j < NL; j++) C.v[j] = L.p[j][i];
-    uint64_t w4[4];
-    kmer256_limbs<NL>(C, k, w4);
-    const uint64_t raw0 = hash_seed(hash_pre(w4), kSeed1);
-    const uint64_t fb = filter_bit(sv, raw0);
+    for (int j = 0; j < NL; j++) C.v[j] = sv.L.p[j][i];
+    const uint64_t x = set_hash<NL>(C);
+    const uint32_t fb = filter_bit(sv, x);
     atomicOr(sv.filter + (fb >> 5), 1u << (fb & 31));
-    uint64_t h = raw0 >> (64 - sv.log2cap);
+    uint64_t h = x >> (64 - sv.log2cap) & ~3ULL;
     // keys are distinct and the set is at most 2/3 full, so a free slot is found
-    for (uint64_t probe = 0; probe <= mask; probe++, h = (h + 1) & mask) {
-      if constexpr (NL == 1) {
-        if (atomicCAS((unsigned long long*)sv.keys + h, kEmpty, (unsigned long long)C.v[0]) == kEmpty)
-          break;
-      } else if constexpr (NL == 2) {
-        const U128 old = atomicCAS((U128*)sv.keys + h, U128{kEmpty, kEmpty}, U128{C.v[0], C.v[NL - 1]});
-        if (old.x == kEmpty && old.y == kEmpty) break;
-      } else {
-        uint64_t* kp = sv.keys + (uint64_t)NL * h;
-        if (atomicCAS((unsigned long long*)(kp + NL - 1), kEmpty, (unsigned long long)C.v[NL - 1]) == kEmpty) {
-#pragma unroll
-          for (int j = 0; j < NL - 1; j++) kp[j] = C.v[j];
-          break;
-        }
-      }
-    }
+    for (uint64_t probe = 0; probe <= mask; probe++, h = (h + 1) & mask)
+      if (atomicCAS(sv.slots + h, (unsigned long long)kEmpty, (unsigned long long)(x << 32 | i)) == kEmpty) break;
   }
 }
 
+// Whether C, of hash x, is in the set.
 template <int NL>
-__device__ __forceinline__ bool set_has(const SetView& sv, const Seq<NL>& C, uint64_t raw0) {
-  const uint64_t fb = filter_bit(sv, raw0);
-  if (!((__ldg(sv.filter + (fb >> 5)) >> (fb & 31)) & 1u)) return false;
+__device__ __forceinline__ bool set_has(const SetView& sv, const Seq<NL>& C, uint64_t x) {
   const uint64_t mask = (1ULL << sv.log2cap) - 1;
-  uint64_t h = raw0 >> (64 - sv.log2cap);
-  for (uint64_t probe = 0; probe <= mask; probe++, h = (h + 1) & mask) {
-    if constexpr (NL == 1) {
-      const uint64_t v = __ldg(sv.keys + h);
-      if (v == C.v[0]) return true;
-      if (v == kEmpty) return false;
-    } else if constexpr (NL == 2) {
-      const ulonglong2 v = __ldg((const ulonglong2*)sv.keys + h);
-      if (v.x == C.v[0] && v.y == C.v[NL - 1]) return true;
-      if (v.x == kEmpty && v.y == kEmpty) return false;
-    } else {
-      const uint64_t* kp = sv.keys + (uint64_t)NL * h;
-      const uint64_t top = __ldg(kp + NL - 1);
-      if (top == kEmpty) return false;
-      bool eq = top == C.v[NL - 1];
+  uint64_t h = x >> (64 - sv.log2cap) & ~3ULL;
+  for (uint64_t probe = 0; probe <= mask; probe += 4, h = (h + 4) & mask) {
+    const ulonglong2 a = __ldg((const ulonglong2*)(sv.slots + h)), b = __ldg((const ulonglong2*)(sv.slots + h) + 1);
+    const uint64_t v[4] = {a.x, a.y, b.x, b.y};
 #pragma unroll
-      for (int j = 0; j < NL - 1; j++) eq &= __ldg(kp + j) == C.v[j];
+    for (int q = 0; q < 4; q++) {
+      if ((uint32_t)(v[q] >> 32) != (uint32_t)x || v[q] == kEmpty) continue;
+      const uint32_t i = (uint32_t)v[q];
+      bool eq = true;
+#pragma unroll
+      for (int j = 0; j < NL; j++) eq &= __ldg(sv.L.p[j] + i) == C.v[j];
       if (eq) return true;
     }
+    if (b.y == kEmpty) return false;  // (the last slot to fill)
   }
   return false;
 }
 
-template <int NL, int NLE, bool SET>
-__global__ void __launch_bounds__(kBlock) k_edges(const uint64_t* l0, const uint64_t* l1,
-                                                   const uint64_t* l2, const uint64_t* l3,
-                                                   const uint32_t* __restrict__ cnt, uint64_t n,
-                                                   const uint32_t* __restrict__ thr, TableView t,
-                                                   SetView sv, unsigned k, uint64_t* e0, uint64_t* e1,
-                                                   uint64_t* e2, uint64_t* e3, uint64_t out_cap,
-                                                   unsigned long long* __restrict__ counter) {
+// Bound by the latency of its random reads.  An edge is looked up only from the
+// end where it is its own canonical form (four of a solid k-mer's eight on
+// average), the filter words of all of those are read together, and only the few
+// that pass (one and a quarter on average) go on to the set, one after another.
+constexpr int kEdgeRounds = 4;  // k-mers per thread and reservation
+template <int NL, int NLE>
+__global__ void __launch_bounds__(kBlock) k_edges(const uint32_t* __restrict__ cnt, uint64_t n,
+                                                   const uint32_t* __restrict__ thr, SetView sv, unsigned k,
+                                                   uint64_t* e0, uint64_t* e1, uint64_t* e2, uint64_t* e3,
+                                                   uint64_t out_cap, unsigned long long* __restrict__ counter) {
+  constexpr int U = kEdgeRounds;
+  __shared__ uint32_t wsum[kBlock / 32];
+  __shared__ unsigned long long s_base;
   const uint32_t cutoff = thr[0];
-  const unsigned lane = threadIdx.x & 31;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  const uint64_t start = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  for (uint64_t base = start - lane; base < n; base += stride) {
-    const uint64_t i = base + lane;
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (uint64_t tile = blockIdx.x * (uint64_t)(U * kBlock); tile < n; tile += (uint64_t)gridDim.x * (U * kBlock)) {
+  uint32_t em = 0;  // byte u: bit 4o + b: the edge of orientation o and base b of the round's k-mer
+#pragma unroll 1
+  for (int u = 0; u < U; u++) {
+    const uint64_t i = tile + (uint64_t)u * kBlock + threadIdx.x;
     Seq<NL> S;
     bool solid = false;
     if (i < n) {
-      S.v[0] = l0[i];
-      if (NL > 1) S.v[NL > 1 ? 1 : 0] = l1[i];
-      if (NL > 2) S.v[NL > 2 ? 2 : 0] = l2[i];
-      if (NL > 3) S.v[NL > 3 ? 3 : 0] = l3[i];
+#pragma unroll
+      for (int j = 0; j < NL; j++) S.v[j] = sv.L.p[j][i];
       solid = cnt[i] >= cutoff;
     }
-    uint32_t emits = 0;  // bit 4o + b: the edge of orientation o and base b
+    uint32_t emits = 0;
     Seq<NL> RS;
     if (solid) RS = revcomp<NL>(S, k);
-    for (int o = 0; o < 2; o++) {
-      // the oriented k-mer and its reverse complement
-      const Seq<NL> EX = o ? RS : S;
-      const Seq<NL> RX = o ? S : RS;
-      bool ok = solid;
-      if (o == 1 && ok) ok = !seq_eq<NL>(RS, S);  // a palindromic k-mer (even k) has one orientation
-      for (unsigned b = 0; b < 4; b++) {
-        bool emit = false;
-        if (ok) {
-          const Seq<NL> NB = shl_append<NL>(EX, b, k);
-          const Seq<NL> RB = shr_prepend<NL>(RX, 3u - b, k);
-          const Seq<NL> CN = seq_le<NL>(NB, RB) ? NB : RB;  // canonical, src/dna.rs:185-192
-          uint64_t w4[4];
-          kmer256_limbs<NL>(CN, k, w4);
-          const HashPre hp = hash_pre(w4);
-          const uint64_t raw0 = hash_seed(hp, kSeed1);
-          bool solid_nb;
-          if (SET) {
-            solid_nb = set_has<NL>(sv, CN, raw0);
-          } else {
-            const uint32_t c = table_find<NL>(t, CN, table_home(t, raw0));
-            solid_nb = c && !(c & kRejected) && c >= cutoff;
-          }
-          if (solid_nb) {
-            const Seq<NLE> E = widen_append<NL, NLE>(EX, b);
-            emit = seq_le<NLE>(E, prepend_wide<NL, NLE>(RX, 3u - b, k));
-          }
-        }
-        if (emit) emits |= 1u << (4 * o + b);
-      }
-    }
-    // One reservation per warp for all its edges, then write them (the
-    // edge (k+1)-mer is rebuilt from the oriented k-mer and the base).
-    const uint32_t ne = __popc(emits);
-    uint32_t incl = ne;
+    // the neighbour across base b of orientation o, canonical (src/dna.rs:185-192)
+    auto neighbour = [&](int o, unsigned b) {
+      const Seq<NL> NB = shl_append<NL>(o ? RS : S, b, k);
+      const Seq<NL> RB = shr_prepend<NL>(o ? S : RS, 3u - b, k);
+      return seq_le<NL>(NB, RB) ? NB : RB;
+    };
+    const bool both = solid && !seq_eq<NL>(RS, S);  // a palindromic k-mer (even k) has one orientation
+    uint32_t fw[8], fs[8];  // filter words and shifts; a word of 0: not looked up
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t v = __shfl_up_sync(FULL, incl, d);
-      if ((int)lane >= d) incl += v;
-    }
-    const uint32_t wtot = __shfl_sync(FULL, incl, 31);
-    if (!wtot) continue;
-    unsigned long long wb = 0;
-    if (lane == 0) wb = atomicAdd(counter, (unsigned long long)wtot);
-    uint64_t p = __shfl_sync(FULL, wb, 0) + incl - ne;
-    for (int o = 0; o < 2; o++) {
-      if (!(emits >> (4 * o) & 15u)) continue;
-      const Seq<NL> EX = o ? revcomp<NL>(S, k) : S;
-      for (unsigned b = 0; b < 4; b++) {
-        if (!(emits >> (4 * o + b) & 1u)) continue;
-        const Seq<NLE> E = widen_append<NL, NLE>(EX, b);
-        if (p < out_cap) {
-          e0[p] = E.v[0];
-          if (NLE > 1) e1[p] = E.v[NLE > 1 ? 1 : 0];
-          if (NLE > 2) e2[p] = E.v[NLE > 2 ? 2 : 0];
-          if (NLE > 3) e3[p] = E.v[NLE > 3 ? 3 : 0];
-        }
-        p++;
+    for (int q = 0; q < 8; q++) {
+      const int o = q >> 2;
+      const unsigned b = q & 3;
+      fw[q] = fs[q] = 0;
+      if ((o ? both : solid) && seq_le<NLE>(widen_append<NL, NLE>(o ? RS : S, b),
+                                            prepend_wide<NL, NLE>(o ? S : RS, 3u - b, k))) {
+        const uint32_t fb = filter_bit(sv, set_hash<NL>(neighbour(o, b)));
+        fw[q] = __ldg(sv.filter + (fb >> 5));
+        fs[q] = fb & 31;
       }
     }
+    uint32_t pass = 0;
+#pragma unroll
+    for (int q = 0; q < 8; q++) pass |= (fw[q] >> fs[q] & 1u) << q;
+    for (; pass; pass &= pass - 1) {
+      const unsigned q = __ffs(pass) - 1;
+      const Seq<NL> C = neighbour((int)(q >> 2), q & 3);
+      if (set_has<NL>(sv, C, set_hash<NL>(C))) emits |= 1u << q;
+    }
+    em |= emits << (8 * u);
+  }
+  // One reservation for the tile's edges, then write them (the edge (k+1)-mer
+  // is rebuilt from the oriented k-mer and the base).
+  const uint32_t ne = __popc(em);
+  uint32_t incl = ne;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t v = __shfl_up_sync(FULL, incl, d);
+    if ((int)lane >= d) incl += v;
+  }
+  if (lane == 31) wsum[warp] = incl;
+  __syncthreads();
+  uint32_t before = 0, total = 0;
+#pragma unroll
+  for (unsigned w = 0; w < kBlock / 32; w++) {
+    if (w < warp) before += wsum[w];
+    total += wsum[w];
+  }
+  if (threadIdx.x == 0) s_base = total ? atomicAdd(counter, (unsigned long long)total) : 0ULL;
+  __syncthreads();
+  uint64_t p = s_base + before + incl - ne;
+  for (uint32_t left = em; left; left &= left - 1) {
+    const unsigned q = __ffs(left) - 1, o = q >> 2 & 1, b = q & 3;
+    const uint64_t i = tile + (uint64_t)(q >> 3) * kBlock + threadIdx.x;
+    Seq<NL> S;
+#pragma unroll
+    for (int j = 0; j < NL; j++) S.v[j] = sv.L.p[j][i];
+    const Seq<NLE> E = widen_append<NL, NLE>(o ? revcomp<NL>(S, k) : S, b);
+    if (p < out_cap) {
+      e0[p] = E.v[0];
+      if (NLE > 1) e1[p] = E.v[NLE > 1 ? 1 : 0];
+      if (NLE > 2) e2[p] = E.v[NLE > 2 ? 2 : 0];
+      if (NLE > 3) e3[p] = E.v[NLE > 3 ? 3 : 0];
+    }
+    p++;
+  }
   }
 }
 
@@ -2673,42 +2647,44 @@ static void launch_admit(spk_ctx* ctx, cudaStream_t st, const TableView& t, unsi
                                                           rejected);
 }
 template <int NL, int NLE>
-static void launch_edges_t(spk_ctx* ctx, cudaStream_t st, uint64_t* l[4], const uint32_t* cnt,
-                           uint64_t n, const uint32_t* thr, const TableView& t, const SetView* sv,
-                           unsigned k, uint64_t* e[4], uint64_t out_cap,
+static void launch_edges_t(spk_ctx* ctx, cudaStream_t st, const uint32_t* cnt, uint64_t n, const uint32_t* thr,
+                           const SetView& sv, unsigned k, uint64_t* e[4], uint64_t out_cap,
                            unsigned long long* counter) {
-  if (sv)
-    k_edges<NL, NLE, true><<<grid_for(ctx, 8), kBlock, 0, st>>>(
-        l[0], l[1], l[2], l[3], cnt, n, thr, t, *sv, k, e[0], e[1], e[2], e[3], out_cap, counter);
-  else
-    k_edges<NL, NLE, false><<<grid_for(ctx, 8), kBlock, 0, st>>>(
-        l[0], l[1], l[2], l[3], cnt, n, thr, t, SetView{nullptr, 0, 0, nullptr}, k, e[0], e[1], e[2], e[3],
-        out_cap, counter);
+  k_solid_set<NL><<<grid_for(ctx, 8), kBlock, 0, st>>>(cnt, n, thr, sv);
+  k_edges<NL, NLE><<<grid_for(ctx, 8), kBlock, 0, st>>>(cnt, n, thr, sv, k, e[0], e[1], e[2], e[3], out_cap,
+                                                       counter);
 }
-// sv: the solid set, or nullptr to probe the count table.
-static void launch_edges(spk_ctx* ctx, cudaStream_t st, int nl, int nle, uint64_t* l[4],
-                         const uint32_t* cnt, uint64_t n, const uint32_t* thr, const TableView& t,
-                         const SetView* sv, unsigned k, uint64_t* e[4], uint64_t out_cap,
-                         unsigned long long* counter) {
-  if (nl == 1 && nle == 1) launch_edges_t<1, 1>(ctx, st, l, cnt, n, thr, t, sv, k, e, out_cap, counter);
-  else if (nl == 1) launch_edges_t<1, 2>(ctx, st, l, cnt, n, thr, t, sv, k, e, out_cap, counter);
-  else if (nl == 2 && nle == 2) launch_edges_t<2, 2>(ctx, st, l, cnt, n, thr, t, sv, k, e, out_cap, counter);
-  else if (nl == 2) launch_edges_t<2, 3>(ctx, st, l, cnt, n, thr, t, sv, k, e, out_cap, counter);
-  else if (nl == 3 && nle == 3) launch_edges_t<3, 3>(ctx, st, l, cnt, n, thr, t, sv, k, e, out_cap, counter);
-  else if (nl == 3) launch_edges_t<3, 4>(ctx, st, l, cnt, n, thr, t, sv, k, e, out_cap, counter);
-  else launch_edges_t<4, 4>(ctx, st, l, cnt, n, thr, t, sv, k, e, out_cap, counter);
+// The solid k-mers of the list l (n entries, n_solid of them solid) as a set and
+// their edges, unsorted; `set` is the set's memory.
+static int launch_edges(spk_ctx* ctx, cudaStream_t st, int nl, int nle, uint64_t* const l[4], const uint32_t* cnt,
+                        uint64_t n, uint64_t n_solid, const uint32_t* thr, unsigned k, DevBuf& set, uint64_t* e[4],
+                        uint64_t out_cap, unsigned long long* counter) {
+  if (n >= 0xFFFFFFFFULL) return fail(SPK_E_INVALID_ARG, "edges: more than 2^32 listed k-mers");
+  uint32_t lg = 10;
+  while ((1ULL << lg) < n_solid + (n_solid >> 1) + 1) lg++;
+  uint32_t lf = 15;
+  while (lf < 31 && (1ULL << lf) < n_solid * 16) lf++;  // ~1/16 false positives
+  const size_t slot_bytes = (size_t)8 << lg, filter_bytes = (size_t)1 << (lf - 3);
+  int rc;
+  if ((rc = set.alloc(slot_bytes + filter_bytes, st))) return rc;
+  SPK_CUDA(cudaMemsetAsync(set.p, 0xFF, slot_bytes, st));
+  SPK_CUDA(cudaMemsetAsync(set.as<uint8_t>() + slot_bytes, 0, filter_bytes, st));
+  const SetView sv{set.as<unsigned long long>(), lg, lf, (uint32_t*)(set.as<uint8_t>() + slot_bytes),
+                   ListCols{{l[0], l[1], l[2], l[3]}}};
+  if (nl == 1 && nle == 1) launch_edges_t<1, 1>(ctx, st, cnt, n, thr, sv, k, e, out_cap, counter);
+  else if (nl == 1) launch_edges_t<1, 2>(ctx, st, cnt, n, thr, sv, k, e, out_cap, counter);
+  else if (nl == 2 && nle == 2) launch_edges_t<2, 2>(ctx, st, cnt, n, thr, sv, k, e, out_cap, counter);
+  else if (nl == 2) launch_edges_t<2, 3>(ctx, st, cnt, n, thr, sv, k, e, out_cap, counter);
+  else if (nl == 3 && nle == 3) launch_edges_t<3, 3>(ctx, st, cnt, n, thr, sv, k, e, out_cap, counter);
+  else if (nl == 3) launch_edges_t<3, 4>(ctx, st, cnt, n, thr, sv, k, e, out_cap, counter);
+  else launch_edges_t<4, 4>(ctx, st, cnt, n, thr, sv, k, e, out_cap, counter);
+  SPK_CUDA(cudaGetLastError());
+  return SPK_OK;
 }
-static void launch_solid_set(spk_ctx* ctx, cudaStream_t st, int nl, uint64_t* const l[4], const uint32_t* cnt,
-                             uint64_t n, const uint32_t* thr, unsigned k, const SetView& sv) {
-  const ListCols L{{l[0], l[1], l[2], l[3]}};
-  const int g = grid_for(ctx, 8);
-  switch (nl) {
-    case 1: k_solid_set<1><<<g, kBlock, 0, st>>>(L, cnt, n, thr, k, sv); break;
-    case 2: k_solid_set<2><<<g, kBlock, 0, st>>>(L, cnt, n, thr, k, sv); break;
-    case 3: k_solid_set<3><<<g, kBlock, 0, st>>>(L, cnt, n, thr, k, sv); break;
-    default: k_solid_set<4><<<g, kBlock, 0, st>>>(L, cnt, n, thr, k, sv); break;
-  }
-}
+// Most edges of n solid k-mers: each of their 8 n oriented extensions is half an
+// edge, or a whole one that is its own reverse complement (one base at most
+// makes it so, for each orientation).
+static uint64_t max_edges(uint64_t n) { return 5 * n; }
 
 static uint64_t next_pow2(uint64_t x) {
   uint64_t p = 1;
@@ -3379,32 +3355,16 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
   kr.nle = (int)((k + 1 + 31) / 32);
   if ((o.flags & SPK_F_EDGES) && info.n_solid > 0) {
     uint64_t* ep[4] = {nullptr, nullptr, nullptr, nullptr};
-    const uint64_t ecap = info.n_solid * 8;  // at most 8 canonical edges per solid k-mer
+    const uint64_t ecap = max_edges(info.n_solid);
     for (int j = 0; j < kr.nle; j++) {
       if ((rc = kr.edges[j].alloc(ecap * 8, st))) return rc;
       ep[j] = kr.edges[j].as<uint64_t>();
     }
-    // For k <= 64 the neighbours are looked up in a set of the solid k-mers
-    // (at most 2/3 full), built from the list; wider keys probe the table.
-    DevBuf set, filt;
-    SetView sv{nullptr, 0, 0, nullptr};
-    if (nl <= 2) {
-      uint32_t lg = 10, lf = 20;
-      while ((1ULL << lg) < info.n_solid + (info.n_solid >> 1) + 1) lg++;
-      while (lf < 30 && (1ULL << lf) < info.n_solid * 16) lf++;  // ~1/16 false positives
-      if ((rc = set.alloc((1ULL << lg) * nl * 8, st)) || (rc = filt.alloc((1ULL << lf) / 8, st)))
-        return rc;
-      SPK_CUDA(cudaMemsetAsync(set.p, 0xFF, (1ULL << lg) * nl * 8, st));
-      SPK_CUDA(cudaMemsetAsync(filt.p, 0, (1ULL << lf) / 8, st));
-      sv = SetView{set.as<uint64_t>(), lg, lf, filt.as<uint32_t>()};
-      launch_solid_set(ctx, st, nl, lp, kr.list[4].as<uint32_t>(), kr.list_len, thr, k, sv);
-      SPK_CUDA(cudaGetLastError());
-      launches++;
-    }
-    launch_edges(ctx, st, nl, kr.nle, lp, kr.list[4].as<uint32_t>(), kr.list_len, thr, kr.table,
-                 nl <= 2 ? &sv : nullptr, k, ep, ecap, su + S_EDGES);
-    SPK_CUDA(cudaGetLastError());
-    launches++;
+    DevBuf set;
+    if ((rc = launch_edges(ctx, st, nl, kr.nle, lp, kr.list[4].as<uint32_t>(), kr.list_len, info.n_solid, thr, k, set,
+                           ep, ecap, su + S_EDGES)))
+      return rc;
+    launches += 2;
     if ((rc = fetch(S_EDGES + 1))) return rc;
     info.n_edges = host[S_EDGES];
     if (info.n_edges > ecap) return fail(SPK_E_CUDA, "edge list larger than its bound");
@@ -3916,29 +3876,19 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   // ---- edges ----
   kr.nle = (int)((k + 1 + 31) / 32);
   uint64_t ecap = 0;
-  DevBuf set, filt;
+  DevBuf set;
   if ((o.flags & SPK_F_EDGES) && info.n_solid > 0) {
     uint64_t* ep[4] = {nullptr, nullptr, nullptr, nullptr};
-    ecap = info.n_solid * 8;  // at most 8 canonical edges per solid k-mer
+    ecap = max_edges(info.n_solid);
     for (int j = 0; j < kr.nle; j++) {
       if ((rc = kr.edges[j].alloc(ecap * 8, st))) return rc;
       ep[j] = kr.edges[j].as<uint64_t>();
     }
-    uint32_t lg = 10, lf = 20;
-    while ((1ULL << lg) < info.n_solid + (info.n_solid >> 1) + 1) lg++;
-    while (lf < 30 && (1ULL << lf) < info.n_solid * 16) lf++;  // ~1/16 false positives
-    if ((rc = set.alloc((1ULL << lg) * nl * 8, st)) || (rc = filt.alloc((1ULL << lf) / 8, st))) return rc;
-    SPK_CUDA(cudaMemsetAsync(set.p, 0xFF, (1ULL << lg) * nl * 8, st));
-    SPK_CUDA(cudaMemsetAsync(filt.p, 0, (1ULL << lf) / 8, st));
-    SetView sv{set.as<uint64_t>(), lg, lf, filt.as<uint32_t>()};
-    launch_solid_set(ctx, st, nl, lp, kr.list[4].as<uint32_t>(), kr.list_len, thr, k, sv);
-    SPK_CUDA(cudaGetLastError());
-    launch_edges(ctx, st, nl, kr.nle, lp, kr.list[4].as<uint32_t>(), kr.list_len, thr, kr.table, &sv, k, ep,
-                 ecap, su + S_EDGES);
-    SPK_CUDA(cudaGetLastError());
+    if ((rc = launch_edges(ctx, st, nl, kr.nle, lp, kr.list[4].as<uint32_t>(), kr.list_len, info.n_solid, thr, k, set,
+                           ep, ecap, su + S_EDGES)))
+      return rc;
     launches += 2;
     set.release();
-    filt.release();
     if ((rc = sort_dev_enqueue(st, kr.nle, ecap, su + S_EDGES, 2 * (k + 1), kr.edges, nullptr, nullptr, esort,
                                &launches)))
       return rc;
