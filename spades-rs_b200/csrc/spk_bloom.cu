@@ -174,7 +174,7 @@ int bloom_insert(spk_bloom* b, const uint64_t* keys, size_t n, int wide, uint8_t
       (rc = dinit.alloc(ops, st)) || (rc = mk.alloc(mcap * 8, st)) || (rc = mv.alloc(mcap * 8, st)) ||
       (rc = dprom.alloc(n, st)))
     return rc;
-  SPK_CUDA(cudaMemcpyAsync(dk.p, keys, n * limbs * 8, cudaMemcpyHostToDevice, st));
+  if ((rc = xfer_h2d(ctx, dk.p, keys, n * limbs * 8, st))) return rc;
   SPK_CUDA(cudaMemsetAsync(mk.p, 0xFF, mcap * 8, st));
   SPK_CUDA(cudaMemsetAsync(mv.p, 0xFF, mcap * 8, st));
   BloomKeys K{dk.as<uint64_t>(), n, wide};
@@ -187,7 +187,7 @@ int bloom_insert(spk_bloom* b, const uint64_t* keys, size_t n, int wide, uint8_t
                                              mcap - 1, b->seen.as<unsigned long long>(),
                                              b->solid.as<unsigned long long>(), dprom.as<uint8_t>());
   SPK_CUDA(cudaGetLastError());
-  if (promoted) SPK_CUDA(cudaMemcpyAsync(promoted, dprom.p, n, cudaMemcpyDeviceToHost, st));
+  if (promoted && (rc = xfer_d2h(ctx, promoted, dprom.p, n, st))) return rc;
   SPK_CUDA(cudaStreamSynchronize(st));
   return SPK_OK;
 }
@@ -200,20 +200,21 @@ int bloom_query(spk_bloom* b, const uint64_t* keys, size_t n, int wide, uint8_t*
   DevBuf dk, dout;
   int rc;
   if ((rc = dk.alloc(n * limbs * 8, st)) || (rc = dout.alloc(n, st))) return rc;
-  SPK_CUDA(cudaMemcpyAsync(dk.p, keys, n * limbs * 8, cudaMemcpyHostToDevice, st));
+  if ((rc = xfer_h2d(ctx, dk.p, keys, n * limbs * 8, st))) return rc;
   BloomKeys K{dk.as<uint64_t>(), n, wide};
   k_api_query<<<grid_n(ctx, n), kB, 0, st>>>(K, b->fm, b->solid.as<unsigned long long>(),
                                              dout.as<uint8_t>());
   SPK_CUDA(cudaGetLastError());
-  SPK_CUDA(cudaMemcpyAsync(out, dout.p, n, cudaMemcpyDeviceToHost, st));
+  if ((rc = xfer_d2h(ctx, out, dout.p, n, st))) return rc;
   SPK_CUDA(cudaStreamSynchronize(st));
   return SPK_OK;
 }
 
 int bloom_download(spk_bloom* b, uint64_t* seen, uint64_t* solid) {
   cudaStream_t st = b->ctx->stream;
-  if (seen) SPK_CUDA(cudaMemcpyAsync(seen, b->seen.p, b->num_words * 8, cudaMemcpyDeviceToHost, st));
-  if (solid) SPK_CUDA(cudaMemcpyAsync(solid, b->solid.p, b->num_words * 8, cudaMemcpyDeviceToHost, st));
+  int rc;
+  if (seen && (rc = xfer_d2h(b->ctx, seen, b->seen.p, b->num_words * 8, st))) return rc;
+  if (solid && (rc = xfer_d2h(b->ctx, solid, b->solid.p, b->num_words * 8, st))) return rc;
   SPK_CUDA(cudaStreamSynchronize(st));
   return SPK_OK;
 }

@@ -302,16 +302,16 @@ extern "C" int spk_bloom_correct_reads(spk_bloom* bloom, uint32_t k, const uint8
       (rc = doff.alloc(std::max<size_t>(n_reads, 1) * 8, st)) ||
       (rc = dlen.alloc(std::max<size_t>(n_reads, 1) * 4, st)) || (rc = dcor.alloc(std::max<size_t>(n_reads, 1), st)))
     return rc;
-  if (data_len) SPK_CUDA(cudaMemcpyAsync(dd.p, data, data_len, cudaMemcpyHostToDevice, st));
+  if ((rc = xfer_h2d(ctx, dd.p, data, data_len, st))) return rc;
   if (n_reads) {
-    SPK_CUDA(cudaMemcpyAsync(doff.p, offsets, n_reads * 8, cudaMemcpyHostToDevice, st));
-    SPK_CUDA(cudaMemcpyAsync(dlen.p, lengths, n_reads * 4, cudaMemcpyHostToDevice, st));
+    if ((rc = xfer_h2d(ctx, doff.p, offsets, n_reads * 8, st))) return rc;
+    if ((rc = xfer_h2d(ctx, dlen.p, lengths, n_reads * 4, st))) return rc;
   }
   uint64_t nc = 0;
   if ((rc = correct_device(bloom, k, dd.as<uint8_t>(), data_len, doff.as<uint64_t>(), dlen.as<uint32_t>(), n_reads,
                            dout.as<uint8_t>(), dcor.as<uint8_t>(), &nc)))
     return rc;
-  if (data_len) SPK_CUDA(cudaMemcpyAsync(data_out, dout.p, data_len, cudaMemcpyDeviceToHost, st));
+  if ((rc = xfer_d2h(ctx, data_out, dout.p, data_len, st))) return rc;
   if (corrected && n_reads) SPK_CUDA(cudaMemcpyAsync(corrected, dcor.p, n_reads, cudaMemcpyDeviceToHost, st));
   SPK_CUDA(cudaStreamSynchronize(st));
   if (n_corrected) *n_corrected = nc;

@@ -4161,11 +4161,12 @@ int download_bloom(spk_result* res, int ki, uint64_t* seen, uint64_t* twice, uin
   cudaStream_t st = res->stream;
   if (!kr.seen.p) return fail(SPK_E_INVALID_ARG, "Bloom tiers were not kept (SPK_F_KEEP_BLOOM)");
   const uint64_t n = kr.num_words;
-  if (seen) SPK_CUDA(cudaMemcpyAsync(seen, kr.seen.p, n * 8, cudaMemcpyDeviceToHost, st));
-  if (twice) SPK_CUDA(cudaMemcpyAsync(twice, kr.twice.p, n * 8, cudaMemcpyDeviceToHost, st));
+  int rc;
+  if (seen && (rc = xfer_d2h(res->ctx, seen, kr.seen.p, n * 8, st))) return rc;
+  if (twice && (rc = xfer_d2h(res->ctx, twice, kr.twice.p, n * 8, st))) return rc;
   if (ref_solid) {
     if (!kr.ref_solid.p) return fail(SPK_E_INVALID_ARG, "reference solid tier not built (SPK_F_REF_SOLID)");
-    SPK_CUDA(cudaMemcpyAsync(ref_solid, kr.ref_solid.p, n * 8, cudaMemcpyDeviceToHost, st));
+    if ((rc = xfer_d2h(res->ctx, ref_solid, kr.ref_solid.p, n * 8, st))) return rc;
   }
   SPK_CUDA(cudaStreamSynchronize(st));
   return SPK_OK;

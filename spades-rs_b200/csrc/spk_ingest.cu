@@ -543,7 +543,7 @@ static int ig_text(spk_ctx* ctx, cudaStream_t st, const uint8_t* host, uint64_t 
   const uint64_t n = n_all - off;
   if (n >= 0xFFFFFFF0ull) return fail(SPK_E_INVALID_ARG, "a FASTQ/FASTA text of 4 GiB or more");
   if ((rc = T.text.alloc(n + 64, st))) return rc;
-  SPK_CUDA(cudaMemcpyAsync(T.text.p, host + off, n, cudaMemcpyHostToDevice, st));
+  if ((rc = xfer_h2d(ctx, T.text.p, host + off, n, st))) return rc;
   const uint8_t* t = T.text.as<uint8_t>();
   DevBuf cnt, sums, err;
   const uint32_t nchunks = (uint32_t)((n + kIgChunk - 1) / kIgChunk);
@@ -774,11 +774,10 @@ extern "C" int spk_packed_download(spk_packed* p, uint8_t* data, uint64_t* offse
   if (!p) return fail(SPK_E_INVALID_ARG, "null packed reads");
   SPK_CUDA(cudaSetDevice(p->ctx->device));
   cudaStream_t st = p->ctx->stream;
-  if (data && p->data_len) SPK_CUDA(cudaMemcpyAsync(data, p->data.p, p->data_len, cudaMemcpyDeviceToHost, st));
-  if (offsets && p->n_reads)
-    SPK_CUDA(cudaMemcpyAsync(offsets, p->offsets.p, p->n_reads * 8, cudaMemcpyDeviceToHost, st));
-  if (lengths && p->n_reads)
-    SPK_CUDA(cudaMemcpyAsync(lengths, p->lengths.p, p->n_reads * 4, cudaMemcpyDeviceToHost, st));
+  int rc;
+  if (data && (rc = xfer_d2h(p->ctx, data, p->data.p, p->data_len, st))) return rc;
+  if (offsets && (rc = xfer_d2h(p->ctx, offsets, p->offsets.p, p->n_reads * 8, st))) return rc;
+  if (lengths && (rc = xfer_d2h(p->ctx, lengths, p->lengths.p, p->n_reads * 4, st))) return rc;
   SPK_CUDA(cudaStreamSynchronize(st));
   if (sidecar && !p->sidecar.empty()) memcpy(sidecar, p->sidecar.data(), p->sidecar.size());
   if (sidecar_lengths && !p->sidecar_len.empty())
