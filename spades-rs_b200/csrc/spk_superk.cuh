@@ -67,9 +67,16 @@ __device__ __forceinline__ uint32_t sk_bin(uint32_t h, uint32_t nbins) {
   return __umulhi(g, nbins);
 }
 
-// One warp per read, 32 R m-mer positions at a time (position p of the segment
-// in register p / 32 of lane p % 32).  The sliding minimum over the w = k - m + 1
-// m-mers of a window doubles its reach with log2(w) exchanges of neighbours.
+template <int V>
+struct SkInt {
+  static constexpr int value = V;
+};
+// One warp per read, 32 R m-mer positions at a time, R neighbouring ones per lane.
+// The sliding minimum over the w = k - m + 1 m-mers of a window doubles its reach
+// with log2(w) steps.  Bound by issue (about 350 instructions a read of 150 bases):
+// with a lane's positions side by side, most of the first steps stay inside the
+// lane and the others are one exchange per position (32 apart, each step took an
+// exchange and a select per position, 440 instructions).
 // rpw: reads a warp takes at a time (at most 32).
 template <int R>
 __global__ void __launch_bounds__(kSkReadBlock) k_sk_reads(ReadsView rd, unsigned k, unsigned m, uint32_t rpw,
@@ -79,7 +86,7 @@ __global__ void __launch_bounds__(kSkReadBlock) k_sk_reads(ReadsView rd, unsigne
   const unsigned msh = 32 - 2 * m;
   unsigned p2 = 1;  // largest power of two <= w
   while (2 * p2 <= w) p2 *= 2;
-  const unsigned d = w - p2, dr = d >> 5, ds = d & 31;
+  const unsigned dr = (w - p2) % R, dq = (w - p2) / R;
   uint64_t occ = 0;
   uint64_t cur = 0;   // this warp's reserved stream entries
   uint32_t rem = 0;
@@ -133,70 +140,67 @@ __global__ void __launch_bounds__(kSkReadBlock) k_sk_reads(ReadsView rd, unsigne
       for (uint32_t a = 0; a < nwin; a += seg) {
         const uint32_t nw = min(seg, nwin - a), nm = nw + w - 1;
         const uint64_t base = base0 + a, bit0 = 2 * base;
-        const unsigned s = (unsigned)(bit0 & 63);
         const uint64_t* p = rd.words + (bit0 >> 6);
+        const uint32_t s = (uint32_t)(bit0 & 63);
         const uint32_t need = s + 2 * (nm + m - 1);  // bits from p that the segment covers
-        uint64_t A[R + 1];
-        {
-          uint64_t u = bswap64(__ldg(p));
-#pragma unroll
-          for (int r = 0; r <= R; r++) {
-            const uint64_t v = 64u * (r + 1) < need ? bswap64(__ldg(p + r + 1)) : 0ULL;
-            A[r] = shl2(u, v, s);
-            u = v;
-          }
-        }
+        // the lane's R positions: the 32 bases from its first
+        const uint32_t lb = s + 2 * R * lane, wi = lb >> 6;
+        const uint64_t u = R * lane < nm ? bswap64(__ldg(p + wi)) : 0ULL;
+        const uint64_t v = 64 * (wi + 1) < need ? bswap64(__ldg(p + wi + 1)) : 0ULL;
+        const uint64_t x = shl2(u, v, lb & 63);
         uint32_t M[R], T[R];
 #pragma unroll
         for (int r = 0; r < R; r++) {
-          // the 16 bases from position 32 r + lane
-          const uint32_t x0 = (uint32_t)(A[r] >> 32), x1 = (uint32_t)A[r], x2 = (uint32_t)(A[r + 1] >> 32);
-          const uint32_t v = __funnelshift_l(lane < 16 ? x1 : x2, lane < 16 ? x0 : x1, (2 * lane) & 31) >> msh;
-          uint32_t z = __brev(~(v << msh) & (~0u << msh));  // the complement, bits reversed: low 2m bits
+          const uint32_t f = __funnelshift_l((uint32_t)x, (uint32_t)(x >> 32), 2 * r) >> msh;
+          uint32_t z = __brev(~(f << msh) & (~0u << msh));  // the complement, bits reversed: low 2m bits
           z = ((z >> 1) & 0x55555555u) | ((z & 0x55555555u) << 1);
-          const uint32_t h = sk_hash(min(v, z));
-          M[r] = 32u * r + lane < nm ? h : 0xFFFFFFFFu;
+          const uint32_t h = sk_hash(min(f, z));
+          M[r] = R * lane + r < nm ? h : 0xFFFFFFFFu;
         }
+        // M[r]: the minimum of the e m-mers from its position.  (What comes from
+        // past lane 31 reaches no window of the segment.)
+        auto reach = [&](auto at, unsigned q0) {  // ... and of as many `at` + R q0 positions on
+          constexpr int A = decltype(at)::value;
 #pragma unroll
-        for (unsigned e = 1; e <= 16; e *= 2) {
-          if (2 * e > w) break;
-#pragma unroll
-          for (int r = 0; r < R; r++) T[r] = __shfl_sync(FULL, M[r], (lane + e) & 31);
-#pragma unroll
-          for (int r = 0; r < R; r++)
-            M[r] = min(M[r], lane + e < 32 ? T[r] : r + 1 < R ? T[r + 1 < R ? r + 1 : r] : 0xFFFFFFFFu);
-        }
-        if (64 <= w) {
-#pragma unroll
-          for (int r = 0; r + 1 < R; r++) M[r] = min(M[r], M[r + 1]);
-        }
-        if (d) {
-#pragma unroll
-          for (int r = 0; r < R; r++) T[r] = __shfl_sync(FULL, M[r], (lane + ds) & 31);
-          if (dr == 0) {
-#pragma unroll
-            for (int r = 0; r < R; r++)
-              M[r] = min(M[r], lane + ds < 32 ? T[r] : r + 1 < R ? T[r + 1 < R ? r + 1 : r] : 0xFFFFFFFFu);
-          } else {
-#pragma unroll
-            for (int r = 0; r < R; r++)
-              M[r] = min(M[r], lane + ds < 32 ? (r + 1 < R ? T[r + 1 < R ? r + 1 : r] : 0xFFFFFFFFu)
-                                              : (r + 2 < R ? T[r + 2 < R ? r + 2 : r] : 0xFFFFFFFFu));
+          for (int r = 0; r < R; r++) {
+            const unsigned q = q0 + (r + A) / R;
+            T[r] = M[(r + A) % R];
+            if ((r + A) / R || q0) T[r] = __shfl_down_sync(FULL, T[r], q);
           }
+#pragma unroll
+          for (int r = 0; r < R; r++) M[r] = min(M[r], T[r]);
+        };
+        if (w >= 2) reach(SkInt<1 % R>{}, 1 / R);
+        if (w >= 4) reach(SkInt<2 % R>{}, 2 / R);
+        if (w >= 8) reach(SkInt<4 % R>{}, 4 / R);
+        if (w >= 16) reach(SkInt<8 % R>{}, 8 / R);
+        if (w >= 32) reach(SkInt<16 % R>{}, 16 / R);
+        if (w >= 64) reach(SkInt<32 % R>{}, 32 / R);
+        switch (dr) {  // the last d = w - p2 positions: d = dr + R dq
+          case 0: if (dq) reach(SkInt<0>{}, dq); break;
+          case 1: reach(SkInt<1>{}, dq); break;
+          case 2: reach(SkInt<2>{}, dq); break;
+          case 3: reach(SkInt<(R > 3 ? 3 : 0)>{}, dq); break;
+          case 4: reach(SkInt<(R > 4 ? 4 : 0)>{}, dq); break;
+          case 5: reach(SkInt<(R > 5 ? 5 : 0)>{}, dq); break;
+          case 6: reach(SkInt<(R > 6 ? 6 : 0)>{}, dq); break;
+          default: reach(SkInt<(R > 7 ? 7 : 0)>{}, dq); break;
         }
         // runs of equal minima among the segment's nw windows: their first
         // windows and minima side by side in shared memory, then a lane per run
-#pragma unroll
-        for (int r = 0; r < R; r++) T[r] = __shfl_sync(FULL, M[r], (lane + 31) & 31);
-        uint32_t nruns = 0;
+        const uint32_t left = __shfl_up_sync(FULL, M[R - 1], 1);
+        uint32_t nruns = 0, at = 0, starts = 0;
 #pragma unroll
         for (int r = 0; r < R; r++) {
-          const uint32_t pv = lane ? T[r] : r ? T[r ? r - 1 : 0] : ~M[0];
-          const bool start = 32u * r + lane < nw && M[r] != pv;
+          const bool start = R * lane + r < nw && (M[r] != (r ? M[r ? r - 1 : 0] : left) || (r == 0 && lane == 0));
           const unsigned mk = __ballot_sync(FULL, start);
-          if (start) runs[nruns + __popc(mk & lanemask_lt())] = make_uint2(32u * r + lane, M[r]);
+          starts |= (start ? 1u : 0u) << r;
           nruns += __popc(mk);
+          at += __popc(mk & lanemask_lt());
         }
+#pragma unroll
+        for (int r = 0; r < R; r++)
+          if (starts >> r & 1) runs[at++] = make_uint2(R * lane + r, M[r]);
         if (lane == 0) runs[nruns] = make_uint2(nw, 0);
         __syncwarp();
         for (uint32_t t0 = 0; t0 < nruns; t0 += 32) {
