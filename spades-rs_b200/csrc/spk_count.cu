@@ -2154,38 +2154,55 @@ __global__ void __launch_bounds__(256) k_count_solid(const uint32_t* __restrict_
   warp_add_u64(out, s);
 }
 
-// out: [0] cutoff, [1] list threshold
+// out: [0] cutoff, [1] list threshold.  One warp, eight bins per lane (the whole
+// rule on one thread waited for its 256 reads one after another: 8 to 15 us).
 __global__ void k_cutoff(const unsigned long long* __restrict__ hist, uint32_t fixed,
                          uint32_t list_min, uint32_t* __restrict__ out) {
-  if (threadIdx.x | blockIdx.x) return;
+  const unsigned lane = threadIdx.x & 31;
+  constexpr int PER = kHistBins / 32;
+  __shared__ unsigned long long h[kHistBins];
+  unsigned long long sum = 0;
+#pragma unroll
+  for (int j = 0; j < PER; j++) {
+    const unsigned long long v = hist[lane * PER + j];
+    h[lane * PER + j] = v;
+    sum += v;
+  }
+  unsigned long long x = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const unsigned long long y = __shfl_up_sync(FULL, x, d);
+    if ((int)lane >= d) x += y;
+  }
+  const unsigned long long n = __shfl_sync(FULL, x, 31);
+  __syncwarp();
   uint32_t cutoff = 2;
   if (fixed) {
     cutoff = fixed;
-  } else {
-    unsigned long long n = 0;
-    for (int c = 0; c < kHistBins; c++) n += hist[c];
-    if (n > 100) {
-      const unsigned long long rank = n * 95 / 100;
-      unsigned long long cum = 0;
-      uint32_t top = kHistBins - 1;  // bin 255 means >= 255
-      for (int c = 0; c < kHistBins; c++) {
-        cum += hist[c];
-        if (cum > rank) { top = c; break; }
+  } else if (n > 100) {
+    const unsigned long long rank = n * 95 / 100;
+    unsigned long long cum = x - sum;
+    uint32_t top = kHistBins - 1;  // bin 255 means >= 255
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+      cum += h[lane * PER + j];
+      if (cum > rank && top == kHistBins - 1) top = min(top, lane * PER + j);
+    }
+    top = __reduce_min_sync(FULL, top);  // the first bin whose cumulative count passes the rank
+    if (top >= 30) {
+      uint32_t mvs = min(max(top / 4, 10u), 35u);
+      uint32_t valley = 2;
+      unsigned long long min_val = ~0ULL;
+      bool found = false;
+      for (uint32_t c = 2; c <= mvs; c++) {
+        unsigned long long v = h[c];
+        if (v <= min_val) { min_val = v; valley = c; }
+        else if (v > min_val * 2 && c > valley + 2) { found = true; break; }
       }
-      if (top >= 30) {
-        uint32_t mvs = min(max(top / 4, 10u), 35u);
-        uint32_t valley = 2;
-        unsigned long long min_val = ~0ULL;
-        bool found = false;
-        for (uint32_t c = 2; c <= mvs; c++) {
-          unsigned long long h = hist[c];
-          if (h <= min_val) { min_val = h; valley = c; }
-          else if (h > min_val * 2 && c > valley + 2) { found = true; break; }
-        }
-        cutoff = found ? valley : 2;
-      }
+      cutoff = found ? valley : 2;
     }
   }
+  if (lane) return;
   out[0] = cutoff;
   out[1] = max(1u, min(cutoff, list_min));
 }
@@ -2300,13 +2317,12 @@ __device__ __forceinline__ bool set_has(const SetView& sv, const Seq<NL>& C, uin
 // end where it is its own canonical form (four of a solid k-mer's eight on
 // average), the filter words of all of those are read together, and only the few
 // that pass (one and a quarter on average) go on to the set, one after another.
-constexpr int kEdgeRounds = 4;  // k-mers per thread and reservation
+constexpr int kEdgeRounds = 4;  // most k-mers per thread and reservation
 template <int NL, int NLE>
 __global__ void __launch_bounds__(kBlock) k_edges(const uint32_t* __restrict__ cnt, uint64_t n,
-                                                   const uint32_t* __restrict__ thr, SetView sv, unsigned k,
+                                                   const uint32_t* __restrict__ thr, SetView sv, unsigned k, int U,
                                                    uint64_t* e0, uint64_t* e1, uint64_t* e2, uint64_t* e3,
                                                    uint64_t out_cap, unsigned long long* __restrict__ counter) {
-  constexpr int U = kEdgeRounds;
   __shared__ uint32_t wsum[kBlock / 32];
   __shared__ unsigned long long s_base;
   const uint32_t cutoff = thr[0];
@@ -2508,6 +2524,10 @@ __global__ void __launch_bounds__(kBlock) k_read_order(const uint64_t* __restric
 // Host side
 // ---------------------------------------------------------------------------
 static int grid_for(spk_ctx* ctx, int blocks_per_sm) { return ctx->sm_count * blocks_per_sm; }
+// ... and at most one block per `per` of n items.
+static int grid_items(spk_ctx* ctx, int blocks_per_sm, uint64_t n, uint64_t per) {
+  return (int)std::max<uint64_t>(std::min<uint64_t>((n + per - 1) / per, (uint64_t)grid_for(ctx, blocks_per_sm)), 1);
+}
 
 // F<NL>(args...) for the key width nl at run time (F returns a status).
 #define SPK_NL_CALL(nl, F, ...)                                                              \
@@ -2650,9 +2670,11 @@ template <int NL, int NLE>
 static void launch_edges_t(spk_ctx* ctx, cudaStream_t st, const uint32_t* cnt, uint64_t n, const uint32_t* thr,
                            const SetView& sv, unsigned k, uint64_t* e[4], uint64_t out_cap,
                            unsigned long long* counter) {
-  k_solid_set<NL><<<grid_for(ctx, 8), kBlock, 0, st>>>(cnt, n, thr, sv);
-  k_edges<NL, NLE><<<grid_for(ctx, 8), kBlock, 0, st>>>(cnt, n, thr, sv, k, e[0], e[1], e[2], e[3], out_cap,
-                                                       counter);
+  k_solid_set<NL><<<grid_items(ctx, 8, n, kBlock), kBlock, 0, st>>>(cnt, n, thr, sv);
+  // (a list that does not fill the device four k-mers a thread takes them one by one)
+  const int U = n >= (uint64_t)grid_for(ctx, 8) * kBlock * kEdgeRounds / 2 ? kEdgeRounds : 1;
+  k_edges<NL, NLE><<<grid_items(ctx, 8, n, (uint64_t)U * kBlock), kBlock, 0, st>>>(cnt, n, thr, sv, k, U, e[0], e[1], e[2],
+                                                                                  e[3], out_cap, counter);
 }
 // The solid k-mers of the list l (n entries, n_solid of them solid) as a set and
 // their edges, unsorted; `set` is the set's memory.
@@ -2660,8 +2682,10 @@ static int launch_edges(spk_ctx* ctx, cudaStream_t st, int nl, int nle, uint64_t
                         uint64_t n, uint64_t n_solid, const uint32_t* thr, unsigned k, DevBuf& set, uint64_t* e[4],
                         uint64_t out_cap, unsigned long long* counter) {
   if (n >= 0xFFFFFFFFULL) return fail(SPK_E_INVALID_ARG, "edges: more than 2^32 listed k-mers");
+  // at most 2/3 full; a third where the slots are a small part of L2 anyway (the
+  // longest chain of claims, not the traffic, bounds a small set: 24 us for 10 k)
   uint32_t lg = 10;
-  while ((1ULL << lg) < n_solid + (n_solid >> 1) + 1) lg++;
+  while ((1ULL << lg) < (n_solid < (1u << 20) ? 3 * n_solid : n_solid + (n_solid >> 1)) + 1) lg++;
   uint32_t lf = 15;
   while (lf < 31 && (1ULL << lf) < n_solid * 16) lf++;  // ~1/16 false positives
   const size_t slot_bytes = (size_t)8 << lg, filter_bytes = (size_t)1 << (lf - 3);
@@ -3637,7 +3661,6 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   // Buffers of the span count, filled over every group's pass (allocated
   // after the first group's partition, when a single group has freed its
   // coarse buckets, so that they never coexist).
-  const bool early_sort = lmin_pre >= 2;
   DevSort lsort, esort;
   DevBuf rbase, rfill, ops, sgl[4];
   RangeView bv{};
@@ -3778,15 +3801,6 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
     SPK_CUDA(cudaGetLastError());
     launches++;
   }
-  if (early_sort) {
-    // The list is final (singletons are not listed): sorted here, while the
-    // host waits for the readback below, with the singleton buffers as
-    // temporaries.  On a second stream beside the Bloom and admission kernels
-    // (which read the tier from L2 that the sort's scattered writes evict) the
-    // three took 3.2 ms at 5 Mb x 100x, k = 55, one after another 1.95.
-    if ((rc = sort_dev_enqueue(st, nl, lcap_, su + S_LFILL, 2 * k, kr.list, &kr.list[4], sgl, lsort, &launches)))
-      return rc;
-  }
   uint32_t* thr = (uint32_t*)(sw + S_THR);
   k_cutoff<<<1, 32, 0, st>>>(su + S_HIST, fixed, list_min, thr);
   SPK_CUDA(cudaGetLastError());
@@ -3846,10 +3860,11 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   }
   SPK_CUDA(cudaEventRecord(e3.e, st));
 
-  // ---- sort of the list, unless it ran early (the singleton buffers, read by
-  // admission, are its temporaries here) ----
-  if (!early_sort &&
-      (rc = sort_dev_enqueue(st, nl, kr.list_len, nullptr, 2 * k, kr.list, &kr.list[4], sgl, lsort, &launches)))
+  // ---- sort of the list, into buffers of its size (the singleton buffers,
+  // read by admission, are its temporaries).  On a second stream beside the Bloom
+  // and admission kernels, whose tier its scattered writes evict from L2, the
+  // three took 3.2 ms at 5 Mb x 100x, k = 55, one after another 1.95. ----
+  if ((rc = sort_dev_enqueue(st, nl, kr.list_len, nullptr, 2 * k, kr.list, &kr.list[4], sgl, true, lsort, &launches)))
     return rc;
   uint64_t* lp[4] = {nullptr, nullptr, nullptr, nullptr};
   for (int j = 0; j < nl; j++) lp[j] = kr.list[j].as<uint64_t>();
@@ -3889,7 +3904,7 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
       return rc;
     launches += 2;
     set.release();
-    if ((rc = sort_dev_enqueue(st, kr.nle, ecap, su + S_EDGES, 2 * (k + 1), kr.edges, nullptr, nullptr, esort,
+    if ((rc = sort_dev_enqueue(st, kr.nle, ecap, su + S_EDGES, 2 * (k + 1), kr.edges, nullptr, nullptr, false, esort,
                                &launches)))
       return rc;
   }
@@ -3919,6 +3934,14 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   if (info.n_edges > ecap) return fail(SPK_E_CUDA, "edge list larger than its bound");
   const unsigned nbig_l = hb[0], nbig_e = hb[1];
   if ((rc = sort_dev_finish(st, lsort, kr.list, &kr.list[4], kr.list_len, nbig_l, host, &launches))) return rc;
+  if (nbig_l && want_solid) {  // the list was not in order yet when its solid k-mers were copied
+    uint64_t m = kr.conv.n;
+    if ((rc = ordered_convert(st, nl, kr.list_len, k, kr.list, kr.list[4].as<uint32_t>(), info.cutoff, &kr.conv.keys,
+                              &kr.conv.cnt, host, &m, m)))
+      return rc;
+    if (m && o.solid_keys_out && (rc = xfer_d2h(ctx, o.solid_keys_out, kr.conv.keys.p, m * nl * 8, st))) return rc;
+    if (m && o.solid_counts_out && (rc = xfer_d2h(ctx, o.solid_counts_out, kr.conv.cnt.p, m * 4, st))) return rc;
+  }
   if ((rc = sort_dev_finish(st, esort, kr.edges, nullptr, info.n_edges, nbig_e, host, &launches))) return rc;
   if ((rc = keep_results(kr, st, o.flags))) return rc;
   SPK_CUDA(cudaEventRecord(e6.e, st));

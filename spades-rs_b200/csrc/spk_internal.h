@@ -309,7 +309,7 @@ struct DevSort {
   }
 };
 int sort_dev_enqueue(cudaStream_t st, int nl, uint64_t n_cap, const unsigned long long* n_dev,
-                     unsigned nbits, DevBuf* keys, DevBuf* vals, DevBuf* tmp_keys, DevSort& ds,
+                     unsigned nbits, DevBuf* keys, DevBuf* vals, DevBuf* tmp_keys, bool exact, DevSort& ds,
                      uint32_t* launches = nullptr);
 // Device word counting the buckets left for sort_dev_finish.
 const unsigned* sort_dev_nbig(const DevSort& ds);

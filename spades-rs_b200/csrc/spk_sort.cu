@@ -136,7 +136,33 @@ __global__ void __launch_bounds__(SC_BLOCK) k_scan_apply(uint32_t* __restrict__ 
   }
 }
 
+// Short arrays by one block of 1024 threads, up to 16 items each: one launch of
+// about 4 us where the three above take 9 with their gaps.
+constexpr uint64_t SC_SMALL = 16384;
+__global__ void __launch_bounds__(1024) k_scan_small(uint32_t* __restrict__ a, uint32_t n) {
+  __shared__ uint32_t ws[32];
+  const uint32_t ipt = (n + 1023) / 1024, base = threadIdx.x * ipt;
+  uint32_t v[SC_SMALL / 1024], s = 0;
+#pragma unroll
+  for (uint32_t j = 0; j < SC_SMALL / 1024; j++) {
+    v[j] = j < ipt && base + j < n ? a[base + j] : 0u;
+    s += v[j];
+  }
+  uint32_t run = block_excl_scan(s, ws, nullptr);
+#pragma unroll
+  for (uint32_t j = 0; j < SC_SMALL / 1024; j++) {
+    if (j < ipt && base + j < n) a[base + j] = run;
+    run += v[j];
+  }
+}
+
 int scan_u32(cudaStream_t st, uint32_t* a, uint64_t n, DevBuf& sums, uint32_t* launches) {
+  if (n <= SC_SMALL) {
+    k_scan_small<<<1, 1024, 0, st>>>(a, (uint32_t)n);
+    SPK_CUDA(cudaGetLastError());
+    if (launches) *launches += 1;
+    return SPK_OK;
+  }
   const uint64_t nb = (n + SC_CHUNK - 1) / SC_CHUNK;
   int rc;
   if (sums.bytes < nb * 4 && (rc = sums.alloc(nb * 4, st))) return rc;
@@ -372,12 +398,13 @@ __global__ void __launch_bounds__(BS_BLOCK) k_bs_coarse(Limbs L, uint64_t n, con
   __syncthreads();
   if (!last) return;
   __threadfence();
-  const uint64_t per = max((uint64_t)BS_PER, (n + BS_MAX_BUCKETS - 1) / BS_MAX_BUCKETS);
+  const uint32_t per = (uint32_t)max((uint64_t)BS_PER, (n + BS_MAX_BUCKETS - 1) / BS_MAX_BUCKETS);
   constexpr uint32_t IPT = BS_COARSE / BS_BLOCK;
   uint32_t v[IPT], s = 0;
 #pragma unroll
   for (uint32_t j = 0; j < IPT; j++) {
-    v[j] = (uint32_t)((__ldcg(W.coarse + threadIdx.x * IPT + j) + per - 1) / per);
+    const uint32_t c = __ldcg(W.coarse + threadIdx.x * IPT + j);
+    v[j] = c / per + (c % per != 0);
     s += v[j];
   }
   uint32_t tot, run = block_excl_scan(s, ws, &tot);
@@ -643,15 +670,16 @@ static void launch_segments(cudaStream_t st, bool hasv, Limbs L, uint32_t* lv, L
   else k_bs_segments<NL, false><<<nseg, BS_BLOCK, 0, st>>>(L, lv, C, cv, seg, back);
 }
 
+// K, v: the list; T, tv: its bucketed copy; D, dv: the sorted list (may be K, v).
 template <int NL, bool HASV>
-static int bs_launch(cudaStream_t st, Limbs K, uint32_t* v, Limbs T, uint32_t* tv, uint64_t n,
+static int bs_launch(cudaStream_t st, Limbs K, uint32_t* v, Limbs T, uint32_t* tv, Limbs D, uint32_t* dv, uint64_t n,
                      const unsigned long long* n_dev, unsigned nbits, const BsWork& W, uint32_t* launches) {
   const int sms = current_sm_count();
   const uint32_t nb = bs_max_buckets(n);
   const unsigned g = (unsigned)std::max<uint64_t>(
       std::min<uint64_t>((n + BS_BLOCK - 1) / BS_BLOCK, (uint64_t)sms * 16), 1);
   // (a CTA of the coarse count flushes its 4,096 bins: a few CTAs per SM)
-  const unsigned gc = (unsigned)std::max<uint64_t>(std::min<uint64_t>(n / 4096, (uint64_t)sms * 4), 1);
+  const unsigned gc = (unsigned)std::max<uint64_t>(std::min<uint64_t>(n / 1024, (uint64_t)sms * 4), 1);
   k_bs_coarse<NL><<<gc, BS_BLOCK, 0, st>>>(K, n, n_dev, nbits, W);
   k_bs_hist<NL><<<g, BS_BLOCK, 0, st>>>(K, n, n_dev, nbits, W);
   DevBuf sums;
@@ -661,23 +689,23 @@ static int bs_launch(cudaStream_t st, Limbs K, uint32_t* v, Limbs T, uint32_t* t
   const size_t smem = BS_LOCAL * (NL * 8 + (HASV ? 4 : 0));
   if ((rc = raise_smem_limit((const void*)k_bs_local<NL, HASV>, smem))) return rc;
   const unsigned gl = (unsigned)std::min<uint32_t>((nb + BS_CHUNK - 1) / BS_CHUNK, (uint32_t)sms * 8);
-  k_bs_local<NL, HASV><<<gl, BS_BLOCK, smem, st>>>(T, tv, K, v, W);
+  k_bs_local<NL, HASV><<<gl, BS_BLOCK, smem, st>>>(T, tv, D, dv, W);
   SPK_CUDA(cudaGetLastError());
   if (launches) *launches += 4;
   return SPK_OK;
 }
 static int bs_launch_nl(int nl, bool hasv, cudaStream_t st, Limbs K, uint32_t* v, Limbs T, uint32_t* tv,
-                        uint64_t n, const unsigned long long* n_dev, unsigned nbits, const BsWork& W,
+                        Limbs D, uint32_t* dv, uint64_t n, const unsigned long long* n_dev, unsigned nbits, const BsWork& W,
                         uint32_t* launches) {
   switch (nl * 2 + (hasv ? 1 : 0)) {
-    case 2: return bs_launch<1, false>(st, K, v, T, tv, n, n_dev, nbits, W, launches);
-    case 3: return bs_launch<1, true>(st, K, v, T, tv, n, n_dev, nbits, W, launches);
-    case 4: return bs_launch<2, false>(st, K, v, T, tv, n, n_dev, nbits, W, launches);
-    case 5: return bs_launch<2, true>(st, K, v, T, tv, n, n_dev, nbits, W, launches);
-    case 6: return bs_launch<3, false>(st, K, v, T, tv, n, n_dev, nbits, W, launches);
-    case 7: return bs_launch<3, true>(st, K, v, T, tv, n, n_dev, nbits, W, launches);
-    case 8: return bs_launch<4, false>(st, K, v, T, tv, n, n_dev, nbits, W, launches);
-    default: return bs_launch<4, true>(st, K, v, T, tv, n, n_dev, nbits, W, launches);
+    case 2: return bs_launch<1, false>(st, K, v, T, tv, D, dv, n, n_dev, nbits, W, launches);
+    case 3: return bs_launch<1, true>(st, K, v, T, tv, D, dv, n, n_dev, nbits, W, launches);
+    case 4: return bs_launch<2, false>(st, K, v, T, tv, D, dv, n, n_dev, nbits, W, launches);
+    case 5: return bs_launch<2, true>(st, K, v, T, tv, D, dv, n, n_dev, nbits, W, launches);
+    case 6: return bs_launch<3, false>(st, K, v, T, tv, D, dv, n, n_dev, nbits, W, launches);
+    case 7: return bs_launch<3, true>(st, K, v, T, tv, D, dv, n, n_dev, nbits, W, launches);
+    case 8: return bs_launch<4, false>(st, K, v, T, tv, D, dv, n, n_dev, nbits, W, launches);
+    default: return bs_launch<4, true>(st, K, v, T, tv, D, dv, n, n_dev, nbits, W, launches);
   }
 }
 
@@ -700,7 +728,7 @@ int sort_bufs(cudaStream_t st, int nl, uint64_t n, unsigned nbits, DevBuf* keys,
   const BsWork W = bs_work(work.as<uint32_t>());
   uint32_t* v = vals ? vals->as<uint32_t>() : nullptr;
   uint32_t* tvp = vals ? tv.as<uint32_t>() : nullptr;
-  if ((rc = bs_launch_nl(nl, vals != nullptr, st, K, v, T, tvp, n, nullptr, nbits, W, launches))) return rc;
+  if ((rc = bs_launch_nl(nl, vals != nullptr, st, K, v, T, tvp, K, v, n, nullptr, nbits, W, launches))) return rc;
   uint64_t* hs = h_staging + BS_STAGE_WORDS;
   SPK_CUDA(cudaMemcpyAsync(hs, W.nbig, 4, cudaMemcpyDeviceToHost, st));
   SPK_CUDA(cudaStreamSynchronize(st));
@@ -740,9 +768,11 @@ int sort_bufs(cudaStream_t st, int nl, uint64_t n, unsigned nbits, DevBuf* keys,
 // reading anything back.  Buckets over BS_LOCAL items stay in the bucketed
 // copy and are listed on the device; sort_dev_finish sorts them once the
 // host has the counts.  Temporaries: tmp_keys (nullable, NL limb arrays of
-// n_cap items that the caller no longer needs) or new allocations.
+// n_cap items that the caller no longer needs) or new allocations.  exact: n_cap
+// is the length, and the sorted list goes to new buffers of its size that a result
+// keeps (keys and vals then hold those).
 int sort_dev_enqueue(cudaStream_t st, int nl, uint64_t n_cap, const unsigned long long* n_dev,
-                     unsigned nbits, DevBuf* keys, DevBuf* vals, DevBuf* tmp_keys, DevSort& ds,
+                     unsigned nbits, DevBuf* keys, DevBuf* vals, DevBuf* tmp_keys, bool exact, DevSort& ds,
                      uint32_t* launches) {
   if (n_cap >= (1ULL << 32)) return fail(SPK_E_INVALID_ARG, "sort: more than 2^32 items");
   ds.nl = nl;
@@ -762,9 +792,24 @@ int sort_dev_enqueue(cudaStream_t st, int nl, uint64_t n_cap, const unsigned lon
   SPK_CUDA(cudaMemsetAsync(ds.work.p, 0, bs_work_bytes(n_cap), st));
   uint32_t* v = vals ? vals->as<uint32_t>() : nullptr;
   uint32_t* tvp = vals ? ds.tv.as<uint32_t>() : nullptr;
-  if ((rc = bs_launch_nl(nl, vals != nullptr, st, K, v, T, tvp, n_cap, n_dev, nbits,
+  DevBuf dk[4], dvb;
+  Limbs D = K;
+  uint32_t* dv = v;
+  if (exact) {
+    for (int j = 0; j < nl; j++) {
+      if ((rc = dk[j].alloc_keep(std::max<uint64_t>(n_cap, 2) * 8, st))) return rc;
+      D.p[j] = dk[j].as<uint64_t>();
+    }
+    if (vals && (rc = dvb.alloc_keep(std::max<uint64_t>(n_cap, 4) * 4, st))) return rc;
+    if (vals) dv = dvb.as<uint32_t>();
+  }
+  if ((rc = bs_launch_nl(nl, vals != nullptr, st, K, v, T, tvp, D, dv, n_cap, n_dev, nbits,
                          bs_work(ds.work.as<uint32_t>()), launches)))
     return rc;
+  if (exact) {  // (the old buffers are freed after the sort, in stream order)
+    for (int j = 0; j < nl; j++) keys[j] = std::move(dk[j]);
+    if (vals) *vals = std::move(dvb);
+  }
   ds.pending = true;
   return SPK_OK;
 }
@@ -918,11 +963,47 @@ __global__ void __launch_bounds__(OC_BLOCK) k_oc_write(const uint64_t* l0, const
   }
 }
 
-// Returns the number of kept items in *m (host value; synchronises st).
+// The conversion of a whole list (no filter).
+struct ListLimbs {
+  const uint64_t* p[4];
+};
+template <int NL>
+__global__ void __launch_bounds__(OC_BLOCK) k_oc_all(ListLimbs L, uint64_t n, unsigned k, uint64_t* __restrict__ out) {
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+    Seq<NL> V;
+#pragma unroll
+    for (int j = 0; j < NL; j++) V.v[j] = __ldcs(L.p[j] + i);
+    uint64_t w[4];
+    kmer256_limbs<NL>(V, k, w);
+#pragma unroll
+    for (int q = 0; q < NL; q++) out[i * NL + q] = w[q];
+  }
+}
+
+// Returns the number of kept items in *m (host value; synchronises st when cin
+// filters and the number is not known).
 int ordered_convert(cudaStream_t st, int nl, uint64_t n, unsigned k, DevBuf* limbs,
                     const uint32_t* cin, uint32_t min_count, DevBuf* out, DevBuf* cout,
                     uint64_t* h_staging, uint64_t* m, uint64_t known_m) {
   int rc;
+  if (!cin) {  // every item is kept: nothing to count
+    *m = n;
+    if ((rc = out->alloc_keep(std::max<uint64_t>(n, 1) * nl * 8, st))) return rc;
+    if (n) {
+      const ListLimbs L{{limbs[0].as<uint64_t>(), nl > 1 ? limbs[1].as<uint64_t>() : nullptr,
+                         nl > 2 ? limbs[2].as<uint64_t>() : nullptr, nl > 3 ? limbs[3].as<uint64_t>() : nullptr}};
+      const unsigned g = (unsigned)std::min<uint64_t>((n + OC_BLOCK - 1) / OC_BLOCK, (uint64_t)current_sm_count() * 16);
+      uint64_t* o = out->as<uint64_t>();
+      switch (nl) {
+        case 1: k_oc_all<1><<<g, OC_BLOCK, 0, st>>>(L, n, k, o); break;
+        case 2: k_oc_all<2><<<g, OC_BLOCK, 0, st>>>(L, n, k, o); break;
+        case 3: k_oc_all<3><<<g, OC_BLOCK, 0, st>>>(L, n, k, o); break;
+        default: k_oc_all<4><<<g, OC_BLOCK, 0, st>>>(L, n, k, o); break;
+      }
+      SPK_CUDA(cudaGetLastError());
+    }
+    return SPK_OK;
+  }
   const uint32_t nt = (uint32_t)std::max<uint64_t>((n + OC_TILE - 1) / OC_TILE, 1);
   DevBuf bc;
   if ((rc = bc.alloc((uint64_t)(nt + 1) * 4, st))) return rc;

@@ -29,7 +29,7 @@ namespace spk {
 
 constexpr uint32_t kSkChunk = 128;    // stream entries a warp reserves at a time
 constexpr int kSkReadBlock = 256;
-constexpr uint32_t kSkBinBlock = 256, kSkBinIpt = 16, kSkBinChunk = kSkBinBlock * kSkBinIpt;
+constexpr uint32_t kSkBinBlock = 256, kSkBinIpt = 4, kSkBinChunk = kSkBinBlock * kSkBinIpt;
 constexpr uint32_t kSkMaxBins = 1u << 22;
 constexpr uint32_t kSkWinBits = 36;   // bins: windows in the low bits, records above
 constexpr uint64_t kSkWinMask = (1ULL << kSkWinBits) - 1;
