@@ -2142,6 +2142,95 @@ __global__ void __launch_bounds__(kBlock) k_admit_singletons(ListOut lo, unsigne
   warp_add_u64(lo.hist + 1, adm);
 }
 
+// Admission of a counted list against tiers of other reads (SPK_F_CORRECT: the
+// tiers of the reads before correction): n k-mers with counts cin (nullptr: one
+// each) are admitted when their three twice bits are set; admitted ones go to the
+// histogram and, counted lmin times or more, to the list o, in tiles of 1,024 with
+// one reservation each.  sums as k_admit_compact's.
+constexpr int kAdmitTile = 4;  // k-mers per thread and reservation
+template <int NL>
+__global__ void __launch_bounds__(kBlock) k_admit_list(ListOut in, int singles, unsigned k, FastMod fm,
+                                                       const uint64_t* __restrict__ twice, uint32_t lmin, ListOut o,
+                                                       unsigned long long* __restrict__ sums) {
+  constexpr int U = kAdmitTile;
+  __shared__ unsigned sh[kHistBins];
+  __shared__ uint32_t wsum[kBlock / 32];
+  __shared__ unsigned long long s_base;
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < kHistBins; i += kBlock) sh[i] = 0;
+  __syncthreads();
+  const uint64_t n = min((uint64_t)in.fill[singles], singles ? in.scap : in.cap);
+  uint64_t n_adm = 0, occ = 0;
+  for (uint64_t tile = blockIdx.x * (uint64_t)(U * kBlock); tile < n; tile += (uint64_t)gridDim.x * (U * kBlock)) {
+    uint32_t c[U];
+    uint64_t tw[U][3];
+    uint32_t sf[U][3];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const uint64_t i = tile + (uint64_t)u * kBlock + threadIdx.x;
+      c[u] = 0;
+      if (i < n) {
+        c[u] = singles ? 1u : in.cnt[i];
+        Seq<NL> C;
+#pragma unroll
+        for (int j = 0; j < NL; j++) C.v[j] = singles ? in.s[j][i] : in.l[j][i];
+        uint64_t raw[3], pos[3];
+        bloom_positions<NL>(C, k, fm, raw, pos);
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+          tw[u][j] = __ldg(twice + (pos[j] >> 6));
+          sf[u][j] = (uint32_t)(pos[j] & 63);
+        }
+      }
+    }
+    uint32_t keep = 0;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      if (!c[u] || !((tw[u][0] >> sf[u][0]) & (tw[u][1] >> sf[u][1]) & (tw[u][2] >> sf[u][2]) & 1)) continue;
+      n_adm++;
+      occ += c[u];
+      atomicAdd(&sh[c[u] < kHistBins - 1 ? c[u] : kHistBins - 1], 1u);
+      keep |= (c[u] >= lmin ? 1u : 0u) << u;
+    }
+    const uint32_t ne = __popc(keep);
+    uint32_t incl = ne;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t v = __shfl_up_sync(FULL, incl, d);
+      if ((int)lane >= d) incl += v;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    uint32_t before = 0, total = 0;
+#pragma unroll
+    for (unsigned w = 0; w < kBlock / 32; w++) {
+      if (w < warp) before += wsum[w];
+      total += wsum[w];
+    }
+    if (threadIdx.x == 0) s_base = total ? atomicAdd(sums + 3, (unsigned long long)total) : 0ULL;
+    __syncthreads();
+    uint64_t p = s_base + before + incl - ne;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      if (!(keep >> u & 1)) continue;
+      const uint64_t i = tile + (uint64_t)u * kBlock + threadIdx.x;
+      if (p < o.cap) {
+#pragma unroll
+        for (int j = 0; j < NL; j++) o.l[j][p] = singles ? in.s[j][i] : in.l[j][i];
+        o.cnt[p] = c[u];
+      }
+      p++;
+    }
+    __syncthreads();  // wsum and s_base are used again
+  }
+  warp_add_u64(sums + 0, n_adm);
+  if (singles) warp_add_u64(sums + 1, n_adm);
+  warp_add_u64(sums + 2, occ);
+  __syncthreads();
+  for (int i = threadIdx.x; i < kHistBins; i += kBlock)
+    if (sh[i]) atomicAdd(o.hist + i, (unsigned long long)sh[i]);
+}
+
 // Solid k-mers of the list (count >= cutoff), for cutoffs the histogram cannot resolve.
 __global__ void __launch_bounds__(256) k_count_solid(const uint32_t* __restrict__ cnt, uint64_t n,
                                                      const uint32_t* __restrict__ thr,
@@ -2548,6 +2637,12 @@ static void launch_admit_singletons(spk_ctx* ctx, cudaStream_t st, const ListOut
   k_admit_singletons<NL><<<grid_for(ctx, 8), kBlock, 0, st>>>(lo, k, fm, twice, sums);
 }
 template <int NL>
+static void launch_admit_list(spk_ctx* ctx, cudaStream_t st, const ListOut& in, int singles, unsigned k,
+                              const FastMod& fm, const uint64_t* twice, uint32_t lmin, const ListOut& o,
+                              unsigned long long* sums) {
+  k_admit_list<NL><<<grid_for(ctx, 4), kBlock, 0, st>>>(in, singles, k, fm, twice, lmin, o, sums);
+}
+template <int NL>
 static void launch_fused(spk_ctx* ctx, cudaStream_t st, const ReadsView& rv, unsigned k,
                          const FastMod& fm, U128* tiers, unsigned long long* ref,
                          const TableView& t, unsigned long long* occ) {
@@ -2849,6 +2944,110 @@ static int keep_results(KResult& kr, cudaStream_t st, uint32_t flags) {
   return SPK_OK;
 }
 
+constexpr int kNotThisPath = -100, kRedo = -101, kGrow = -102;  // of the paths below
+// The super-k-mer records of a read set, by bin, and the batches of bins.
+struct SkJob {
+  DevBuf recs, bstart;
+  uint32_t nbat = 0;
+};
+template <int R>
+static void launch_sk_reads(spk_ctx* ctx, cudaStream_t st, const ReadsView& rv, unsigned k, const SkStream& S,
+                            unsigned long long* occ) {
+  const int grid = grid_for(ctx, 8);
+  const uint64_t warps = (uint64_t)grid * (kSkReadBlock / 32);
+  const uint32_t rpw = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(rv.n_reads / (warps * 4), 1), 32);
+  k_sk_reads<R><<<grid, kSkReadBlock, 0, st>>>(rv, k, sk_m(k), rpw, S, occ);
+}
+// occ: the k-mer windows of the reads; longest: the longest read.
+template <int NL>
+static int sk_partition(spk_ctx* ctx, cudaStream_t st, const ReadsView& rv, unsigned k, uint64_t occ,
+                        uint64_t longest, bool per_chunk, int* errp, unsigned long long* occ_out,
+                        unsigned long long* fill, SkJob& sj, uint32_t* launches) {
+  const uint32_t m = sk_m(k), w = k - m + 1;
+  // m-mer positions a warp holds: the longest read's, if that is at most 256
+  // (else in segments of 256), and at least 32 windows' worth
+  const uint64_t want = std::max<uint64_t>(longest > m ? longest - m + 1 : 1, w + 31);
+  const uint32_t R = want <= 96 ? 3 : want <= 128 ? 4 : want <= 160 ? 5 : want <= 192 ? 6 : 8;
+  const uint32_t seg = 32 * R - w + 1;
+  // A random sequence has 2 / (w + 1) runs per window, every read and segment
+  // one more; a stream that overflows (sequences made of other things) sends
+  // the job to the general path.
+  uint32_t nbins = 4096;
+  while (nbins < kSkMaxBins && (uint64_t)nbins * 512 < occ) nbins *= 2;
+  const uint64_t warps = (uint64_t)grid_for(ctx, 8) * (kSkReadBlock / 32);
+  const uint64_t cap = (uint64_t)((double)occ * (2.8 / (w + 1) + 1.0 / seg)) + rv.n_reads + rv.n_reads / 2 +
+                       (rv.chunks ? rv.chunks->n : 1) * std::min<uint64_t>(warps, rv.n_reads) * kSkChunk + 4096;
+  if (cap >= (1ULL << 32)) return kNotThisPath;
+  // Windows per batch: what fits a table, or fewer so that every CTA has one
+  const uint32_t T = (uint32_t)std::min<uint64_t>(
+      SkShape<NL>::T, std::max<uint64_t>(occ / ((uint64_t)ctx->sm_count * SkShape<NL>::ctas), 1024));
+  sj.nbat = (uint32_t)(occ / T) + 1;
+  int rc;
+  DevBuf stream, bins, sums, base;
+  const uint32_t nchunks = (nbins + kSkBinChunk - 1) / kSkBinChunk;
+  if ((rc = stream.alloc(cap * 16, st)) || (rc = bins.alloc((uint64_t)nbins * 8, st)) ||
+      (rc = sums.alloc((uint64_t)nchunks * 16, st)) || (rc = base.alloc((uint64_t)nbins * 4, st)) ||
+      (rc = sj.bstart.alloc(((uint64_t)sj.nbat + 1) * 4, st)) || (rc = sj.recs.alloc(cap * 8, st)))
+    return rc;
+  SPK_CUDA(cudaMemsetAsync(bins.p, 0, (uint64_t)nbins * 8, st));
+  SkStream S{stream.as<uint4>(), cap, fill, bins.as<unsigned long long>(), nbins, errp};
+  auto reads = [&](const ReadsView& r) {
+    switch (R) {
+      case 3: launch_sk_reads<3>(ctx, st, r, k, S, occ_out); break;
+      case 4: launch_sk_reads<4>(ctx, st, r, k, S, occ_out); break;
+      case 5: launch_sk_reads<5>(ctx, st, r, k, S, occ_out); break;
+      case 6: launch_sk_reads<6>(ctx, st, r, k, S, occ_out); break;
+      default: launch_sk_reads<8>(ctx, st, r, k, S, occ_out); break;
+    }
+    ++*launches;
+  };
+  if (per_chunk) {
+    // the reads of each uploaded piece as soon as it is on the device
+    uint64_t r0 = 0;
+    for (int c = 0; c < rv.chunks->n; c++) {
+      SPK_CUDA(cudaStreamWaitEvent(st, rv.chunks->ready[c], 0));
+      const uint64_t r1 = std::min<uint64_t>(std::max<uint64_t>(rv.chunks->read_end[c], r0), rv.n_reads);
+      if (r1 > r0) {
+        ReadsView p = rv;
+        p.offsets += r0;
+        p.lengths += r0;
+        p.n_reads = r1 - r0;
+        reads(p);
+      }
+      r0 = r1;
+    }
+  } else {
+    if (rv.chunks) SPK_CUDA(cudaStreamWaitEvent(st, rv.chunks->ready[rv.chunks->n - 1], 0));
+    reads(rv);
+  }
+  k_sk_bins_reduce<<<nchunks, kSkBinBlock, 0, st>>>(S.bins, nbins, sums.as<unsigned long long>());
+  k_sk_bins_apply<<<nchunks, kSkBinBlock, 0, st>>>(S.bins, nbins, sums.as<unsigned long long>(), T, sj.nbat,
+                                                  base.as<uint32_t>(), sj.bstart.as<uint32_t>());
+  k_sk_place<<<grid_for(ctx, 8), 256, 0, st>>>(S, base.as<uint32_t>(), sj.recs.as<uint64_t>());
+  SPK_CUDA(cudaGetLastError());
+  *launches += 3;
+  return SPK_OK;
+}
+template <int NL>
+static int sk_count(spk_ctx* ctx, cudaStream_t st, const ReadsView& rv, const SkJob& sj,
+                    unsigned long long* next_batch, unsigned k, const FastMod& fm, const RangeView* bv,
+                    const ListOut& lo, int* errp) {
+  const SkStage g = sk_stage<NL>(k);
+  int rc;
+  if ((rc = raise_smem_limit((const void*)k_sk_count<NL>, g.smem))) return rc;
+  const int grid = (int)std::min<uint64_t>(sj.nbat, (uint64_t)ctx->sm_count * SkShape<NL>::ctas);
+  k_sk_count<NL><<<grid, SkShape<NL>::threads, g.smem, st>>>(rv.words, sj.recs.as<uint64_t>(),
+                                                             sj.bstart.as<uint32_t>(), sj.nbat, next_batch, k, g.rc,
+                                                             g.dd, lo, errp);
+  if (bv) {  // the Bloom operations too
+    const size_t osm = ops_smem(bv->nranges);
+    if ((rc = raise_smem_limit((const void*)k_bloom_ops<NL>, osm))) return rc;
+    k_bloom_ops<NL><<<grid_for(ctx, 3), kOpsBlock, osm, st>>>(lo, k, fm, *bv);
+  }
+  SPK_CUDA(cudaGetLastError());
+  return SPK_OK;
+}
+
 int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& rv_in, unsigned k,
                 const spk_count_opts& o, KResult& kr) {
   kr.k = k;
@@ -2865,9 +3064,11 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
   int rc;
 
   DevBuf scratch;
-  if ((rc = scratch.alloc(S_WORDS * 8, st))) return rc;
+  // the longest read, super-k-mer stream entries, the next batch to count
+  constexpr int S_LONGEST = S_WORDS, S_SKFILL = S_WORDS + 1, S_SKNEXT = S_WORDS + 2, kWords = S_WORDS + 3;
+  if ((rc = scratch.alloc(kWords * 8, st))) return rc;
   uint64_t* sw = scratch.as<uint64_t>();
-  SPK_CUDA(cudaMemsetAsync(sw, 0, S_WORDS * 8, st));
+  SPK_CUDA(cudaMemsetAsync(sw, 0, kWords * 8, st));
   unsigned long long* su = (unsigned long long*)sw;
   int* errp = (int*)(sw + S_ERR);
   ReadsView rv = rv_in;
@@ -2932,6 +3133,20 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
   bool list_mode = false;  // the span count wrote the list (no table)
   ListOut lo{};
   DevBuf sgl[4];           // list mode: keys of the k-mers counted once
+  // Error correction with super-k-mers: the counted k-mers, the windows of the
+  // reads and the longest read.
+  bool sk = false;
+  DevBuf sk_list[4], sk_cnt;
+  uint64_t sk_occ = 0, sk_longest = 0;
+  // Partition and count of rv's super-k-mers into lo (and their Bloom operations).
+  auto sk_both = [&](const RangeView* ranges) -> int {
+    SkJob sj;
+    int r2 = SPK_NL_CALL(nl, sk_partition, ctx, st, rv, k, sk_occ, sk_longest, false, errp, su + S_OCC, su + S_SKFILL,
+                         sj, &launches);
+    if (!r2) r2 = SPK_NL_CALL(nl, sk_count, ctx, st, rv, sj, su + S_SKNEXT, k, kr.fm, ranges, lo, errp);
+    launches += ranges ? 2 : 1;
+    return r2;
+  };
   if (!gated) {
     // ---- fused: Bloom and the count of every k-mer in one pass ----
     k_occ<<<grid_for(ctx, 2), kBlock, 0, st>>>(rv.lengths, rv.n_reads, k, su + S_OCC0, nullptr);
@@ -3160,12 +3375,59 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
     }
   } else {
     // ---- gated: Stage 2 first ----
+    // With error correction (and no use for a table), both stages count super-
+    // k-mers as the default job does, if the k-mers of the reads take at most an
+    // eighth of the memory: the tiers come from the distinct k-mers of the reads,
+    // and the corrected reads' k-mers are admitted against them once counted.
+    // (SPK_F_GATED alone asks for a table of the admitted k-mers only.)
+    if (correct && !ref && !table_wanted && !o.table_log2 && !o.span_groups_log2 && use_ops && sk_fits(k)) {
+      k_occ<<<grid_for(ctx, 2), kBlock, 0, st>>>(rv.lengths, rv.n_reads, k, su + S_OCC0, su + S_LONGEST);
+      SPK_CUDA(cudaGetLastError());
+      launches++;
+      if ((rc = fetch(kWords))) return rc;
+      sk_occ = host[S_OCC0];
+      sk_longest = host[S_LONGEST];
+      cap = list_capacity(sk_occ, nl);
+      if (sk_occ > 0 && cap <= ctx->total_mem / 8 / (16 * nl + 20)) {
+        const uint64_t rcap = 3 * cap / nranges + 1 + 3 * cap / nranges / 4 + 1024;
+        if ((rc = rbase.alloc((nranges + 1) * 8, st)) || (rc = rfill.alloc(nranges * 4 * kFillStride, st)) ||
+            (rc = ops.alloc(nranges * rcap * 4, st)) || (rc = sk_cnt.alloc(cap * 4, st)))
+          return rc;
+        for (int j = 0; j < nl; j++)
+          if ((rc = sk_list[j].alloc(cap * 8, st)) || (rc = sgl[j].alloc(cap * 8, st))) return rc;
+        SPK_CUDA(cudaMemsetAsync(rfill.p, 0, nranges * 4 * kFillStride, st));
+        bv = RangeView{ops.as<uint32_t>(), rbase.as<uint64_t>(), rfill.as<unsigned int>(), rcap, (uint32_t)nranges, errp};
+        for (int j = 0; j < nl; j++) {
+          lo.l[j] = sk_list[j].as<uint64_t>();
+          lo.s[j] = sgl[j].as<uint64_t>();
+        }
+        lo.cnt = sk_cnt.as<uint32_t>();
+        lo.cap = lo.scap = cap;
+        lo.lmin = 2;
+        lo.fill = su + S_LFILL;
+        lo.hist = su + S_HIST;
+        lo.occ2 = su + S_OCC2;
+        SPK_CUDA(cudaEventRecord(kb0.e, st));
+        rc = sk_both(&bv);
+        if (!rc) rc = fetch(kWords);
+        if (rc && rc != kNotThisPath) return rc;
+        sk = !rc && !((int)host[S_ERR] & (int)(1 | kErrRegion | kErrRange)) && host[S_LFILL] <= cap &&
+             host[S_LFILL + 1] <= cap;
+        if (!sk) {  // sequences or coverage this was not sized for: the reference's two passes
+          bv.ops = nullptr;
+          ops.release();
+          SPK_CUDA(cudaMemsetAsync(sw, 0, kWords * 8, st));
+        }
+      }
+    }
+    if (!sk) {
     if ((rc = reset_tiers())) return rc;
     SPK_CUDA(cudaEventRecord(kb0.e, st));
     SPK_DISPATCH_NL(nl, launch_bloom, ctx, st, rv, k, kr.fm, tiers, refp, su + S_OCC);
     SPK_CUDA(cudaGetLastError());
     SPK_CUDA(cudaEventRecord(kb1.e, st));
     launches++;
+    }
   }
   // the compact tiers (every schedule)
   if ((rc = kr.seen.alloc(kr.num_words * 8, st))) return rc;
@@ -3209,7 +3471,36 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
     rv.words = cdata.as<uint64_t>();
     rv.byte_base = 0;
   }
-  if (gated) {
+  if (sk) {
+    // ---- Stage 3: the corrected reads' k-mers, admitted against the tiers ----
+    for (int j = 0; j < nl; j++)
+      if ((rc = kr.list[j].alloc(cap * 8, st))) return rc;
+    if ((rc = kr.list[4].alloc(cap * 4, st))) return rc;
+    SPK_CUDA(cudaMemsetAsync(su + S_SUMS, 0, 4 * 8, st));
+    SPK_CUDA(cudaMemsetAsync(su + S_LFILL, 0, (S_WORDS - S_LFILL) * 8, st));  // fills, occurrences, histogram
+    SPK_CUDA(cudaMemsetAsync(su + S_SKFILL, 0, 2 * 8, st));
+    SPK_CUDA(cudaEventRecord(kc0.e, st));
+    if ((rc = sk_both(nullptr)) && rc != kNotThisPath) return rc;
+    const bool part = !rc;
+    // (the count's own histogram is of all its k-mers: admission starts it again)
+    SPK_CUDA(cudaMemsetAsync(su + S_HIST, 0, kHistBins * 8, st));
+    ListOut out = lo;
+    for (int j = 0; j < nl; j++) out.l[j] = kr.list[j].as<uint64_t>();
+    out.cnt = kr.list[4].as<uint32_t>();
+    if (part)
+      for (int singles = 0; singles < 2; singles++) {
+        SPK_DISPATCH_NL(nl, launch_admit_list, ctx, st, lo, singles, k, kr.fm, kr.twice.as<uint64_t>(), lmin_pre, out,
+                        su + S_SUMS);
+        SPK_CUDA(cudaGetLastError());
+        launches++;
+      }
+    SPK_CUDA(cudaEventRecord(kc1.e, st));
+    if ((rc = fetch(kWords))) return rc;
+    sk = part && !((int)host[S_ERR] & (int)(1 | kErrRegion)) && host[S_LFILL] <= cap && host[S_LFILL + 1] <= cap &&
+         host[S_SUMS + 3] <= cap;
+    if (!sk) SPK_CUDA(cudaMemsetAsync(su + S_SUMS, 0, (S_WORDS - S_SUMS) * 8, st));
+  }
+  if (gated && !sk) {
     // ---- gated: Stage 3 over admitted occurrences ----
     cap = o.table_log2 ? (1ULL << std::min<uint32_t>(o.table_log2, 40))
                        : gated_capacity(size_bits, info.seen_popcount, info.twice_popcount);
@@ -3302,7 +3593,9 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
     if (kr.list_min <= 1) est += std::max(n_all - n2, 0.0) * ft * ft * ft * 1.5 + 65536;
     lcap = std::min<uint64_t>((uint64_t)est, cap);
   }
-  for (int pass = 0; !list_mode; pass++) {
+  if (sk)
+    for (int j = 0; j < nl; j++) lp[j] = kr.list[j].as<uint64_t>();
+  for (int pass = 0; !list_mode && !sk; pass++) {
     for (int j = 0; j < nl; j++) {
       if ((rc = kr.list[j].alloc(std::max<uint64_t>(lcap, 1) * 8, st))) return rc;
       lp[j] = kr.list[j].as<uint64_t>();
@@ -3434,7 +3727,6 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
 // Returns kNotThisPath when the inputs need another layout (count_one_k
 // handles them), kRedo after an overflow, else the status.
 // ---------------------------------------------------------------------------
-constexpr int kNotThisPath = -100, kRedo = -101, kGrow = -102;
 constexpr uint32_t kMaxLog2Groups = 4;  // at most 16 passes over the reads
 
 // A second stream of one job, joined back to the job's stream by events.
@@ -3454,107 +3746,6 @@ struct SideStream {
     pooled_event_put(join, false);
   }
 };
-
-// The super-k-mer records of a read set, by bin, and the batches of bins.
-struct SkJob {
-  DevBuf recs, bstart;
-  uint32_t nbat = 0;
-};
-template <int R>
-static void launch_sk_reads(spk_ctx* ctx, cudaStream_t st, const ReadsView& rv, unsigned k, const SkStream& S,
-                            unsigned long long* occ) {
-  const int grid = grid_for(ctx, 8);
-  const uint64_t warps = (uint64_t)grid * (kSkReadBlock / 32);
-  const uint32_t rpw = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(rv.n_reads / (warps * 4), 1), 32);
-  k_sk_reads<R><<<grid, kSkReadBlock, 0, st>>>(rv, k, sk_m(k), rpw, S, occ);
-}
-// occ: the k-mer windows of the reads; longest: the longest read.
-template <int NL>
-static int sk_partition(spk_ctx* ctx, cudaStream_t st, const ReadsView& rv, unsigned k, uint64_t occ,
-                        uint64_t longest, bool per_chunk, int* errp, unsigned long long* occ_out,
-                        unsigned long long* fill, SkJob& sj, uint32_t* launches) {
-  const uint32_t m = sk_m(k), w = k - m + 1;
-  // m-mer positions a warp holds: the longest read's, if that is at most 256
-  // (else in segments of 256), and at least 32 windows' worth
-  const uint64_t want = std::max<uint64_t>(longest > m ? longest - m + 1 : 1, w + 31);
-  const uint32_t R = want <= 96 ? 3 : want <= 128 ? 4 : want <= 160 ? 5 : want <= 192 ? 6 : 8;
-  const uint32_t seg = 32 * R - w + 1;
-  // A random sequence has 2 / (w + 1) runs per window, every read and segment
-  // one more; a stream that overflows (sequences made of other things) sends
-  // the job to the general path.
-  uint32_t nbins = 4096;
-  while (nbins < kSkMaxBins && (uint64_t)nbins * 512 < occ) nbins *= 2;
-  const uint64_t warps = (uint64_t)grid_for(ctx, 8) * (kSkReadBlock / 32);
-  const uint64_t cap = (uint64_t)((double)occ * (2.8 / (w + 1) + 1.0 / seg)) + rv.n_reads + rv.n_reads / 2 +
-                       (rv.chunks ? rv.chunks->n : 1) * std::min<uint64_t>(warps, rv.n_reads) * kSkChunk + 4096;
-  if (cap >= (1ULL << 32)) return kNotThisPath;
-  // Windows per batch: what fits a table, or fewer so that every CTA has one
-  const uint32_t T = (uint32_t)std::min<uint64_t>(
-      SkShape<NL>::T, std::max<uint64_t>(occ / ((uint64_t)ctx->sm_count * SkShape<NL>::ctas), 1024));
-  sj.nbat = (uint32_t)(occ / T) + 1;
-  int rc;
-  DevBuf stream, bins, sums, base;
-  const uint32_t nchunks = (nbins + kSkBinChunk - 1) / kSkBinChunk;
-  if ((rc = stream.alloc(cap * 16, st)) || (rc = bins.alloc((uint64_t)nbins * 8, st)) ||
-      (rc = sums.alloc((uint64_t)nchunks * 16, st)) || (rc = base.alloc((uint64_t)nbins * 4, st)) ||
-      (rc = sj.bstart.alloc(((uint64_t)sj.nbat + 1) * 4, st)) || (rc = sj.recs.alloc(cap * 8, st)))
-    return rc;
-  SPK_CUDA(cudaMemsetAsync(bins.p, 0, (uint64_t)nbins * 8, st));
-  SkStream S{stream.as<uint4>(), cap, fill, bins.as<unsigned long long>(), nbins, errp};
-  auto reads = [&](const ReadsView& r) {
-    switch (R) {
-      case 3: launch_sk_reads<3>(ctx, st, r, k, S, occ_out); break;
-      case 4: launch_sk_reads<4>(ctx, st, r, k, S, occ_out); break;
-      case 5: launch_sk_reads<5>(ctx, st, r, k, S, occ_out); break;
-      case 6: launch_sk_reads<6>(ctx, st, r, k, S, occ_out); break;
-      default: launch_sk_reads<8>(ctx, st, r, k, S, occ_out); break;
-    }
-    ++*launches;
-  };
-  if (per_chunk) {
-    // the reads of each uploaded piece as soon as it is on the device
-    uint64_t r0 = 0;
-    for (int c = 0; c < rv.chunks->n; c++) {
-      SPK_CUDA(cudaStreamWaitEvent(st, rv.chunks->ready[c], 0));
-      const uint64_t r1 = std::min<uint64_t>(std::max<uint64_t>(rv.chunks->read_end[c], r0), rv.n_reads);
-      if (r1 > r0) {
-        ReadsView p = rv;
-        p.offsets += r0;
-        p.lengths += r0;
-        p.n_reads = r1 - r0;
-        reads(p);
-      }
-      r0 = r1;
-    }
-  } else {
-    if (rv.chunks) SPK_CUDA(cudaStreamWaitEvent(st, rv.chunks->ready[rv.chunks->n - 1], 0));
-    reads(rv);
-  }
-  k_sk_bins_reduce<<<nchunks, kSkBinBlock, 0, st>>>(S.bins, nbins, sums.as<unsigned long long>());
-  k_sk_bins_apply<<<nchunks, kSkBinBlock, 0, st>>>(S.bins, nbins, sums.as<unsigned long long>(), T, sj.nbat,
-                                                  base.as<uint32_t>(), sj.bstart.as<uint32_t>());
-  k_sk_place<<<grid_for(ctx, 8), 256, 0, st>>>(S, base.as<uint32_t>(), sj.recs.as<uint64_t>());
-  SPK_CUDA(cudaGetLastError());
-  *launches += 3;
-  return SPK_OK;
-}
-template <int NL>
-static int sk_count(spk_ctx* ctx, cudaStream_t st, const ReadsView& rv, const SkJob& sj,
-                    unsigned long long* next_batch, unsigned k, const FastMod& fm, const RangeView& bv,
-                    const ListOut& lo, int* errp) {
-  const SkStage g = sk_stage<NL>(k);
-  int rc;
-  if ((rc = raise_smem_limit((const void*)k_sk_count<NL>, g.smem))) return rc;
-  const int grid = (int)std::min<uint64_t>(sj.nbat, (uint64_t)ctx->sm_count * SkShape<NL>::ctas);
-  k_sk_count<NL><<<grid, SkShape<NL>::threads, g.smem, st>>>(rv.words, sj.recs.as<uint64_t>(),
-                                                             sj.bstart.as<uint32_t>(), sj.nbat, next_batch, k, g.rc,
-                                                             g.dd, lo, errp);
-  const size_t osm = ops_smem(bv.nranges);
-  if ((rc = raise_smem_limit((const void*)k_bloom_ops<NL>, osm))) return rc;
-  k_bloom_ops<NL><<<grid_for(ctx, 3), kOpsBlock, osm, st>>>(lo, k, fm, bv);
-  SPK_CUDA(cudaGetLastError());
-  return SPK_OK;
-}
 
 // *slots (0: sized here) is the room for distinct k-mers; after kGrow it holds
 // what the super-k-mers' count found, or 0 when the table's spans ran out.
@@ -3695,7 +3886,7 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
     info.span_groups = 1;
     if ((rc = alloc_count_buffers())) return rc;
     SPK_CUDA(cudaEventRecord(kc0.e, st));
-    rc = SPK_NL_CALL(nl, sk_count, ctx, st, rv, sj, su + S_SKNEXT, k, kr.fm, bv, lo, errp);
+    rc = SPK_NL_CALL(nl, sk_count, ctx, st, rv, sj, su + S_SKNEXT, k, kr.fm, &bv, lo, errp);
     if (rc) return rc;
     launches += 2;
   }

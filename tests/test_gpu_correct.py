@@ -116,3 +116,38 @@ def test_count_with_correction(spk, ora, k, genome):
     plain = spk.count(p, [k], bloom_bits=bits, list_min_count=1, flags=0x1 | 0x4 | 0x8)
     assert info["n_table"] < plain.info(0)["n_table"]
     np.testing.assert_array_equal(r.bloom(0)[0], ref.bloom()[0])
+
+
+@pytest.mark.parametrize("k,kind", [(21, "sample"), (32, "sample"), (47, "sample"), (95, "sample"), (55, "distinct")])
+@pytest.mark.parametrize("list_min,min_count", [(1, 0), (2, 4), (6, 5)])
+def test_correcting_count_thresholds(spk, ora, k, kind, list_min, min_count):
+    """The correcting count's admission of its counted list (k-mers below the
+    list's threshold still count), at the edges of the key widths; and reads of
+    mostly distinct k-mers, which fall back to the reference's two passes."""
+    from spk import synth
+    if kind == "sample":
+        p = synth.sample(4_000, 40.0, seed=k, err=(0.004, 0.008), ks=(k,)).packed
+    else:
+        rng = np.random.default_rng(k)
+        p = spk.PackedReads.from_clean_reads(["".join(rng.choice(list("ACGT"), 200)) for _ in range(600)])
+    bits = 1 << 22
+    ref = ora.count(p.data, p.offsets, p.lengths, k, bits, mode=ora.MODE_TWICE, correct=True)
+    tk, tc = ref.table(1)
+    r = spk.count(p, [k], bloom_bits=bits, list_min_count=list_min, min_count=min_count,
+                  flags=spk.SPK_F_EDGES | spk.SPK_F_KEEP_BLOOM | spk.SPK_F_CORRECT)
+    info = r.info(0)
+    cut = min_count or ora.cutoff(tc, 5.0)
+    thr = min(list_min, cut)
+    assert info["cutoff"] == cut and info["n_table"] == tk.shape[0]
+    assert info["n_singletons"] == int((tc == 1).sum())
+    assert info["admitted_occurrences"] == int(tc.astype(np.int64).sum())
+    gk, gc = r.kmers(0, 1)
+    np.testing.assert_array_equal(gk, tk[tc >= thr])
+    np.testing.assert_array_equal(gc, tc[tc >= thr])
+    seen, twice = r.bloom(0)
+    oseen, otwice = ref.bloom()
+    np.testing.assert_array_equal(seen, oseen)
+    np.testing.assert_array_equal(twice, otwice)
+    assert info["n_corrected_reads"] == ref.stats()["corrected_reads"]
+    sk, _ = r.solid(0)
+    np.testing.assert_array_equal(r.edges(0), ora.edges(sk, k))
