@@ -994,16 +994,29 @@ def main():
             # reads every key back and writes it to its span
             cands += [("k_part_coarse", coarse_ms, occ * (sb + 16)),
                       ("k_part_fine", scatter_ms - coarse_ms, occ * 32)]
+        elif info.get("part_passes") == 2:
+            # super-k-mers: the read stream in; a record of 16 bytes per run of
+            # windows out and in again, 8 bytes to its bin (a random sequence
+            # has 2 / (k - 13) runs per window with minimizers of 15 bases)
+            runs = occ * 2.0 / (K - 13) + len(p.lengths)
+            sname = "k_sk_reads+k_sk_place"
+            cands += [(sname, scatter_ms, occ * sb + runs * (16 + 16 + 8))]
         else:
             # read stream and one streamed key write per occurrence (the
             # algorithm's need; the two-level form moves the keys twice more)
             cands += [(sname, scatter_ms, occ * (sb + 16))]
-        cands += [
+        if coarse_ms > 0 or info.get("part_passes") != 2:
             # keys read back; out: the k-mers counted twice or more as list
             # entries (key + count), the singleton keys, and three 4-byte Bloom
             # operations per distinct k-mer (the table itself is not written)
-            ("k_part_count", count_ms,
-             occ * 16 + n_ge2 * 20 + (info["n_distinct"] - n_ge2) * 16 + ops * 4),
+            cands += [("k_part_count", count_ms,
+                       occ * 16 + n_ge2 * 20 + (info["n_distinct"] - n_ge2) * 16 + ops * 4)]
+        else:
+            # records and their bases in (two sectors a run); list entries and
+            # singleton keys out and in again, three operations per k-mer out
+            cands += [("k_sk_count+k_bloom_ops", count_ms,
+                       runs * (8 + 64) + 2 * (n_ge2 * 20 + (info["n_distinct"] - n_ge2) * 16) + ops * 4)]
+        cands += [
             # Bloom ops read, both tiers written
             ("k_bloom_apply", bloom_ms, ops * 4 + 2 * info["bloom_size_bits"] / 8),
         ]

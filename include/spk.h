@@ -220,9 +220,10 @@ int spk_packed_free(spk_packed* p);
                                         global atomics (SPK_F_DIRECT; k = 96; k > 64 on read sets
                                         too small for two partition levels); the Bloom tiers are
                                         derived from the table afterwards */
-#define SPK_SCHEDULE_PARTITIONED 3u  /* the default: the read pass scatters keys by table span,
-                                        each span is counted in shared memory and written once,
-                                        with the Bloom tiers derived from its counts */
+#define SPK_SCHEDULE_PARTITIONED 3u  /* the default: the reads' super-k-mers go to minimizer bins
+                                        (or, with a table or groups of the caller's size, their
+                                        keys to table spans), which are counted in shared memory,
+                                        with the Bloom tiers derived from the counts */
 
 typedef struct spk_count_opts {
   uint64_t bloom_bits;    /* bits per tier; 0 = 512 Mi (src/assemble.rs:84) */
@@ -308,12 +309,13 @@ typedef struct spk_result_info {
   uint64_t n_corrected_reads;    /* SPK_F_CORRECT: reads with a corrected base */
   float ms_correct;              /* SPK_F_CORRECT: device time of the correction */
   uint32_t part_passes;          /* partitioned: 1 = the keys went to their spans in one pass,
-                                    2 = through coarse buckets first (ms_scatter_kernel covers
-                                    both passes) */
+                                    2 = through an intermediate form first: super-k-mer records
+                                    or coarse buckets (ms_scatter_kernel covers both passes) */
   uint32_t span_groups;          /* partitioned: passes over the reads, each partitioning and
                                     counting one group of spans (read sets too large for one) */
-  float ms_coarse_kernel;        /* two-level partition in one group: the coarse pass alone
-                                    (ms_scatter_kernel - ms_coarse_kernel is the fine pass) */
+  float ms_coarse_kernel;        /* coarse buckets in one group: the coarse pass alone
+                                    (ms_scatter_kernel - ms_coarse_kernel is the fine pass);
+                                    0 for super-k-mers */
   uint32_t solid_copied;         /* 1: the solid list went to spk_count_opts.solid_*_out */
   uint32_t reserved2;
 } spk_result_info;

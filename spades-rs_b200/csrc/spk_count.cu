@@ -16,10 +16,11 @@
 // (SPK_F_REF_SOLID).
 //
 // Three schedules compute that same admitted table:
-//   count-first  (default) one pass over the reads counts every canonical
-//                k-mer occurrence in a table that holds every distinct
-//                k-mer, with one hash and one table update per occurrence.
-//                The Bloom tiers are then derived from the table (a k-mer
+//   count-first  (default) every canonical k-mer of the reads is counted once,
+//                in shared memory, by minimizer bins (spk_superk.cuh) or, where
+//                the caller sizes or keeps the table, by its spans; or in the
+//                table itself with one update per occurrence.
+//                The Bloom tiers are then derived from the counts (a k-mer
 //                counted c times makes c insert operations on each of its
 //                three bits; the tiers do not depend on their order), and
 //                each k-mer seen once is kept only if its three twice bits
@@ -3821,7 +3822,8 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   // the list gets half the slots: k-mers counted twice or more are a small
   // share of the distinct ones (the mid-job readback sends the job back if
   // it overflowed).
-  const uint64_t lcap_ = lg ? cap >> 1 : cap, scap_ = cap;
+  // Super-k-mers too: their count starts again with more room if the list did not fit.
+  const uint64_t lcap_ = lg || superk ? cap >> 1 : cap, scap_ = cap;
   kr.k = k;
   kr.nl = nl;
   kr.num_words = num_words;
@@ -4006,7 +4008,7 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   if (superk && !(err & (int)kErrRegion) && (host[S_LFILL] > lcap_ || host[S_LFILL + 1] > scap_)) {
     // more distinct k-mers than the buffers were sized for (reads of low
     // coverage or many errors): again with room for them
-    *slots = next_pow2(host[S_LFILL] + host[S_LFILL + 1]);
+    *slots = next_pow2(std::max(2 * host[S_LFILL], host[S_LFILL] + host[S_LFILL + 1]));
     return kGrow;
   }
   if (err & (kErrRegion | kErrRange)) return kRedo;  // an overflowed region

@@ -129,7 +129,7 @@ def test_correcting_count_thresholds(spk, ora, k, kind, list_min, min_count):
         p = synth.sample(4_000, 40.0, seed=k, err=(0.004, 0.008), ks=(k,)).packed
     else:
         rng = np.random.default_rng(k)
-        p = spk.PackedReads.from_clean_reads(["".join(rng.choice(list("ACGT"), 200)) for _ in range(600)])
+        p = spk.PackedReads.from_clean_reads(["".join(rng.choice(list("ACGT"), 200)) for _ in range(80)])
     bits = 1 << 22
     ref = ora.count(p.data, p.offsets, p.lengths, k, bits, mode=ora.MODE_TWICE, correct=True)
     tk, tc = ref.table(1)
