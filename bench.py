@@ -1067,8 +1067,7 @@ def main():
     roofline = {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": peak,
                 "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
                 # the captured DRAM bytes of the kernel over its live time: what
-                # it really moves (the two-level partition moves every key three
-                # times against the algorithm's once)
+                # it really moves (null for kernels not captured)
                 "traffic_achieved": (traffic / (kms / 1e3) / 1e9) if traffic else None,
                 "traffic_frac": (traffic / (kms / 1e3) / 1e9 / peak) if traffic else None,
                 "peak_source": peak_src, "algorithmic_bytes_per_launch": kbytes,
