@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
   uint32_t* seq = (uint32_t*)uni;        // word i (16 bases, the first on top) of record t: seq[i * RC + t]
   uint32_t* mult = seq + (size_t)SW * RC;
   uint32_t* dd = mult + RC;
-  uint32_t* lrec = dd;                   // live records: first window << 16 | record (over the records' table)
+  uint32_t* lrec = dd;                   // live records: first window << 11 | record (over the records' table)
   uint8_t* nws = (uint8_t*)(dd + DD);
   __shared__ uint32_t lw[2][kRounds * kWarps];
   __shared__ uint32_t wsum[kWarps];
