@@ -25,14 +25,15 @@
 // distinct k-mers than slots is counted in parts (by hash bits), alone.
 #pragma once
 
+#include "spk_bins.h"
+
 namespace spk {
 
 constexpr uint32_t kSkChunk = 128;    // stream entries a warp reserves at a time
 constexpr int kSkReadBlock = 256;
 constexpr uint32_t kSkBinBlock = 256, kSkBinIpt = 4, kSkBinChunk = kSkBinBlock * kSkBinIpt;
 constexpr uint32_t kSkMaxBins = 1u << 22;
-constexpr uint32_t kSkWinBits = 36;   // bins: windows in the low bits, records above
-constexpr uint64_t kSkWinMask = (1ULL << kSkWinBits) - 1;
+typedef BinWord<36> SkBin;            // 2^36 windows; 2^28 records, of which half are used
 
 // Length of the minimizers: 15 above 32 bases; 13 and 11 below, where a longer
 // one leaves fewer windows per super-k-mer.
@@ -45,7 +46,7 @@ struct SkStream {
   uint4* rec;                 // x, y: record; z: bin; w: rank in the bin
   uint64_t cap;
   unsigned long long* fill;   // entries reserved (a record of no windows is a gap)
-  unsigned long long* bins;   // per bin: records << kSkWinBits | windows
+  unsigned long long* bins;   // per bin: its records and windows (SkBin)
   uint32_t nbins;
   int* err;
 };
@@ -217,7 +218,7 @@ __global__ void __launch_bounds__(kSkReadBlock) k_sk_reads(ReadsView rd, unsigne
           do {
             const uint32_t c = min(left, w);
             uint32_t rank = 0;
-            if (c) rank = (uint32_t)(atomicAdd(S.bins + bin, (1ULL << kSkWinBits) | c) >> kSkWinBits);
+            if (c) rank = SkBin::rank(atomicAdd(S.bins + bin, (unsigned long long)SkBin::record(c)));
             const uint64_t at = place(c > 0);
             if (c) put(at, base + at0, c, bin, rank);
             at0 += c;
@@ -243,8 +244,8 @@ __global__ void __launch_bounds__(kSkBinBlock) k_sk_bins_reduce(const unsigned l
   for (uint32_t j = 0; j < kSkBinIpt; j++) {
     const uint32_t i = blockIdx.x * kSkBinChunk + j * kSkBinBlock + threadIdx.x;
     const uint64_t v = i < n ? bins[i] : 0;
-    r += v >> kSkWinBits;
-    w += v & kSkWinMask;
+    r += SkBin::records(v);
+    w += SkBin::windows(v);
   }
   warp_add_u64(&sr, r);
   warp_add_u64(&sw, w);
@@ -282,8 +283,8 @@ __global__ void __launch_bounds__(kSkBinBlock) k_sk_bins_apply(const unsigned lo
 #pragma unroll
   for (uint32_t j = 0; j < kSkBinIpt; j++) {
     v[j] = i0 + j < n ? bins[i0 + j] : 0;
-    r += v[j] >> kSkWinBits;
-    w += v[j] & kSkWinMask;
+    r += SkBin::records(v[j]);
+    w += SkBin::windows(v[j]);
   }
   uint64_t xr = r, xw = w;
 #pragma unroll
@@ -304,7 +305,7 @@ __global__ void __launch_bounds__(kSkBinBlock) k_sk_bins_apply(const unsigned lo
     pr += wr[q];
     pw += ww[q];
   }
-  uint64_t prevw = (i0 > 0 && i0 <= n) ? bins[i0 - 1] & kSkWinMask : 0;
+  uint64_t prevw = (i0 > 0 && i0 <= n) ? SkBin::windows(bins[i0 - 1]) : 0;
 #pragma unroll
   for (uint32_t j = 0; j < kSkBinIpt; j++) {
     const uint32_t i = i0 + j;
@@ -313,15 +314,17 @@ __global__ void __launch_bounds__(kSkBinBlock) k_sk_bins_apply(const unsigned lo
     const uint32_t b1 = (uint32_t)(pw / T);
     const uint32_t b0 = i ? (uint32_t)((pw - prevw) / T) + 1 : 0;
     for (uint32_t b = b0; b <= b1 && b <= nbat; b++) bstart[b] = (uint32_t)pr;
-    prevw = v[j] & kSkWinMask;
-    pr += v[j] >> kSkWinBits;
+    prevw = SkBin::windows(v[j]);
+    pr += SkBin::records(v[j]);
     pw += prevw;
     if (i == n - 1)
       for (uint32_t b = b1 + 1; b <= nbat; b++) bstart[b] = (uint32_t)pr;
   }
 }
 
-// The stream's records to their bins.
+// The stream's records to their bins.  A bin of more records than its word counts
+// (2^27 short reads of one sequence) sends the job to the general path, as a stream
+// that overflowed does.
 __global__ void __launch_bounds__(256) k_sk_place(SkStream S, const uint32_t* __restrict__ base,
                                                    uint64_t* __restrict__ out) {
   const uint64_t n = min((uint64_t)*S.fill, S.cap);
@@ -330,6 +333,7 @@ __global__ void __launch_bounds__(256) k_sk_place(SkStream S, const uint32_t* __
     const uint4 q = __ldcs(S.rec + i);
     const uint64_t r = (uint64_t)q.y << 32 | q.x;
     const uint64_t at = (r & 255) ? (uint64_t)__ldg(base + q.z) + q.w : S.cap;
+    if (SkBin::too_many(q.w)) atomicOr(S.err, (int)kErrRegion);
     if (at < S.cap) out[at] = r;  // (beyond it only after the stream overflowed: the job runs again)
   }
 }
