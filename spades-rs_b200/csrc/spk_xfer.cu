@@ -170,9 +170,17 @@ static bool is_pageable(const void* p) {
   return a.type == cudaMemoryTypeUnregistered;
 }
 
+// The workers' copies of a chunked transfer, or nullptr for one copy by the caller.
+// cudaStreamPerThread names another stream in every thread that uses it, so a
+// worker's copies would not be in the caller's order: the caller makes those.
+static XferPool* chunked(spk_ctx* ctx, const void* host, size_t n, cudaStream_t st) {
+  if (n < kXferDirect || st == cudaStreamPerThread || !is_pageable(host)) return nullptr;
+  return xfer_pool(ctx);
+}
+
 int xfer_h2d(spk_ctx* ctx, void* dst, const void* src, size_t n, cudaStream_t st) {
   if (n == 0) return SPK_OK;
-  XferPool* pool = n >= kXferDirect && is_pageable(src) ? xfer_pool(ctx) : nullptr;
+  XferPool* pool = chunked(ctx, src, n, st);
   if (!pool) {
     SPK_CUDA(cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, st));
     return SPK_OK;
@@ -197,7 +205,7 @@ int xfer_h2d(spk_ctx* ctx, void* dst, const void* src, size_t n, cudaStream_t st
 
 int xfer_d2h(spk_ctx* ctx, void* dst, const void* src, size_t n, cudaStream_t st) {
   if (n == 0) return SPK_OK;
-  XferPool* pool = n >= kXferDirect && is_pageable(dst) ? xfer_pool(ctx) : nullptr;
+  XferPool* pool = chunked(ctx, dst, n, st);
   if (!pool) {
     SPK_CUDA(cudaMemcpyAsync(dst, src, n, cudaMemcpyDeviceToHost, st));
     SPK_CUDA(cudaStreamSynchronize(st));

@@ -52,3 +52,34 @@ def test_pageable_and_pinned_uploads_agree(spk):
         np.testing.assert_array_equal(gc, ca)
     a.close()
     b.close()
+
+
+def test_per_thread_stream_keeps_its_order(spk):
+    """A context on cudaStreamPerThread (handle 2): copies of pageable memory
+    above the chunked size still follow, and are followed by, the kernels of the
+    calling thread's stream, which a sleeping kernel holds up for some ms."""
+    import torch
+    rng = np.random.default_rng(8)
+    keys = rng.integers(0, 1 << 62, size=9 << 20, dtype=np.uint64)  # 72 MiB of keys, 9 MiB of flags
+    keys[1::2] = keys[::2]  # each key twice: the second insert promotes it
+    bits = 1 << 27          # 16 MiB per tier
+    want = spk.TwoTierFilter(bits, ctx=spk.Context(0))
+    promoted, tiers, solid = want.insert_batch(keys), want.download(), want.is_solid_batch(keys)
+    ctx = spk.Context(0)
+    ctx.set_stream(2)
+    per_thread = torch.cuda.ExternalStream(2)
+
+    def busy():
+        with torch.cuda.stream(per_thread):
+            torch.cuda._sleep(40_000_000)
+
+    f = spk.TwoTierFilter(bits, ctx=ctx)
+    busy()
+    np.testing.assert_array_equal(f.insert_batch(keys), promoted)
+    busy()
+    for a, b in zip(f.download(), tiers):
+        np.testing.assert_array_equal(a, b)
+    busy()
+    np.testing.assert_array_equal(f.is_solid_batch(keys), solid)
+    f.close()
+    want.close()
