@@ -532,13 +532,19 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
   const SkCut<NL> cut = sk_cut<NL>(k);
   constexpr uint64_t kFree = REF ? 0ULL : kEmpty;  // an empty slot
   uint64_t occ2 = 0;
-  if (*(volatile int*)err & (int)kErrRegion) return;  // the stream overflowed: records are missing
   for (int i = threadIdx.x; i < kHistBins; i += TH) s_hist[i] = 0;
   for (uint32_t i = threadIdx.x; i < S * KW; i += TH) keys[i] = kFree;
   for (uint32_t i = threadIdx.x; i < S; i += TH) cnt[i] = 0;
   for (;;) {
     __syncthreads();
-    if (threadIdx.x == 0) s_batch = (uint32_t)min((unsigned long long)nbat, atomicAdd(next_batch, 1ULL));
+    // No more batches once records are missing (the stream overflowed) or a batch
+    // is too large: the job runs again another way.  Another CTA may raise the
+    // flag at any time, so one thread reads it for all.
+    if (threadIdx.x == 0) {
+      const int e = *(volatile int*)err;
+      const unsigned long long b = atomicAdd(next_batch, 1ULL);
+      s_batch = (e & (int)kErrRegion) ? nbat : (uint32_t)min((unsigned long long)nbat, b);
+    }
     __syncthreads();
     const uint32_t bt = s_batch;
     if (bt >= nbat) break;
