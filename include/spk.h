@@ -297,7 +297,8 @@ typedef struct spk_result_info {
                                     schedule, whose one kernel is ms_bloom_kernel; the span
                                     count for the partitioned schedule) */
   uint32_t schedule;             /* SPK_SCHEDULE_* */
-  uint32_t part_rescatters;      /* partitioned: read passes repeated with exact region sizes */
+  uint32_t part_rescatters;      /* partitioned: read passes repeated with exact region sizes, or by
+                                    table spans after the super-k-mers were given up */
   uint64_t n_distinct;           /* distinct k-mers in the table before singleton admission
                                     (n_table plus the rejected singletons) */
   float ms_scatter_kernel;       /* partitioned: the read pass that scatters keys by span */

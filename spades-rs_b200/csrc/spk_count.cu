@@ -1018,6 +1018,8 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* m, uint32_t parity) {
 // chunk takes microseconds; this is tens of milliseconds).
 constexpr uint32_t kStageSpinLimit = 1u << 20;
 constexpr uint32_t kErrStage = 32;  // a staged copy never completed (the job fails)
+constexpr uint32_t kErrHot = 64;    // a minimizer bin too large for one CTA
+constexpr uint32_t kErrRepeat = 128;  // ... and a k-mer in it that would overflow its span
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* m, uint32_t parity) {
   for (uint32_t i = 0; i < kStageSpinLimit; i++)
     if (mbar_try_wait(m, parity)) return true;
@@ -2945,7 +2947,16 @@ static int keep_results(KResult& kr, cudaStream_t st, uint32_t flags) {
   return SPK_OK;
 }
 
-constexpr int kNotThisPath = -100, kRedo = -101, kGrow = -102;  // of the paths below
+// What the region of a span holds of a read set, and how much of that is beyond
+// its mean share: 1.5x the mean, 2x for the smaller spans of keys wider than 64
+// bits (fewer k-mers per span, so its share varies more).
+static uint64_t span_region(uint64_t per, int nl) { return nl >= 3 ? 2 * per + 512 : per + (per >> 1) + 256; }
+static uint64_t span_slack(uint64_t occ, int nl) {
+  const uint64_t per = occ / std::max<uint64_t>(list_capacity(occ, nl) >> part_log2span(nl), 1);
+  return span_region(per, nl) - per;
+}
+
+constexpr int kNotThisPath = -100, kRedo = -101, kGrow = -102, kSpans = -103;  // of the paths below
 // The super-k-mer records of a read set, by bin, and the batches of bins.
 struct SkJob {
   DevBuf recs, bstart;
@@ -3031,7 +3042,7 @@ static int sk_partition(spk_ctx* ctx, cudaStream_t st, const ReadsView& rv, unsi
 }
 template <int NL>
 static int sk_count(spk_ctx* ctx, cudaStream_t st, const ReadsView& rv, const SkJob& sj,
-                    unsigned long long* next_batch, unsigned k, const FastMod& fm, const RangeView* bv,
+                    unsigned long long* next_batch, unsigned k, uint64_t occ, const FastMod& fm, const RangeView* bv,
                     const ListOut& lo, int* errp) {
   const SkStage g = sk_stage<NL>(k);
   int rc;
@@ -3039,7 +3050,7 @@ static int sk_count(spk_ctx* ctx, cudaStream_t st, const ReadsView& rv, const Sk
   const int grid = (int)std::min<uint64_t>(sj.nbat, (uint64_t)ctx->sm_count * SkShape<NL>::ctas);
   k_sk_count<NL><<<grid, SkShape<NL>::threads, g.smem, st>>>(rv.words, sj.recs.as<uint64_t>(),
                                                              sj.bstart.as<uint32_t>(), sj.nbat, next_batch, k, g.rc,
-                                                             g.dd, lo, errp);
+                                                             g.dd, sk_limits(occ, span_slack(occ, NL)), lo, errp);
   if (bv) {  // the Bloom operations too
     const size_t osm = ops_smem(bv->nranges);
     if ((rc = raise_smem_limit((const void*)k_bloom_ops<NL>, osm))) return rc;
@@ -3144,7 +3155,7 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
     SkJob sj;
     int r2 = SPK_NL_CALL(nl, sk_partition, ctx, st, rv, k, sk_occ, sk_longest, false, errp, su + S_OCC, su + S_SKFILL,
                          sj, &launches);
-    if (!r2) r2 = SPK_NL_CALL(nl, sk_count, ctx, st, rv, sj, su + S_SKNEXT, k, kr.fm, ranges, lo, errp);
+    if (!r2) r2 = SPK_NL_CALL(nl, sk_count, ctx, st, rv, sj, su + S_SKNEXT, k, sk_occ, kr.fm, ranges, lo, errp);
     launches += ranges ? 2 : 1;
     return r2;
   };
@@ -3412,7 +3423,7 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
         rc = sk_both(&bv);
         if (!rc) rc = fetch(kWords);
         if (rc && rc != kNotThisPath) return rc;
-        sk = !rc && !((int)host[S_ERR] & (int)(1 | kErrRegion | kErrRange)) && host[S_LFILL] <= cap &&
+        sk = !rc && !((int)host[S_ERR] & (int)(kErrHot | kErrRegion | kErrRange)) && host[S_LFILL] <= cap &&
              host[S_LFILL + 1] <= cap;
         if (!sk) {  // sequences or coverage this was not sized for: the reference's two passes
           bv.ops = nullptr;
@@ -3497,7 +3508,7 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
       }
     SPK_CUDA(cudaEventRecord(kc1.e, st));
     if ((rc = fetch(kWords))) return rc;
-    sk = part && !((int)host[S_ERR] & (int)(1 | kErrRegion)) && host[S_LFILL] <= cap && host[S_LFILL + 1] <= cap &&
+    sk = part && !((int)host[S_ERR] & (int)(kErrHot | kErrRegion)) && host[S_LFILL] <= cap && host[S_LFILL + 1] <= cap &&
          host[S_SUMS + 3] <= cap;
     if (!sk) SPK_CUDA(cudaMemsetAsync(su + S_SUMS, 0, (S_WORDS - S_SUMS) * 8, st));
   }
@@ -3750,8 +3761,9 @@ struct SideStream {
 
 // *slots (0: sized here) is the room for distinct k-mers; after kGrow it holds
 // what the super-k-mers' count found, or 0 when the table's spans ran out.
+// spans: no super-k-mers (after they returned kSpans).
 int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& rv_in, unsigned k,
-                     const spk_count_opts& o, uint64_t* slots, KResult& kr) {
+                     const spk_count_opts& o, bool spans, uint64_t* slots, KResult& kr) {
   const int nl = (int)((k + 31) / 32);
   // (k = 96 fills its top limb, which the solid set's empty mark needs free)
   if (k < 12 || (nl >= 3 && 2 * k == 64u * nl)) return kNotThisPath;
@@ -3795,7 +3807,7 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   // Super-k-mers unless the caller sizes the table or the groups of spans: read
   // sets of any size for k <= 63, and for wider keys those with spans enough for
   // two partition levels (smaller ones count with global atomics).
-  bool superk = sk_fits(k) && !o.table_log2 && !o.span_groups_log2 && occ0 > 0 &&
+  bool superk = !spans && sk_fits(k) && !o.table_log2 && !o.span_groups_log2 && occ0 > 0 &&
                 (nl <= 2 || log2cap > log2span + kCoarseBits);
   if (!superk && log2cap <= log2span) return kNotThisPath;
   const uint32_t log2parts = log2cap > log2span ? log2cap - log2span : 0;
@@ -3803,9 +3815,7 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   // buckets, 2.6 keys per occurrence) would pass a quarter of the device is
   // partitioned and counted in 2^lg passes, each keeping the keys of one group
   // of spans (the reads are streamed once per pass).
-  // Span regions hold 1.5x their mean share of occurrences, 2x for the
-  // smaller spans of keys wider than 64 bits (fewer k-mers per span, so its
-  // share varies more); the coarse buckets 1.125x.
+  // (The coarse buckets hold 1.125x their mean share.)
   const uint64_t part_keys4 = nl >= 3 ? 13 : 11;  // regions + buckets, in quarter keys per occurrence
   auto part_bytes = [&](uint32_t g) { return ((occ0 >> g) * part_keys4 / 4 + (1u << 22)) * (uint64_t)nl * 8; };
   uint32_t lg = std::min<uint32_t>(o.span_groups_log2, kMaxLog2Groups);
@@ -3882,13 +3892,14 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
     SkJob sj;
     rc = SPK_NL_CALL(nl, sk_partition, ctx, st, rv, k, occ0, host[S_LONGEST], per_chunk, errp, su + S_OCC,
                      su + S_SKFILL, sj, &launches);
+    if (rc == kNotThisPath) return kSpans;
     if (rc) return rc;
     SPK_CUDA(cudaEventRecord(ks1.e, st));
     info.part_passes = 2;
     info.span_groups = 1;
     if ((rc = alloc_count_buffers())) return rc;
     SPK_CUDA(cudaEventRecord(kc0.e, st));
-    rc = SPK_NL_CALL(nl, sk_count, ctx, st, rv, sj, su + S_SKNEXT, k, kr.fm, &bv, lo, errp);
+    rc = SPK_NL_CALL(nl, sk_count, ctx, st, rv, sj, su + S_SKNEXT, k, occ0, kr.fm, &bv, lo, errp);
     if (rc) return rc;
     launches += 2;
   }
@@ -3896,7 +3907,7 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   DevBuf cbase, cfill, cregion, cfirst;
   if (!superk) {
   const uint64_t per = occ0 / nparts;
-  const uint64_t capu = nl >= 3 ? 2 * per + 512 : per + (per >> 1) + 256;
+  const uint64_t capu = span_region(per, nl);
   if ((rc = base.alloc((nparts_g + 1) * 8, st)) || (rc = fill.alloc(nparts_g * 4 * kFillStride, st)) ||
       (rc = region.alloc(nparts_g * capu * nl * 8, st)))
     return rc;
@@ -4005,7 +4016,9 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   if (err & 4) return fail(SPK_E_INVALID_ARG, "a read extends past the end of the packed data");
   if (err & 2) return fail(SPK_E_TIMEOUT, "count table: claim wait timed out");
   if (err & (int)kErrStage) return fail(SPK_E_TIMEOUT, "partition: a staged copy never completed");
-  if (superk && !(err & (int)kErrRegion) && (host[S_LFILL] > lcap_ || host[S_LFILL + 1] > scap_)) {
+  if (superk && (err & (int)kErrRepeat)) return kRedo;
+  if (superk && (err & (int)(kErrRegion | kErrHot))) return kSpans;
+  if (superk && (host[S_LFILL] > lcap_ || host[S_LFILL + 1] > scap_)) {
     // more distinct k-mers than the buffers were sized for (reads of low
     // coverage or many errors): again with room for them
     *slots = next_pow2(std::max(2 * host[S_LFILL], host[S_LFILL] + host[S_LFILL + 1]));
@@ -4206,22 +4219,36 @@ static int count_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsVie
 // overflow there) the general one.
 static int count_k_job(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& rv, unsigned k,
                        const spk_count_opts& o, KResult& kr) {
-  uint64_t slots = 0;
-  int rc = count_one_k_list(ctx, st, host, rv, k, o, &slots, kr);
   // More distinct k-mers than the buffers hold: again with room for what the
   // count found; a span with more than its slots: twice the slots, twice at most.
-  for (uint32_t grow = 1; rc == kGrow && grow <= 2; grow++) {
-    SPK_CUDA(cudaStreamSynchronize(st));  // the abandoned job's buffers are freed in stream order
-    spk_count_opts og = o;
-    if (!slots) og.table_log2 = kr.table.log2cap + 1;
-    kr = KResult();
-    rc = count_one_k_list(ctx, st, host, rv, k, og, &slots, kr);
-    if (rc == SPK_OK) {
-      kr.info.table_regrows = grow;
-      return SPK_OK;
+  // Super-k-mers given up (a minimizer too common, records that overflowed their
+  // stream): again by spans.
+  spk_count_opts og = o;
+  uint64_t slots = 0;
+  uint32_t grow = 0;
+  bool spans = false;
+  int rc;
+  for (;;) {
+    rc = count_one_k_list(ctx, st, host, rv, k, og, spans, &slots, kr);
+    if (rc == kSpans) {
+      spans = true;
+      slots = 0;
+      grow = 0;
+    } else if (rc == kGrow && grow < 2) {
+      grow++;
+      if (!slots) og.table_log2 = kr.table.log2cap + 1;
+    } else {
+      break;
     }
-    if (rc == SPK_E_OOM) rc = kRedo;  // the general path instead
+    SPK_CUDA(cudaStreamSynchronize(st));  // the abandoned job's buffers are freed in stream order
+    kr = KResult();
   }
+  if (rc == SPK_OK) {
+    kr.info.table_regrows = grow;
+    if (spans) kr.info.part_rescatters++;
+    return SPK_OK;
+  }
+  if (rc == SPK_E_OOM && (grow || spans)) rc = kRedo;  // the general path instead
   if (rc == kGrow) rc = kRedo;
   if (rc != kNotThisPath && rc != kRedo) return rc;
   // every uploaded piece of the reads, before the general path reads them
@@ -4229,7 +4256,7 @@ static int count_k_job(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const Read
   SPK_CUDA(cudaStreamSynchronize(st));  // the abandoned job's buffers are freed in stream order
   kr = KResult();
   const int rc2 = count_one_k(ctx, st, host, rv, k, o, kr);
-  if (!rc2 && rc == kRedo) kr.info.part_rescatters++;  // the first layout overflowed
+  if (!rc2 && (rc == kRedo || spans)) kr.info.part_rescatters++;  // the first layout overflowed
   return rc2;
 }
 

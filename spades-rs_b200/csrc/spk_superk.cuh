@@ -22,7 +22,9 @@
 //   k_bloom_ops  the Bloom operations of list and singletons, by Bloom range
 //
 // Bins have exact sizes, so no read set overflows them; a batch with more
-// distinct k-mers than slots is counted in parts (by hash bits), alone.
+// distinct k-mers than slots is counted in parts (by hash bits), alone, and a
+// bin too large for one CTA (SkLimits) sends the job to the spans, or where its
+// k-mers repeat too often for those to the general path.
 #pragma once
 
 #include "spk_bins.h"
@@ -323,8 +325,8 @@ __global__ void __launch_bounds__(kSkBinBlock) k_sk_bins_apply(const unsigned lo
 }
 
 // The stream's records to their bins.  A bin of more records than its word counts
-// (2^27 short reads of one sequence) sends the job to the general path, as a stream
-// that overflowed does.
+// (2^27 short reads of one sequence) sends the job to the spans, as a stream that
+// overflowed does.
 __global__ void __launch_bounds__(256) k_sk_place(SkStream S, const uint32_t* __restrict__ base,
                                                    uint64_t* __restrict__ out) {
   const uint64_t n = min((uint64_t)*S.fill, S.cap);
@@ -364,6 +366,28 @@ struct SkShape {
 // 32-bit words a record's bases take: at most w windows, w + k - 1 = 2k - m bases.
 __host__ __device__ __forceinline__ uint32_t sk_words(unsigned k) { return (2 * k - sk_m(k) + 15) / 16; }
 constexpr uint32_t kSkMaxRecs = 2048;  // a record's index takes 11 bits
+// What one CTA may spend on one batch before the job is given up and counted by
+// spans, which do not depend on minimizers.  A bin is never split, and a batch
+// with many times a table's distinct k-mers is counted in as many parts, each
+// staging all of its records: 20,000 reads around one minimizer (k = 55, 820,000
+// distinct k-mers) took 3.1 s on one CTA, by spans 2.7 ms.
+// A CTA counts about 150 windows a microsecond with its SM full.  The spans take
+// 1 to 3 ms of a small job and 0.06 ns an occurrence of a large one, or 0.2 to 0.4
+// where the k-mers repeat too and overflow their regions; the limit lets a CTA work
+// for about as long (1.3 ms and 0.1 ns an occurrence), so that neither a set it
+// would have finished sooner is given up (30 kb at 5,000x, k = 55: 11.8 ms against
+// 33 by spans; 5% of poly-G reads, 150,000 records in one bin: 6.0 against 40) nor
+// much is spent before one is.
+struct SkLimits {
+  uint32_t recs;  // records of a batch (at most 2^25: a reference holds 25 bits of record)
+  uint32_t cost;  // windows counted, and two for every record staged
+  uint32_t hot;   // a k-mer counted more often would overflow its span's region too
+};
+// slack: what a span's region holds beyond its mean share of the occurrences.
+static SkLimits sk_limits(uint64_t occ, uint64_t slack) {
+  const uint32_t cost = (uint32_t)std::min<uint64_t>(200000 + occ / 64, 1u << 26);
+  return SkLimits{cost / 2, cost, (uint32_t)std::min<uint64_t>(slack, 0xFFFFFFFFu)};
+}
 // Records staged at a time, and the entries (a power of two) of their table.
 struct SkStage {
   uint32_t rc, dd;
@@ -503,7 +527,7 @@ template <int NL>
 __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
     k_sk_count(const uint64_t* __restrict__ words, const uint64_t* __restrict__ recs,
                const uint32_t* __restrict__ bstart, uint32_t nbat, unsigned long long* __restrict__ next_batch,
-               unsigned k, uint32_t RC, uint32_t DD, ListOut lo, int* __restrict__ err) {
+               unsigned k, uint32_t RC, uint32_t DD, SkLimits lim, ListOut lo, int* __restrict__ err) {
   typedef SkShape<NL> P;
   constexpr uint32_t S = P::S;
   constexpr int TH = P::threads, kWarps = TH / 32, kRounds = (S + TH - 1) / TH;
@@ -526,33 +550,39 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
   __shared__ unsigned long long lbase[2];
   __shared__ unsigned s_hist[kHistBins];
   __shared__ uint32_t s_batch, s_used, s_live;
-  __shared__ int s_full;
+  __shared__ uint32_t s_spent, s_cost, s_staged;  // of the batch's parts before, of this one; its records staged
+  __shared__ int s_full, s_stop;
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t lmin = lo.lmin < 2 ? 2u : lo.lmin;
   const SkCut<NL> cut = sk_cut<NL>(k);
   constexpr uint64_t kFree = REF ? 0ULL : kEmpty;  // an empty slot
   uint64_t occ2 = 0;
+  // No more batches for any CTA once records are missing (the stream overflowed) or
+  // a batch is given up: the job runs again another way.  The flag alone would not
+  // do: threads of one CTA could see it or not.
+  auto stop_all = [&](uint32_t why) {
+    if (why) atomicOr(err, (int)why);
+    atomicMax(next_batch, (unsigned long long)nbat);
+  };
+  if (threadIdx.x == 0 && (*(volatile int*)err & (int)kErrRegion)) stop_all(0);
   for (int i = threadIdx.x; i < kHistBins; i += TH) s_hist[i] = 0;
   for (uint32_t i = threadIdx.x; i < S * KW; i += TH) keys[i] = kFree;
   for (uint32_t i = threadIdx.x; i < S; i += TH) cnt[i] = 0;
   for (;;) {
     __syncthreads();
-    // No more batches once records are missing (the stream overflowed) or a batch
-    // is too large: the job runs again another way.  Another CTA may raise the
-    // flag at any time, so one thread reads it for all.
-    if (threadIdx.x == 0) {
-      const int e = *(volatile int*)err;
-      const unsigned long long b = atomicAdd(next_batch, 1ULL);
-      s_batch = (e & (int)kErrRegion) ? nbat : (uint32_t)min((unsigned long long)nbat, b);
-    }
+    if (threadIdx.x == 0) s_batch = (uint32_t)min((unsigned long long)nbat, atomicAdd(next_batch, 1ULL));
     __syncthreads();
     const uint32_t bt = s_batch;
     if (bt >= nbat) break;
     const uint32_t r0 = bstart[bt], r1 = bstart[bt + 1];
     if (r0 == r1) continue;
-    if (REF && r1 - r0 > 1u << 25) {  // (a reference holds 25 bits of record)
-      if (threadIdx.x == 0) atomicOr(err, (int)kErrRegion);
+    if (r1 - r0 > lim.recs) {
+      if (threadIdx.x == 0) stop_all(kErrHot);
       continue;
+    }
+    if (threadIdx.x == 0) {
+      s_spent = s_cost = 0;
+      s_stop = 0;
     }
     // The batch, or the part of it whose hash bits [0, depth) are `part`: a part
     // with too many distinct k-mers for the table is cut in two.
@@ -561,6 +591,8 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
       if (threadIdx.x == 0) {
         s_used = 0;
         s_full = 0;
+        s_spent += s_cost;
+        s_cost = s_staged = 0;
       }
       for (uint32_t q0 = r0; q0 < r1; q0 += RC) {
         // ---- stage up to RC records: their bases, the first on top ----
@@ -644,6 +676,12 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
         }
         __syncthreads();
         const uint32_t nlive = s_live >> 20, nwin = s_live & 0xFFFFF;
+        if (threadIdx.x == 0) {
+          s_cost += nwin + 2 * n;
+          s_staged += n;
+          // (given up, here or by another CTA: a batch of several rounds looks)
+          if (s_spent + s_cost > lim.cost || (q0 != r0 && (*(volatile int*)err & (int)kErrHot))) s_full = s_stop = 1;
+        }
         // ---- count: each warp a share of the windows ----
         // Lanes without a k-mer to place take the next windows, a dozen at a
         // time at least; every turn is one probe step for the lanes that have
@@ -763,14 +801,30 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
       // (REF) the records still staged: those of the last round
       const uint32_t qlast = (r1 - r0 - 1) / RC * RC, nlast = r1 - r0 - qlast;
       if (s_full) {
-        // too many distinct k-mers: this part again as two
+        // too many distinct k-mers: this part again as two, unless the limit is
+        // reached or far away from what is ahead.  The table filled after a share
+        // of the records; if new k-mers kept coming, as many parts as that share
+        // goes into the whole would follow (on the way to the first part: for
+        // each of the parts ahead), each with all of the records.  They come ever
+        // more slowly where reads repeat, so eight times the limit is allowed.
+        uint32_t top = 0;
         for (uint32_t i = threadIdx.x; i < S * KW; i += TH) keys[i] = kFree;
-        for (uint32_t i = threadIdx.x; i < S; i += TH) cnt[i] = 0;
-        if (++depth > 16) {
-          if (threadIdx.x == 0) atomicOr(err, 1);
+        for (uint32_t i = threadIdx.x; i < S; i += TH) {
+          top = max(top, cnt[i]);
+          cnt[i] = 0;
+        }
+        if (threadIdx.x == 0) {
+          const float f = (float)(r1 - r0) / (float)s_staged;
+          const float ahead = (float)s_cost * f * f * (part == 0 ? (float)(1u << depth) : 1.f);
+          if (depth == 16 || ahead > 8.f * lim.cost) s_stop = 1;
+          if (s_stop) stop_all(kErrHot);
+        }
+        depth++;
+        __syncthreads();
+        if (s_stop) {
+          if (top > lim.hot) atomicOr(err, (int)kErrRepeat);
           break;
         }
-        __syncthreads();
         continue;
       }
       // ---- write the part out ----
@@ -851,13 +905,12 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
         for (uint32_t j = 0; j < KW; j++) keys[(size_t)KW * s + j] = kFree;
         cnt[s] = 0;
       }
-      // the next part: the sibling of the deepest one not yet counted
-      while (depth > 0 && (part >> (depth - 1) & 1)) {
-        depth--;
-        part &= (1u << depth) - 1;
-      }
-      if (depth == 0) break;
-      part |= 1u << (depth - 1);
+      // the next part, of the same depth (a shallower one would overflow as the
+      // parts around it did): the first bit counts most
+      uint32_t b = depth;
+      while (b > 0 && (part >> (b - 1) & 1)) part &= ~(1u << --b);
+      if (b == 0) break;
+      part |= 1u << (b - 1);
       __syncthreads();
     }
   }

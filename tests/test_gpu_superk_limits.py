@@ -65,3 +65,88 @@ def test_more_records_than_a_reference_holds(spk, ora):
                          list_min_count=1, flags=spk.SPK_F_EDGES | spk.SPK_F_KEEP_BLOOM)
     assert r.info(0)["occurrences"] == n + m
     check(spk, ora, r, np.concatenate([rest, np.repeat(hot, 3, axis=0)]), k, bits, hot=n)
+
+
+def small_hash_mmer(m):
+    """An m-mer of a small hash (sk_hash in csrc/spk_superk.cuh), as base codes: the
+    minimizer of nearly every window that holds it."""
+    rng = np.random.default_rng(m)
+    code = rng.integers(0, 1 << (2 * m), size=1 << 20, dtype=np.uint64)
+    rev, x = np.zeros_like(code), code.copy()
+    for _ in range(m):
+        rev = (rev << np.uint64(2)) | (np.uint64(3) - (x & np.uint64(3)))
+        x >>= np.uint64(2)
+    h = (np.minimum(code, rev).astype(np.uint32) ^ np.uint32(0x2545F491)) * np.uint32(0x9E3779B1)
+    h = (h ^ (h >> np.uint32(15))) * np.uint32(0x2C1B3C6D)
+    h ^= h >> np.uint32(13)
+    c = int(code[np.argmin(h)])
+    return np.array([(c >> (2 * (m - 1 - i))) & 3 for i in range(m)], np.uint8)
+
+
+def planted(k, n, seed):
+    """n reads of random bases around one m-mer: every window of every read has it
+    as its minimizer, and nearly every one is a k-mer of its own."""
+    m = 15 if k > 32 else 13 if k >= 27 else 11
+    rows = np.random.default_rng(seed).integers(0, 4, size=(n, 2 * k - m), dtype=np.uint8)
+    rows[:, k - m:k] = small_hash_mmer(m)
+    return rows
+
+
+@pytest.mark.parametrize("k,n,given_up", [(21, 1_000, 0), (21, 3_000, 1), (55, 300, 0), (55, 3_000, 1),
+                                          (31, 3_000, 1), (127, 100, 0), (77, 2_000, 1), (127, 3_000, 1)])
+def test_one_minimizer_of_many_kmers(spk, ora, k, n, given_up):
+    """A bin with a few times a table's k-mers is counted in parts; one with many
+    times that is not (its parts would each read all of it: the work grew with the
+    square of the reads) but by spans or, for a small set, in the table."""
+    rows = planted(k, n, seed=k)
+    rng = np.random.default_rng(k + 1)
+    # (k > 64: enough occurrences for the super-k-mers to take the set)
+    extra = rng.integers(0, 4, size=(0 if k <= 64 else 20_000, rows.shape[1]), dtype=np.uint8)
+    rows = np.concatenate([rows, rows[: n // 2], extra])
+    data = pack(rows)
+    nb = data.shape[1]
+    offs, lens = np.arange(rows.shape[0], dtype=np.uint64) * nb, np.full(rows.shape[0], rows.shape[1], np.uint32)
+    r = spk.count((data.reshape(-1), offs, lens), [k], bloom_bits=1 << 24, list_min_count=1,
+                  flags=spk.SPK_F_EDGES | spk.SPK_F_KEEP_BLOOM)
+    assert r.info(0)["part_rescatters"] == given_up
+    check(spk, ora, r, rows, k, 1 << 24)
+
+
+@pytest.mark.parametrize("k", [21, 55])
+def test_correcting_count_gives_up_too(spk, ora, k):
+    """The correcting count of such reads takes the reference's two passes."""
+    rows = np.repeat(planted(k, 3_000, seed=k), 2, axis=0)
+    rows[::7, 3] = (rows[::7, 3] + 1) % 4
+    data = pack(rows)
+    nb = data.shape[1]
+    n = rows.shape[0]
+    offs, lens = np.arange(n, dtype=np.uint64) * nb, np.full(n, rows.shape[1], np.uint32)
+    bits = 1 << 22
+    o = ora.count(data.reshape(-1), offs, lens, k, bits, mode=ora.MODE_TWICE, correct=True)
+    tk, tc = o.table(1)
+    r = spk.count((data.reshape(-1), offs, lens), [k], bloom_bits=bits, list_min_count=1,
+                  flags=spk.SPK_F_EDGES | spk.SPK_F_KEEP_BLOOM | spk.SPK_F_CORRECT)
+    gk, gc = r.kmers(0, 1)
+    np.testing.assert_array_equal(gk, tk)
+    np.testing.assert_array_equal(gc, tc)
+    for a, b in zip(r.bloom(0), o.bloom()):
+        np.testing.assert_array_equal(a, b)
+    assert r.info(0)["n_corrected_reads"] == o.stats()["corrected_reads"]
+
+
+def test_deep_locus(spk, ora):
+    """One locus of 400 bases read 60,000 times with errors: few minimizers, each
+    with thousands of records and of k-mers."""
+    rng = np.random.default_rng(9)
+    g = rng.integers(0, 4, 400, dtype=np.uint8)
+    start = rng.integers(0, 400 - 120, 60_000)
+    rows = g[start[:, None] + np.arange(120)[None, :]]
+    e = rng.random(rows.shape) < 0.004
+    rows[e] = (rows[e] + 1) % 4
+    data = pack(rows)
+    nb = data.shape[1]
+    n = rows.shape[0]
+    offs, lens = np.arange(n, dtype=np.uint64) * nb, np.full(n, 120, np.uint32)
+    r = spk.count((data.reshape(-1), offs, lens), [55], bloom_bits=1 << 24, list_min_count=1,
+                  flags=spk.SPK_F_EDGES | spk.SPK_F_KEEP_BLOOM)
+    check(spk, ora, r, rows, 55, 1 << 24)
