@@ -4018,9 +4018,11 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   if (err & (int)kErrStage) return fail(SPK_E_TIMEOUT, "partition: a staged copy never completed");
   if (superk && (err & (int)kErrRepeat)) return kRedo;
   if (superk && (err & (int)(kErrRegion | kErrHot))) return kSpans;
-  if (superk && (host[S_LFILL] > lcap_ || host[S_LFILL + 1] > scap_)) {
+  if (superk && (host[S_LFILL] > lcap_ || host[S_LFILL + 1] > scap_ ||
+                 ((err & (int)kErrRange) && host[S_LFILL] + host[S_LFILL + 1] > cap))) {
     // more distinct k-mers than the buffers were sized for (reads of low
-    // coverage or many errors): again with room for them
+    // coverage or many errors), each list or their Bloom operations: again with
+    // room for them
     *slots = next_pow2(std::max(2 * host[S_LFILL], host[S_LFILL] + host[S_LFILL + 1]));
     return kGrow;
   }

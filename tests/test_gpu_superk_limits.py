@@ -150,3 +150,22 @@ def test_deep_locus(spk, ora):
     r = spk.count((data.reshape(-1), offs, lens), [55], bloom_bits=1 << 24, list_min_count=1,
                   flags=spk.SPK_F_EDGES | spk.SPK_F_KEEP_BLOOM)
     check(spk, ora, r, rows, 55, 1 << 24)
+
+
+def test_more_bloom_operations_than_room(spk, ora):
+    """Distinct k-mers that fit the singletons' buffer and the list's, but whose Bloom
+    operations overflow theirs (1.4 of the slots): counted once more with room."""
+    rng = np.random.default_rng(6)
+    slots, k, bits = 1 << 17, 31, 1 << 24
+    once = rng.integers(0, 4, size=(int(0.93 * slots) // 101, 131), dtype=np.uint8)
+    more = rng.integers(0, 4, size=(int(0.47 * slots) // 101, 131), dtype=np.uint8)
+    rows = np.concatenate([once, np.repeat(more, 5, axis=0)])
+    assert slots / 2 < 0.3 * rows.shape[0] * 101 < slots
+    data = pack(rows)
+    n, nb = data.shape
+    offs, lens = np.arange(n, dtype=np.uint64) * nb, np.full(n, 131, np.uint32)
+    r = spk.count((data.reshape(-1), offs, lens), [k], bloom_bits=bits, list_min_count=1,
+                  flags=spk.SPK_F_EDGES | spk.SPK_F_KEEP_BLOOM)
+    info = r.info(0)
+    assert info["table_regrows"] == 1 and info["part_rescatters"] == 0
+    check(spk, ora, r, rows, k, bits)
