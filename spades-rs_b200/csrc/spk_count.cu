@@ -3150,6 +3150,31 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
   bool sk = false;
   DevBuf sk_list[4], sk_cnt;
   uint64_t sk_occ = 0, sk_longest = 0;
+  // The lists of such a count; cap entries each.
+  auto sk_lists = [&]() -> int {
+    int r2;
+    for (int j = 0; j < nl; j++)
+      if ((r2 = sk_list[j].alloc(cap * 8, st)) || (r2 = sgl[j].alloc(cap * 8, st))) return r2;
+    if ((r2 = sk_cnt.alloc(cap * 4, st))) return r2;
+    for (int j = 0; j < nl; j++) {
+      lo.l[j] = sk_list[j].as<uint64_t>();
+      lo.s[j] = sgl[j].as<uint64_t>();
+    }
+    lo.cnt = sk_cnt.as<uint32_t>();
+    lo.cap = lo.scap = cap;
+    lo.lmin = 2;
+    lo.fill = su + S_LFILL;
+    lo.hist = su + S_HIST;
+    lo.occ2 = su + S_OCC2;
+    return SPK_OK;
+  };
+  auto sk_release = [&]() {
+    for (int j = 0; j < nl; j++) {
+      sk_list[j].release();
+      sgl[j].release();
+    }
+    sk_cnt.release();
+  };
   // Partition and count of rv's super-k-mers into lo (and their Bloom operations).
   auto sk_both = [&](const RangeView* ranges) -> int {
     SkJob sj;
@@ -3388,9 +3413,10 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
   } else {
     // ---- gated: Stage 2 first ----
     // With error correction (and no use for a table), both stages count super-
-    // k-mers as the default job does, if the k-mers of the reads take at most an
-    // eighth of the memory: the tiers come from the distinct k-mers of the reads,
-    // and the corrected reads' k-mers are admitted against them once counted.
+    // k-mers as the default job does, if the list, the singletons and the Bloom
+    // operations of the reads take at most an eighth of the memory: the tiers come
+    // from the distinct k-mers of the reads, and the corrected reads' k-mers are
+    // admitted against them once counted.
     // (SPK_F_GATED alone asks for a table of the admitted k-mers only.)
     if (correct && !ref && !table_wanted && !o.table_log2 && !o.span_groups_log2 && use_ops && sk_fits(k)) {
       k_occ<<<grid_for(ctx, 2), kBlock, 0, st>>>(rv.lengths, rv.n_reads, k, su + S_OCC0, su + S_LONGEST);
@@ -3401,33 +3427,34 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
       sk_longest = host[S_LONGEST];
       cap = list_capacity(sk_occ, nl);
       if (sk_occ > 0 && cap <= ctx->total_mem / 8 / (16 * nl + 20)) {
-        const uint64_t rcap = 3 * cap / nranges + 1 + 3 * cap / nranges / 4 + 1024;
-        if ((rc = rbase.alloc((nranges + 1) * 8, st)) || (rc = rfill.alloc(nranges * 4 * kFillStride, st)) ||
-            (rc = ops.alloc(nranges * rcap * 4, st)) || (rc = sk_cnt.alloc(cap * 4, st)))
-          return rc;
-        for (int j = 0; j < nl; j++)
-          if ((rc = sk_list[j].alloc(cap * 8, st)) || (rc = sgl[j].alloc(cap * 8, st))) return rc;
-        SPK_CUDA(cudaMemsetAsync(rfill.p, 0, nranges * 4 * kFillStride, st));
-        bv = RangeView{ops.as<uint32_t>(), rbase.as<uint64_t>(), rfill.as<unsigned int>(), rcap, (uint32_t)nranges, errp};
-        for (int j = 0; j < nl; j++) {
-          lo.l[j] = sk_list[j].as<uint64_t>();
-          lo.s[j] = sgl[j].as<uint64_t>();
-        }
-        lo.cnt = sk_cnt.as<uint32_t>();
-        lo.cap = lo.scap = cap;
-        lo.lmin = 2;
-        lo.fill = su + S_LFILL;
-        lo.hist = su + S_HIST;
-        lo.occ2 = su + S_OCC2;
-        SPK_CUDA(cudaEventRecord(kb0.e, st));
-        rc = sk_both(&bv);
-        if (!rc) rc = fetch(kWords);
-        if (rc && rc != kNotThisPath) return rc;
+        auto stage2 = [&]() -> int {
+          int r2;
+          const uint64_t rcap = 3 * cap / nranges + 1 + 3 * cap / nranges / 4 + 1024;
+          if ((r2 = rbase.alloc((nranges + 1) * 8, st)) || (r2 = rfill.alloc(nranges * 4 * kFillStride, st)) ||
+              (r2 = ops.alloc(nranges * rcap * 4, st)) || (r2 = sk_lists()) ||
+              (r2 = kr.seen.alloc(kr.num_words * 8, st)) || (r2 = kr.twice.alloc(kr.num_words * 8, st)))
+            return r2;
+          SPK_CUDA(cudaMemsetAsync(rfill.p, 0, nranges * 4 * kFillStride, st));
+          bv = RangeView{ops.as<uint32_t>(), rbase.as<uint64_t>(), rfill.as<unsigned int>(), rcap, (uint32_t)nranges,
+                         errp};
+          SPK_CUDA(cudaEventRecord(kb0.e, st));
+          if ((r2 = sk_both(&bv))) return r2;
+          return fetch(kWords);
+        };
+        rc = stage2();
+        if (rc && rc != kNotThisPath && rc != SPK_E_OOM) return rc;
         sk = !rc && !((int)host[S_ERR] & (int)(kErrHot | kErrRegion | kErrRange)) && host[S_LFILL] <= cap &&
              host[S_LFILL + 1] <= cap;
-        if (!sk) {  // sequences or coverage this was not sized for: the reference's two passes
+        // Sequences or coverage this was not sized for, or no room: the reference's
+        // two passes, which need less.
+        if (!sk) {
+          sk_release();
           bv.ops = nullptr;
           ops.release();
+          rbase.release();
+          rfill.release();
+          kr.seen.release();
+          kr.twice.release();
           SPK_CUDA(cudaMemsetAsync(sw, 0, kWords * 8, st));
         }
       }
@@ -3442,8 +3469,8 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
     }
   }
   // the compact tiers (every schedule)
-  if ((rc = kr.seen.alloc(kr.num_words * 8, st))) return rc;
-  if ((rc = kr.twice.alloc(kr.num_words * 8, st))) return rc;
+  if (!kr.seen.p && (rc = kr.seen.alloc(kr.num_words * 8, st))) return rc;
+  if (!kr.twice.p && (rc = kr.twice.alloc(kr.num_words * 8, st))) return rc;
   if (bv.ops) {
     // partitioned: apply the binned operations range by range
     SPK_CUDA(cudaEventRecord(kb0.e, st));
@@ -3470,7 +3497,12 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
   DevBuf cdata;  // SPK_F_CORRECT: the corrected copy of the packed reads
   if (correct) {
     // ---- Stage 3 error correction (src/assemble.rs:183-191) into a copy ----
-    if ((rc = cdata.alloc(rv.data_len + 128, st))) return rc;
+    rc = cdata.alloc(rv.data_len + 128, st);
+    if (rc == SPK_E_OOM && sk) {  // (Stage 3 then asks for its lists again)
+      sk_release();
+      rc = cdata.alloc(rv.data_len + 128, st);
+    }
+    if (rc) return rc;
     SPK_CUDA(cudaMemsetAsync(cdata.as<uint8_t>() + rv.data_len, 0, 128, st));
     SPK_CUDA(cudaEventRecord(ec0.e, st));
     uint64_t nc = 0;
@@ -3485,14 +3517,19 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
   }
   if (sk) {
     // ---- Stage 3: the corrected reads' k-mers, admitted against the tiers ----
-    for (int j = 0; j < nl; j++)
-      if ((rc = kr.list[j].alloc(cap * 8, st))) return rc;
-    if ((rc = kr.list[4].alloc(cap * 4, st))) return rc;
-    SPK_CUDA(cudaMemsetAsync(su + S_SUMS, 0, 4 * 8, st));
-    SPK_CUDA(cudaMemsetAsync(su + S_LFILL, 0, (S_WORDS - S_LFILL) * 8, st));  // fills, occurrences, histogram
-    SPK_CUDA(cudaMemsetAsync(su + S_SKFILL, 0, 2 * 8, st));
-    SPK_CUDA(cudaEventRecord(kc0.e, st));
-    if ((rc = sk_both(nullptr)) && rc != kNotThisPath) return rc;
+    auto stage3 = [&]() -> int {
+      int r2;
+      for (int j = 0; j < nl; j++)
+        if ((r2 = kr.list[j].alloc(cap * 8, st))) return r2;
+      if ((r2 = kr.list[4].alloc(cap * 4, st)) || (!sk_cnt.p && (r2 = sk_lists()))) return r2;
+      SPK_CUDA(cudaMemsetAsync(su + S_SUMS, 0, 4 * 8, st));
+      SPK_CUDA(cudaMemsetAsync(su + S_LFILL, 0, (S_WORDS - S_LFILL) * 8, st));  // fills, occurrences, histogram
+      SPK_CUDA(cudaMemsetAsync(su + S_SKFILL, 0, 2 * 8, st));
+      SPK_CUDA(cudaEventRecord(kc0.e, st));
+      return sk_both(nullptr);
+    };
+    rc = stage3();
+    if (rc && rc != kNotThisPath && rc != SPK_E_OOM) return rc;
     const bool part = !rc;
     // (the count's own histogram is of all its k-mers: admission starts it again)
     SPK_CUDA(cudaMemsetAsync(su + S_HIST, 0, kHistBins * 8, st));
@@ -3510,7 +3547,11 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
     if ((rc = fetch(kWords))) return rc;
     sk = part && !((int)host[S_ERR] & (int)(kErrHot | kErrRegion)) && host[S_LFILL] <= cap && host[S_LFILL + 1] <= cap &&
          host[S_SUMS + 3] <= cap;
-    if (!sk) SPK_CUDA(cudaMemsetAsync(su + S_SUMS, 0, (S_WORDS - S_SUMS) * 8, st));
+    sk_release();
+    if (!sk) {
+      for (int j = 0; j < 5; j++) kr.list[j].release();
+      SPK_CUDA(cudaMemsetAsync(su + S_SUMS, 0, (S_WORDS - S_SUMS) * 8, st));
+    }
   }
   if (gated && !sk) {
     // ---- gated: Stage 3 over admitted occurrences ----
