@@ -2970,25 +2970,32 @@ static void launch_sk_reads(spk_ctx* ctx, cudaStream_t st, const ReadsView& rv, 
   const uint32_t rpw = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(rv.n_reads / (warps * 4), 1), 32);
   k_sk_reads<R><<<grid, kSkReadBlock, 0, st>>>(rv, k, sk_m(k), rpw, S, occ);
 }
+// m-mer positions a lane of k_sk_reads holds: those of the longest read if a warp's
+// are at most 256 (else in segments of 256), and at least 32 windows' worth.
+static uint32_t sk_positions(unsigned k, uint64_t longest) {
+  const uint32_t m = sk_m(k), w = k - m + 1;
+  const uint64_t want = std::max<uint64_t>(longest > m ? longest - m + 1 : 1, w + 31);
+  return want <= 96 ? 3 : want <= 128 ? 4 : want <= 160 ? 5 : want <= 192 ? 6 : 8;
+}
+// Stream entries of a read set in `pieces` launches of up to `warps` warps.  A random
+// sequence has 2 / (w + 1) runs per window, every read and segment one more; a
+// stream that overflows (sequences made of other things) sends the job to the spans.
+static uint64_t sk_stream_entries(unsigned k, uint64_t occ, uint64_t n_reads, uint64_t longest, uint64_t warps,
+                                  uint64_t pieces) {
+  const uint32_t w = k - sk_m(k) + 1, seg = 32 * sk_positions(k, longest) - w + 1;
+  return (uint64_t)((double)occ * (2.8 / (w + 1) + 1.0 / seg)) + n_reads + n_reads / 2 +
+         pieces * std::min<uint64_t>(warps, n_reads) * kSkChunk + 4096;
+}
 // occ: the k-mer windows of the reads; longest: the longest read.
 template <int NL>
 static int sk_partition(spk_ctx* ctx, cudaStream_t st, const ReadsView& rv, unsigned k, uint64_t occ,
                         uint64_t longest, bool per_chunk, int* errp, unsigned long long* occ_out,
                         unsigned long long* fill, SkJob& sj, uint32_t* launches) {
-  const uint32_t m = sk_m(k), w = k - m + 1;
-  // m-mer positions a warp holds: the longest read's, if that is at most 256
-  // (else in segments of 256), and at least 32 windows' worth
-  const uint64_t want = std::max<uint64_t>(longest > m ? longest - m + 1 : 1, w + 31);
-  const uint32_t R = want <= 96 ? 3 : want <= 128 ? 4 : want <= 160 ? 5 : want <= 192 ? 6 : 8;
-  const uint32_t seg = 32 * R - w + 1;
-  // A random sequence has 2 / (w + 1) runs per window, every read and segment
-  // one more; a stream that overflows (sequences made of other things) sends
-  // the job to the general path.
+  const uint32_t R = sk_positions(k, longest);
   uint32_t nbins = 4096;
   while (nbins < kSkMaxBins && (uint64_t)nbins * 512 < occ) nbins *= 2;
   const uint64_t warps = (uint64_t)grid_for(ctx, 8) * (kSkReadBlock / 32);
-  const uint64_t cap = (uint64_t)((double)occ * (2.8 / (w + 1) + 1.0 / seg)) + rv.n_reads + rv.n_reads / 2 +
-                       (rv.chunks ? rv.chunks->n : 1) * std::min<uint64_t>(warps, rv.n_reads) * kSkChunk + 4096;
+  const uint64_t cap = sk_stream_entries(k, occ, rv.n_reads, longest, warps, rv.chunks ? rv.chunks->n : 1);
   if (cap >= (1ULL << 32)) return kNotThisPath;
   // Windows per batch: what fits a table, or fewer so that every CTA has one
   const uint32_t T = (uint32_t)std::min<uint64_t>(
@@ -3781,6 +3788,19 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
 // handles them), kRedo after an overflow, else the status.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kMaxLog2Groups = 4;  // at most 16 passes over the reads
+// Partition buffers of a read set in 2^lg groups of spans: regions, and coarse buckets
+// of 1.125x their mean share (2.6 keys per occurrence, in quarter keys).
+static uint64_t span_part_bytes(uint64_t occ, int nl, uint32_t lg) {
+  return ((occ >> lg) * (nl >= 3 ? 13 : 11) / 4 + (1u << 22)) * (uint64_t)nl * 8;
+}
+// Span groups: a read set whose partition buffers would pass a quarter of the device
+// is partitioned and counted in 2^lg passes, each keeping the keys of one group of
+// spans.
+static uint32_t span_groups(uint64_t occ, int nl, uint32_t asked, uint64_t total_mem) {
+  uint32_t lg = std::min<uint32_t>(asked, kMaxLog2Groups);
+  while (lg < kMaxLog2Groups && span_part_bytes(occ, nl, lg) > total_mem / 4) lg++;
+  return lg;
+}
 
 // A second stream of one job, joined back to the job's stream by events.
 struct SideStream {
@@ -3852,20 +3872,13 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
                 (nl <= 2 || log2cap > log2span + kCoarseBits);
   if (!superk && log2cap <= log2span) return kNotThisPath;
   const uint32_t log2parts = log2cap > log2span ? log2cap - log2span : 0;
-  // Span groups: a read set whose partition buffers (span regions and coarse
-  // buckets, 2.6 keys per occurrence) would pass a quarter of the device is
-  // partitioned and counted in 2^lg passes, each keeping the keys of one group
-  // of spans (the reads are streamed once per pass).
-  // (The coarse buckets hold 1.125x their mean share.)
-  const uint64_t part_keys4 = nl >= 3 ? 13 : 11;  // regions + buckets, in quarter keys per occurrence
-  auto part_bytes = [&](uint32_t g) { return ((occ0 >> g) * part_keys4 / 4 + (1u << 22)) * (uint64_t)nl * 8; };
-  uint32_t lg = std::min<uint32_t>(o.span_groups_log2, kMaxLog2Groups);
-  while (lg < kMaxLog2Groups && part_bytes(lg) > ctx->total_mem / 4) lg++;
-  if (part_bytes(lg) > ctx->total_mem / 4) return kNotThisPath;
+  // (Span groups: the reads are streamed once per pass.)
+  uint32_t lg = span_groups(occ0, nl, o.span_groups_log2, ctx->total_mem);
+  if (span_part_bytes(occ0, nl, lg) > ctx->total_mem / 4) return kNotThisPath;
   while (lg > 0 && log2parts - lg <= kCoarseBits) lg--;
   superk = superk && lg == 0;  // (read sets that need groups take them)
   if (!superk && (!SPK_TWO_LEVEL || log2parts - lg <= kCoarseBits || log2parts - lg - kCoarseBits > kFineMaxBits ||
-                  part_bytes(lg) > ctx->total_mem / 4))
+                  span_part_bytes(occ0, nl, lg) > ctx->total_mem / 4))
     return kNotThisPath;
   // The span count holds at most one distinct k-mer per slot (a full span
   // sends the job back), so the singleton keys and the list, up to one entry
@@ -4208,6 +4221,35 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   info.kernel_launches = launches;
   info.schedule = SPK_SCHEDULE_PARTITIONED;
   return SPK_OK;
+}
+
+// Device bytes at the peak of a count by super-k-mers, apart from the reads and what
+// the result keeps; 0 where count_one_k_list (correct: count_one_k) does not take
+// them.  The solid k-mers are taken as a quarter of the slots (coverage of about 10;
+// fewer above).
+uint64_t superk_peak(unsigned k, uint64_t occ, uint64_t n_reads, uint64_t longest, uint64_t words,
+                     const spk_count_opts& o, uint64_t data_len, uint64_t total_mem) {
+  const int nl = (int)((k + 31) / 32), nle = (int)((k + 1 + 31) / 32);
+  const uint64_t cap = list_capacity(occ, nl), key = nl * 8, entry = key + 4;
+  const uint64_t nranges = (words * 64 + (1ULL << kLog2Range) - 1) >> kLog2Range;
+  const bool correct = (o.flags & SPK_F_CORRECT) != 0;
+  if (!sk_fits(k) || o.table_log2 || o.span_groups_log2 || occ == 0 || nranges > kMaxRanges) return 0;
+  if (correct ? cap > total_mem / 8 / (16 * nl + 20)
+              : (nl > 2 && cap >> part_log2span(nl) <= kCoarse) || span_groups(occ, nl, 0, total_mem) != 0)
+    return 0;
+  const uint64_t stream = sk_stream_entries(k, occ, n_reads, longest, 148 * 64, 1);  // 16 bytes, and 8 in their bins
+  const uint64_t ops = (3 * cap * 5 / 4 + 1024 * nranges) * 4, tiers = words * 16;
+  const uint64_t edges = o.flags & SPK_F_EDGES ? 2 * max_edges(cap / 4) * nle * 8 : 0;  // and their sort's copy
+  uint64_t peak;
+  if (correct) {
+    // either stage's lists beside its stream, then Stage 3's list beside its edges
+    peak = std::max(cap * (entry + key) + ops, cap * (2 * entry + key) + data_len) + tiers + 24 * stream;
+    peak = std::max(peak, cap * entry + tiers + edges + data_len);
+  } else {
+    peak = std::max(24 * stream, 8 * stream + cap / 2 * entry + cap * key + ops);
+    peak = std::max(peak, cap * key + edges) + tiers;
+  }
+  return peak + (peak >> 3);  // (requests are rounded up, by an eighth at most)
 }
 
 // Device buffers of a k allocated on another stream: stream-ordered frees

@@ -28,6 +28,9 @@ int upload_reads(spk_result* res, cudaStream_t st, const uint8_t* data, size_t d
                  const uint64_t* offsets, const uint32_t* lengths, size_t n_reads, ReadsView* rv,
                  bool chunked);
 
+uint64_t superk_peak(unsigned k, uint64_t occ, uint64_t n_reads, uint64_t longest, uint64_t words,
+                     const spk_count_opts& o, uint64_t data_len, uint64_t total_mem);
+
 static uint64_t next_pow2_u64(uint64_t x) {
   uint64_t p = 1;
   while (p < x) p <<= 1;
@@ -39,13 +42,16 @@ static uint64_t next_pow2_u64(uint64_t x) {
 // spk_count picks:
 //   occurrences      4 per packed byte less k - 1 per read (reads of >= k bases)
 //   table capacity   next_pow2(0.3 occ), at least 1024 slots
-//   default job      (12 <= k <= 64, partition within a quarter of the device)
+//   super-k-mers     the default job and the correcting one: superk_peak
+//                    (records, list and singleton keys, Bloom operations)
+//   spans            (k = 12..20, 64, or more occurrences than one partition)
 //     first pass     span regions 1.5 occ keys + coarse buckets 1.125 occ keys
 //     span count     regions + list and singleton keys (one entry per slot
 //                    each) + Bloom operations (3.75 per slot) + the list's
 //                    sort temporaries + both tiers
 //   other schedules  the table (slots of 16/32/64 bytes), the interleaved
-//                    tiers, and a list of a quarter of the slots with its sort
+//                    tiers beside the compact ones made of them, and a list of
+//                    a quarter of the slots with its sort
 // Reads and outputs (list, edges, kept tiers) are added on top.  A job that
 // outgrows the estimate still runs; the batch re-runs a job that ran out of
 // memory alone after the others.
@@ -57,6 +63,8 @@ uint64_t job_estimate(const spk_job& j, uint64_t total_mem) {
   uint64_t bytes = j.data_len + 64 + j.n_reads * 12;
   const bool plain = !(o.flags & (SPK_F_GATED | SPK_F_CORRECT | SPK_F_REF_SOLID | SPK_F_DIRECT | SPK_F_KEEP_TABLE)) &&
                      !(o.n_prior > 0 && o.prior_seqs);
+  const bool correcting = (o.flags & SPK_F_CORRECT) && !(o.flags & (SPK_F_REF_SOLID | SPK_F_KEEP_TABLE)) &&
+                          !(o.n_prior > 0 && o.prior_seqs);
   for (int i = 0; i < j.n_k; i++) {
     const uint32_t k = j.ks ? j.ks[i] : 31;
     const uint64_t nl = (k + 31) / 32;
@@ -66,12 +74,15 @@ uint64_t job_estimate(const spk_job& j, uint64_t total_mem) {
     const uint64_t cap = std::max<uint64_t>(next_pow2_u64(nl <= 2 ? occ * 3 / 10 + 1 : occ * 9 / 20 + 1), 1024);
     const uint64_t key = nl * 8, entry = nl * 8 + 4;
     const uint64_t tiers = words * 16 + (o.flags & SPK_F_REF_SOLID ? words * 8 : 0);
-    uint64_t peak;
+    const uint64_t longest = j.n_reads ? b4 / j.n_reads : 0;  // (taken as even)
+    uint64_t peak = plain || correcting ? superk_peak(k, occ, j.n_reads, longest, words, o, j.data_len, total_mem) : 0;
     // span groups: as many passes as keep the partition within a quarter of the device
     const uint64_t q4 = nl >= 3 ? 13 : 11;  // partition keys per occurrence, in quarters
     uint32_t lg = 0;
     while (lg < 4 && ((occ >> lg) * q4 / 4 + (1u << 22)) * key > total_mem / 4) lg++;
-    if (plain && k >= 12 && !(nl >= 3 && 2 * k == 64 * nl) &&
+    if (peak) {
+      // by super-k-mers
+    } else if (plain && k >= 12 && !(nl >= 3 && 2 * k == 64 * nl) &&
         ((occ >> lg) * q4 / 4 + (1u << 22)) * key <= total_mem / 4) {
       const uint64_t og = occ >> lg;
       const uint64_t lcap = lg ? cap / 2 : cap, scap = cap;
@@ -82,7 +93,7 @@ uint64_t job_estimate(const spk_job& j, uint64_t total_mem) {
       peak = std::max(first, count) + (lg ? count - regions : 0);
     } else {
       const uint64_t slot = nl == 1 ? 16 : (nl <= 3 ? 32 : 64);
-      peak = cap * slot + tiers + (cap / 4) * entry * 2;
+      peak = cap * slot + tiers + words * 16 + (cap / 4) * entry * 2;
     }
     // outputs: the list and about one edge per listed k-mer
     peak += (cap / 4) * (entry + (k + 32) / 32 * 8);
