@@ -1302,10 +1302,10 @@ __device__ __forceinline__ uint64_t range_base(const RangeView& rv, uint32_t r) 
 #endif
 constexpr bool kSortedOps = SPK_SORTED_OPS;
 
-// get(i, st): the three positions stashed for item i of nslots, "count >= 2" in
-// bit 31 of the first; false if the item has none.
-template <class Get>
-__device__ __forceinline__ void span_emit_sorted(Get get, uint32_t nslots, uint32_t* buf, uint32_t S,
+// A slot's key holds its k-mer's three positions, "count >= 2" in bit 31 of the first;
+// an empty slot's stays all ones.
+template <int NL>
+__device__ __forceinline__ void span_emit_sorted(const typename SpanKey<NL>::T* keys, uint32_t* buf, uint32_t S,
                                                  uint32_t* rs, uint32_t* rcur,
                                                  const unsigned long long* rbase, const RangeView& rv) {
   __shared__ uint32_t wpart[32], wmax[32], bnd[8];
@@ -1354,9 +1354,9 @@ __device__ __forceinline__ void span_emit_sorted(Get get, uint32_t nslots, uint3
   const uint32_t total = s_total, H = s_maxc <= (S >> 1) ? S - s_maxc : 0u;
   if (H == 0) {
     // direct emission (a range holds more than half a span's worth)
-    for (uint32_t i = threadIdx.x; i < nslots; i += blockDim.x) {
-      uint32_t st[3];
-      if (!get(i, st)) continue;
+    for (uint32_t i = threadIdx.x; i < S; i += blockDim.x) {
+      const uint32_t* st = (const uint32_t*)&keys[i];
+      if (st[1] == 0xFFFFFFFFu) continue;
       const uint32_t flag = st[0] >> 31;
       const uint32_t pk[3] = {st[0] & 0x7FFFFFFFu, st[1], st[2]};
 #pragma unroll
@@ -1386,9 +1386,9 @@ __device__ __forceinline__ void span_emit_sorted(Get get, uint32_t nslots, uint3
   __syncthreads();
   for (uint32_t g = 0; g < G; g++) {
     const uint32_t gb = g * H;
-    for (uint32_t i = threadIdx.x; i < nslots; i += blockDim.x) {
-      uint32_t st[3];
-      if (!get(i, st)) continue;
+    for (uint32_t i = threadIdx.x; i < S; i += blockDim.x) {
+      const uint32_t* st = (const uint32_t*)&keys[i];
+      if (st[1] == 0xFFFFFFFFu) continue;
       const uint32_t flag = st[0] >> 31;
       const uint32_t pk[3] = {st[0] & 0x7FFFFFFFu, st[1], st[2]};
 #pragma unroll
@@ -1658,14 +1658,7 @@ __global__ void __launch_bounds__(kPartBlock, kPartCtasPerSm) k_part_count(PartV
       }
       __syncthreads();
       if (NL >= 2 && kSortedOps) {
-        span_emit_sorted(
-            [&](uint32_t i, uint32_t (&st)[3]) {
-              const uint32_t* q = (const uint32_t*)&keys[i];
-#pragma unroll
-              for (int j = 0; j < 3; j++) st[j] = q[j];
-              return st[1] != 0xFFFFFFFFu;  // (an empty slot's stash stays all ones)
-            },
-            S, cnt, S, rhist, rcur, rbase, rv);
+        span_emit_sorted<NL>(keys, cnt, S, rhist, rcur, rbase, rv);
       } else {
       // Emit the operations.
       for (uint32_t s = threadIdx.x; s < S; s += blockDim.x) {
@@ -3775,17 +3768,17 @@ int count_one_k(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& 
 }
 
 // ---------------------------------------------------------------------------
-// The default job for 12 <= k <= 64 with few host round trips.  It runs the
-// partitioned schedule with the two-level read partition and the span count
-// writing the k-mer list (no table), and reads device values back three
-// times: the occurrence count that sizes the table, one block of counters
-// after the cutoff (sizes of the lists, the histogram, the overflow flags),
-// and the edge count at the end.  Region, bucket and range overflows (skewed
-// inputs) and full spans are only checked at the mid-job readback: the
-// kernels keep every access inside its buffer, and on any overflow the job is
-// counted again by count_one_k, which lays the buffers out exactly.
+// The default job (k >= 12 but 96) with few host round trips.  It counts the reads'
+// super-k-mers (spk_superk.cuh) or, where those are not taken or given up, the keys
+// of a two-level partition by table spans; either writes the k-mer list (no table).
+// Device values are read back three times: the occurrence count that sizes the
+// buffers, one block of counters after the cutoff (sizes of the lists, the
+// histogram, the overflow flags), and the edge count at the end.  Overflows are
+// only checked at the mid-job readback: the kernels keep every access inside its
+// buffer, and on any overflow the job is counted again, with more room (kGrow), by
+// spans (kSpans) or by count_one_k, which lays the buffers out exactly.
 // Returns kNotThisPath when the inputs need another layout (count_one_k
-// handles them), kRedo after an overflow, else the status.
+// handles them), kRedo, kGrow or kSpans after an overflow, else the status.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kMaxLog2Groups = 4;  // at most 16 passes over the reads
 // Partition buffers of a read set in 2^lg groups of spans: regions, and coarse buckets
@@ -3802,21 +3795,19 @@ static uint32_t span_groups(uint64_t occ, int nl, uint32_t asked, uint64_t total
   return lg;
 }
 
-// A second stream of one job, joined back to the job's stream by events.
+// A second stream of one job, forked from the job's stream by an event.
 struct SideStream {
   cudaStream_t s = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr;
+  cudaEvent_t fork = nullptr;
   int open() {
     s = pooled_stream();
     fork = pooled_event(false);
-    join = pooled_event(false);
-    if (!s || !fork || !join) return fail(SPK_E_CUDA, "side stream or events");
+    if (!s || !fork) return fail(SPK_E_CUDA, "side stream or event");
     return SPK_OK;
   }
   ~SideStream() {
     pooled_stream_put(s);  // work still queued on it runs before its next user's
     pooled_event_put(fork, false);
-    pooled_event_put(join, false);
   }
 };
 
@@ -3826,7 +3817,8 @@ struct SideStream {
 int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsView& rv_in, unsigned k,
                      const spk_count_opts& o, bool spans, uint64_t* slots, KResult& kr) {
   const int nl = (int)((k + 31) / 32);
-  // (k = 96 fills its top limb, which the solid set's empty mark needs free)
+  // (k = 96, which fills its top limb, stays with the general path: the solid set no
+  // longer needs a spare bit there, but the schedules below are not tested with it)
   if (k < 12 || (nl >= 3 && 2 * k == 64u * nl)) return kNotThisPath;
   if (o.flags & (SPK_F_GATED | SPK_F_CORRECT | SPK_F_REF_SOLID | SPK_F_DIRECT | SPK_F_KEEP_TABLE))
     return kNotThisPath;
@@ -3865,9 +3857,12 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   const uint32_t log2span = part_log2span(nl);
   uint32_t log2cap = 0;
   while ((1ULL << log2cap) < cap) log2cap++;
-  // Super-k-mers unless the caller sizes the table or the groups of spans: read
-  // sets of any size for k <= 63, and for wider keys those with spans enough for
-  // two partition levels (smaller ones count with global atomics).
+  // Super-k-mers unless the caller sizes the table or the groups of spans: small
+  // read sets too for k <= 63, for wider keys those with spans enough for two
+  // partition levels (smaller ones count with global atomics, as before the super-
+  // k-mers).  Read sets that need span groups are counted by spans: by the spans'
+  // memory, not by what the records need, from about 2.1 G occurrences (k <= 32),
+  // 1.0 G (33..63), 0.6 G (65..95) or 0.4 G (97..127) on.
   bool superk = !spans && sk_fits(k) && !o.table_log2 && !o.span_groups_log2 && occ0 > 0 &&
                 (nl <= 2 || log2cap > log2span + kCoarseBits);
   if (!superk && log2cap <= log2span) return kNotThisPath;

@@ -298,10 +298,6 @@ struct DevSort {
   bool has_vals = false;
   bool pending = false;
   DevBuf tk[4], tv, work;
-  void rehome(cudaStream_t s) {
-    for (DevBuf& b : tk) b.st = s;
-    tv.st = work.st = s;
-  }
   void release() {
     for (DevBuf& b : tk) b.release();
     tv.release();

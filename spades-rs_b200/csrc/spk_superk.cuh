@@ -40,8 +40,9 @@ typedef BinWord<36> SkBin;            // 2^36 windows; 2^28 records, of which ha
 // Length of the minimizers: 15 above 32 bases; 13 and 11 below, where a longer
 // one leaves fewer windows per super-k-mer.
 __host__ __device__ constexpr unsigned sk_m(unsigned k) { return k > 32 ? 15u : k >= 27 ? 13u : 11u; }
-// k this partition takes: windows of at least 11 m-mers (and, for keys of several
-// limbs, a top limb with a bit to spare, as the solid set needs).
+// k this partition takes: windows of at least 11 m-mers.  k = 64 and 96, which fill
+// their top limb, keep the schedules they had (spans, and the table): nothing here
+// needs the spare bits, but the two have not been timed this way.
 __host__ constexpr bool sk_fits(unsigned k) { return k >= 21 && (k <= 32 || 2 * k < 64 * ((k + 31) / 32)); }
 
 struct SkStream {
@@ -359,9 +360,9 @@ struct SkShape {
   // Windows per batch: about a third of the slots filled at the distinct share of
   // the benchmark's reads (0.14 of the occurrences at k = 21, 0.27 at 55, 0.38 at
   // 77, 0.52 at 127); fuller tables probe longer, emptier ones end in more batches
-  // (k = 55: 4.73, 4.50, 4.40, 4.40 ms at 6,500, 5,500, 4,500, 4,000 in 4,096 slots).
+  // (k = 55, 5 Mb x 100x: 4.26, 4.28, 4.25, 4.26, 4.43 ms at 2,000, 2,400, 2,800,
+  // 3,400, 4,000 in 2,048 slots; k = 33, 3 Mb x 60x: 1.53, 1.48, 1.45, 1.46, 1.50).
   static constexpr uint32_t T = NL == 1 ? 3500 : NL == 2 ? 2800 : NL == 3 ? 4100 : 2600;
-  static constexpr uint32_t slot = ref ? 8 : 8 * NL;  // bytes of a slot's key
 };
 // 32-bit words a record's bases take: at most w windows, w + k - 1 = 2k - m bases.
 __host__ __device__ __forceinline__ uint32_t sk_words(unsigned k) { return (2 * k - sk_m(k) + 15) / 16; }
@@ -400,7 +401,7 @@ template <int NL>
 static SkStage sk_stage(unsigned k) {
   typedef SkShape<NL> P;
   const size_t budget = (size_t)(228 * 1024) / P::ctas - 1024 - 2560;  // of one CTA, less its static arrays
-  const size_t table = (size_t)P::S * (P::slot + 4 + 2);
+  const size_t table = (size_t)P::S * (8 + 4 + 2);
   auto bytes = [&](uint32_t rc, uint32_t dd) { return (size_t)rc * (4 * sk_words(k) + 4 + 1) + (size_t)dd * 4; };
   SkStage g{128, 256, 0};
   for (uint32_t rc = 128; rc <= kSkMaxRecs; rc += 64) {
@@ -534,9 +535,8 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
   constexpr int W2 = 2 * NL;  // 32-bit words of a key
   extern __shared__ __align__(16) unsigned char sk_smem_[];
   constexpr bool REF = P::ref;
-  constexpr uint32_t KW = P::slot / 8;  // 64-bit words of a slot
   uint64_t* keys = (uint64_t*)sk_smem_;
-  uint32_t* cnt = (uint32_t*)(keys + (size_t)S * KW);
+  uint32_t* cnt = (uint32_t*)(keys + S);
   uint16_t* used = (uint16_t*)(cnt + S);
   unsigned char* uni = (unsigned char*)(used + S);
   const uint32_t SW = sk_words(k);
@@ -566,7 +566,7 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
   };
   if (threadIdx.x == 0 && (*(volatile int*)err & (int)kErrRegion)) stop_all(0);
   for (int i = threadIdx.x; i < kHistBins; i += TH) s_hist[i] = 0;
-  for (uint32_t i = threadIdx.x; i < S * KW; i += TH) keys[i] = kFree;
+  for (uint32_t i = threadIdx.x; i < S; i += TH) keys[i] = kFree;
   for (uint32_t i = threadIdx.x; i < S; i += TH) cnt[i] = 0;
   for (;;) {
     __syncthreads();
@@ -808,7 +808,7 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
         // each of the parts ahead), each with all of the records.  They come ever
         // more slowly where reads repeat, so eight times the limit is allowed.
         uint32_t top = 0;
-        for (uint32_t i = threadIdx.x; i < S * KW; i += TH) keys[i] = kFree;
+        for (uint32_t i = threadIdx.x; i < S; i += TH) keys[i] = kFree;
         for (uint32_t i = threadIdx.x; i < S; i += TH) {
           top = max(top, cnt[i]);
           cnt[i] = 0;
@@ -879,8 +879,7 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
           const Seq<NL> V = sk_seq<NL>(F), Rc = sk_seq<NL>(G);
           C = seq_le<NL>(V, Rc) ? V : Rc;
         } else {
-#pragma unroll
-          for (int j = 0; j < NL; j++) C.v[j] = keys[(size_t)KW * s + j];
+          C.v[0] = keys[s];
         }
         const unsigned bl = __ballot_sync(FULL, c >= lmin), bs = __ballot_sync(FULL, c == 1);
         if (c >= lmin) {
@@ -901,8 +900,7 @@ __global__ void __launch_bounds__(SkShape<NL>::threads, SkShape<NL>::ctas)
       __syncthreads();
       for (uint32_t i = threadIdx.x; i < n; i += TH) {
         const uint32_t s = used[i];
-#pragma unroll
-        for (uint32_t j = 0; j < KW; j++) keys[(size_t)KW * s + j] = kFree;
+        keys[s] = kFree;
         cnt[s] = 0;
       }
       // the next part, of the same depth (a shallower one would overflow as the
