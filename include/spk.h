@@ -435,7 +435,8 @@ int spk_batch_end(spk_batch* batch);
  * than the whole budget is refused (SPK_E_ADMISSION). */
 int spk_serve_start(spk_ctx* ctx, uint64_t hbm_budget_bytes, int max_inflight);
 int spk_serve_stop(spk_ctx* ctx);
-/* Estimated device bytes a job needs (Bloom + table + reads + outputs). */
+/* Estimated device bytes a job holds at its peak (reads, Bloom tiers, the lists or
+ * the table of its schedule, outputs). */
 int spk_job_hbm_estimate(const spk_job* job, uint64_t* bytes);
 int spk_submit(spk_ctx* ctx, const spk_job* job, uint64_t* ticket);
 /* *done = 1 when the job finished (successfully or not). */

@@ -194,8 +194,7 @@ int spk_serve_start(spk_ctx* ctx, uint64_t hbm_budget_bytes, int max_inflight) {
   // At the arrival rates of a service a job takes a small share of the time
   // between arrivals, so running most jobs alone costs little queueing.
   // The jobs that run side by side share one block of the pool, mapped here
-  // (several times their shared budget: their estimates leave out the list
-  // sort's and the edges' temporaries, and blocks freed by one job in the
+  // (several times their shared budget: blocks freed by one job in the
   // middle of another's are reused only once both are done).
   pool_reserve(ctx, hbm_budget_bytes / 4);
   s->sched = std::make_shared<Scheduler>(hbm_budget_bytes, max_inflight > 0 ? max_inflight : 4,
