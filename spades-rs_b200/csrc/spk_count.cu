@@ -3901,6 +3901,9 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
   }
   const uint32_t list_min = o.list_min_count ? o.list_min_count : 2;
   const uint32_t lmin_pre = std::max(1u, std::min(fixed ? fixed : 2u, list_min));
+  // What the buffers hold: from super-k-mers every k-mer counted twice, whatever the
+  // thresholds, as its Bloom operations are read from there.
+  const uint32_t lmin_buf = superk ? std::min(lmin_pre, 2u) : lmin_pre;
   kr.list_min = lmin_pre;
 
   uint32_t launches = 1;  // k_occ
@@ -3930,7 +3933,7 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
     for (int j = 0; j < nl; j++)
       if ((r2 = kr.list[j].alloc(lcap_ * 8, st)) || (r2 = sgl[j].alloc(scap_ * 8, st))) return r2;
     if ((r2 = kr.list[4].alloc(lcap_ * 4, st))) return r2;
-    lo = list_out(kr, sgl, lcap_, scap_, lmin_pre, su);
+    lo = list_out(kr, sgl, lcap_, scap_, lmin_buf, su);
     return SPK_OK;
   };
 
@@ -4101,20 +4104,26 @@ int count_one_k_list(spk_ctx* ctx, cudaStream_t st, uint64_t* host, const ReadsV
     for (int c = (int)c0; c < kHistBins; c++) ns += host[S_HIST + c];
     return ns;
   };
-  info.n_list = kr.list_min == lmin_pre ? kr.list_len : hist_from(kr.list_min);
   if (kr.list_min != lmin_pre && kr.list_min >= (uint32_t)(kHistBins - 1))
     return fail(SPK_E_INVALID_ARG, "list_min_count above 254 needs a fixed min_count");
-  if (info.cutoff < (uint32_t)(kHistBins - 1)) {
-    info.n_solid = hist_from(info.cutoff);
-  } else {
+  // k-mers of the list that reach a threshold (q: 0 the cutoff, 1 the list's)
+  auto listed_from = [&](int q, uint64_t* out) -> int {
+    if (hthr[q] < (uint32_t)(kHistBins - 1)) {
+      *out = hist_from(hthr[q]);
+      return SPK_OK;
+    }
     SPK_CUDA(cudaMemsetAsync(sw + S_CNT, 0, 8, st));
-    k_count_solid<<<grid_for(ctx, 2), 256, 0, st>>>(kr.list[4].as<uint32_t>(), kr.list_len, thr, su + S_CNT);
+    k_count_solid<<<grid_for(ctx, 2), 256, 0, st>>>(kr.list[4].as<uint32_t>(), kr.list_len, thr + q, su + S_CNT);
     SPK_CUDA(cudaGetLastError());
     launches++;
     SPK_CUDA(cudaMemcpyAsync(host + S_CNT, sw + S_CNT, 8, cudaMemcpyDeviceToHost, st));
     SPK_CUDA(cudaStreamSynchronize(st));
-    info.n_solid = host[S_CNT];
-  }
+    *out = host[S_CNT];
+    return SPK_OK;
+  };
+  info.n_list = kr.list_len;
+  if (kr.list_min != lmin_buf && (rc = listed_from(1, &info.n_list))) return rc;
+  if ((rc = listed_from(0, &info.n_solid))) return rc;
   SPK_CUDA(cudaEventRecord(e3.e, st));
 
   // ---- sort of the list, into buffers of its size (the singleton buffers,

@@ -763,3 +763,34 @@ def test_super_kmer_partition(spk, ora, k, kind):
     dk, dc = d.kmers(0)
     np.testing.assert_array_equal(dk, tk[tc >= 2])
     np.testing.assert_array_equal(dc, tc[tc >= 2])
+
+
+@pytest.mark.parametrize("k,cov", [(21, 30), (33, 30), (55, 40), (77, 40), (127, 40), (31, 700)])
+@pytest.mark.parametrize("list_min,min_count", [(3, 5), (5, 3), (4, 4), (300, 300), (280, 260), (1, 5), (2, 300)])
+def test_thresholds_above_two(spk, ora, k, cov, list_min, min_count):
+    """Thresholds above two on the default job: k-mers below them are not listed, but
+    their Bloom operations are made, and so are the admissions that follow from the
+    tiers; thresholds past the histogram's last bin count the list itself."""
+    from spk import synth
+    # (k > 64: enough occurrences for the super-k-mers to take the set)
+    size = 2_000 if cov > 100 else 20_000 if k <= 64 else 120_000
+    p = synth.sample(size, float(cov), seed=k, err=(0.004, 0.008), ks=(k,)).packed
+    bits = 1 << 20 if k <= 64 else 1 << 23
+    ref = ora.count(p.data, p.offsets, p.lengths, k, bits, mode=ora.MODE_TWICE)
+    tk, tc = ref.table(1)
+    r = spk.count(p, [k], bloom_bits=bits, list_min_count=list_min, min_count=min_count, flags=BASE)
+    info = r.info(0)
+    assert info["schedule"] == 3 and info["cutoff"] == min_count
+    for a, b in zip(r.bloom(0), ref.bloom()):
+        np.testing.assert_array_equal(a, b)
+    assert info["n_table"] == tk.shape[0] and info["n_singletons"] == int((tc == 1).sum())
+    assert info["admitted_occurrences"] == int(tc.astype(np.int64).sum())
+    thr = min(list_min, min_count)
+    assert info["n_list"] == int((tc >= thr).sum()) and info["n_solid"] == int((tc >= min_count).sum())
+    gk, gc = r.kmers(0, 1)
+    np.testing.assert_array_equal(gk, tk[tc >= thr])
+    np.testing.assert_array_equal(gc, tc[tc >= thr])
+    sk, sc = r.solid(0)
+    np.testing.assert_array_equal(sk, tk[tc >= min_count])
+    np.testing.assert_array_equal(sc, tc[tc >= min_count])
+    np.testing.assert_array_equal(r.edges(0), ora.edges(sk, k))
